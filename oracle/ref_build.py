@@ -66,7 +66,7 @@ def cuda_include() -> str:
 
 def available() -> bool:
     """True where the reference sources this recipe compiles are present."""
-    return os.path.isdir(REF)
+    return all(os.path.exists(os.path.join(REF, f)) for f in SOURCES + [RENAMED_MAIN])
 
 
 def build(force: bool = False) -> str:
