@@ -152,9 +152,12 @@ __device__ __forceinline__ int ford(float f) {
     return i >= 0 ? i : i ^ 0x7fffffff;
 }
 
+// Projected bounds of all triangles (b: ordered ints) and the sums of their boxes' widths,
+// heights and areas (finite ones), which choose the cell size.
 template <int AXIS>
-__global__ void k_cg_bounds(const float4* __restrict__ tris, int n, int* __restrict__ b) {
+__global__ void k_cg_bounds(const float4* __restrict__ tris, int n, int* __restrict__ b, double* __restrict__ sums) {
     float ul = INFINITY, uh = -INFINITY, vl = INFINITY, vh = -INFINITY;
+    float sw = 0.0f, sh = 0.0f, sa = 0.0f;  // a thread sums a few dozen boxes: the sizing needs no more digits
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         float a0, a1, a2, a3;
         tri_uv_box<AXIS>(tris, k, a0, a1, a2, a3);
@@ -162,6 +165,12 @@ __global__ void k_cg_bounds(const float4* __restrict__ tris, int n, int* __restr
         uh = fmaxf(uh, a1);
         vl = fminf(vl, a2);
         vh = fmaxf(vh, a3);
+        const float w = a1 - a0, h = a3 - a2;
+        if (w * h < INFINITY) {
+            sw += w;
+            sh += h;
+            sa += w * h;
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -169,30 +178,83 @@ __global__ void k_cg_bounds(const float4* __restrict__ tris, int n, int* __restr
         uh = fmaxf(uh, __shfl_xor_sync(0xffffffffu, uh, o));
         vl = fminf(vl, __shfl_xor_sync(0xffffffffu, vl, o));
         vh = fmaxf(vh, __shfl_xor_sync(0xffffffffu, vh, o));
+        sw += __shfl_xor_sync(0xffffffffu, sw, o);
+        sh += __shfl_xor_sync(0xffffffffu, sh, o);
+        sa += __shfl_xor_sync(0xffffffffu, sa, o);
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&b[0], ford(ul));
-        atomicMax(&b[1], ford(uh));
-        atomicMin(&b[2], ford(vl));
-        atomicMax(&b[3], ford(vh));
+    __shared__ float red[7][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) {
+        const float v[7] = {ul, uh, vl, vh, sw, sh, sa};
+#pragma unroll
+        for (int q = 0; q < 7; ++q) red[q][warp] = v[q];
     }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
+        ul = fminf(ul, red[0][w]);
+        uh = fmaxf(uh, red[1][w]);
+        vl = fminf(vl, red[2][w]);
+        vh = fmaxf(vh, red[3][w]);
+        sw += red[4][w];
+        sh += red[5][w];
+        sa += red[6][w];
+    }
+    atomicMin(&b[0], ford(ul));
+    atomicMax(&b[1], ford(uh));
+    atomicMin(&b[2], ford(vl));
+    atomicMax(&b[3], ford(vh));
+    atomicAdd(&sums[0], (double)sw);
+    atomicAdd(&sums[1], (double)sh);
+    atomicAdd(&sums[2], (double)sa);
 }
 
+// Counts (FILL false) or lists (FILL true, count holding each cell's length) the cells that
+// every triangle's projected box touches.  A warp flattens the rectangles of its 32
+// triangles into one work list, so a lane never walks a large rectangle alone; the fill
+// takes its slots from the cell's end, and the counts are back at zero after it.
 template <int AXIS, bool FILL>
-__global__ void k_cg_cells(const float4* __restrict__ tris, int n, GridView g, uint32_t* __restrict__ count,
-                           uint32_t* __restrict__ list) {
+__global__ void __launch_bounds__(256) k_cg_cells(const float4* __restrict__ tris, int n, GridView g,
+                                                  uint32_t* __restrict__ count, uint32_t* __restrict__ list) {
+    const int lane = threadIdx.x & 31;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    float ul, uh, vl, vh;
-    tri_uv_box<AXIS>(tris, k, ul, uh, vl, vh);
-    const int cu0 = cell_of(ul, g.u0, g.su, g.gu), cu1 = cell_of(uh, g.u0, g.su, g.gu);
-    const int cv0 = cell_of(vl, g.v0, g.sv, g.gv), cv1 = cell_of(vh, g.v0, g.sv, g.gv);
-    for (int cv = cv0; cv <= cv1; ++cv)
-        for (int cu = cu0; cu <= cu1; ++cu) {
-            const int c = cv * g.gu + cu;
-            const uint32_t slot = atomicAdd(&count[c], 1u);
-            if (FILL) list[g.start[c] + slot] = (uint32_t)k;
+    uint32_t cells = 0, first = 0, width = 1;
+    if (k < n) {
+        float ul, uh, vl, vh;
+        tri_uv_box<AXIS>(tris, k, ul, uh, vl, vh);
+        const int cu0 = cell_of(ul, g.u0, g.su, g.gu), cu1 = cell_of(uh, g.u0, g.su, g.gu);
+        const int cv0 = cell_of(vl, g.v0, g.sv, g.gv), cv1 = cell_of(vh, g.v0, g.sv, g.gv);
+        if (cu1 >= cu0 && cv1 >= cv0) {
+            width = (uint32_t)(cu1 - cu0 + 1);
+            cells = width * (uint32_t)(cv1 - cv0 + 1);
+            first = (uint32_t)(cv0 * g.gu + cu0);
         }
+    }
+    uint32_t inc = cells;  // 32 rectangles of at most 2^26 cells fit
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    const uint32_t pre = inc - cells, total = __shfl_sync(0xffffffffu, inc, 31);
+    for (uint32_t base = 0; base < total; base += 32) {
+        const uint32_t j = base + lane;
+        int owner = 0;  // the last lane whose prefix is <= j
+#pragma unroll
+        for (int step = 16; step >= 1; step >>= 1) {
+            const uint32_t pc = __shfl_sync(0xffffffffu, pre, owner + step);
+            if (pc <= j) owner += step;
+        }
+        const uint32_t of = __shfl_sync(0xffffffffu, first, owner), ow = __shfl_sync(0xffffffffu, width, owner);
+        const uint32_t op = __shfl_sync(0xffffffffu, pre, owner);
+        const int ok = __shfl_sync(0xffffffffu, k, owner);
+        if (j < total) {
+            const uint32_t r = (uint32_t)(j - op), row = r / ow;
+            const uint32_t c = of + row * (uint32_t)g.gu + (r - row * ow);
+            if (FILL) list[g.start[c] + atomicSub(&count[c], 1u) - 1u] = (uint32_t)ok;
+            else atomicAdd(&count[c], 1u);
+        }
+    }
 }
 
 std::mutex g_grid_mu;
@@ -204,42 +266,68 @@ float dec_ord(int i) {
     return f;
 }
 
+// Cells of a grid over n triangles with the given projected extent and sums of box widths,
+// heights and areas.  At most four per triangle (and 2^24): more would not shorten the
+// lists of a mesh whose boxes are as small as its cells.  At s cells per unit of length a
+// box of w x h touches about (s w + 1)(s h + 1) cells, so n boxes make about
+// s^2 sum(w h) + s (sum w + sum h) + n list entries; cells are made larger until that is at
+// most kEntries a triangle, since many small objects over a wide scene would otherwise list
+// every triangle in a hundred cells and more.  Up to kFree entries the build takes no longer
+// than its launches and stays at four cells a triangle.
+constexpr double kEntries = 12.0;
+constexpr double kFree = 4194304.0;
+
+double grid_cells(double n, double w, double h, const double* sum) {
+    const double finest = std::min(std::max(4.0 * n, 1.0), (double)(1 << 24));
+    const double budget = std::max(kEntries * n, kFree);
+    if (!(w > 0 && h > 0) || !std::isfinite(w * h)) return finest;
+    const double s0 = std::sqrt(finest / (w * h)), lin = sum[0] + sum[1], area = sum[2];
+    if (!(s0 * s0 * area + s0 * lin + n > budget)) return finest;
+    const double room = budget - n;
+    const double s = area > 0 ? (-lin + std::sqrt(lin * lin + 4.0 * area * room)) / (2.0 * area) : room / lin;
+    return std::min(std::max(finest * (s / s0) * (s / s0), 1.0), finest);
+}
+
 template <int AXIS>
 cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
     rs_column_grid& cg = bvh->cgrid[AXIS];
     const int n = (int)bvh->n_tris;
-    int* b = nullptr;
-    cudaError_t e = dmalloc((void**)&b, 4 * sizeof(int), s);
+    int* b = nullptr;  // four ordered ints, then three sums
+    constexpr size_t kBytes = 4 * sizeof(int) + 3 * sizeof(double);
+    cudaError_t e = dmalloc((void**)&b, kBytes, s);
     if (e != cudaSuccess) return e;
-    const int init[4] = {0x7fffffff, (int)0x80000000, 0x7fffffff, (int)0x80000000};
-    cudaMemcpyAsync(b, init, sizeof(init), cudaMemcpyHostToDevice, s);
-    launch(k_cg_bounds<AXIS>, 2 * sm_count(), 256, 0, s, (const float4*)bvh->tris, n, b);
-    int hb[4];
-    e = cudaMemcpyAsync(hb, b, sizeof(hb), cudaMemcpyDeviceToHost, s);
+    struct {
+        int b[4] = {0x7fffffff, (int)0x80000000, 0x7fffffff, (int)0x80000000};
+        double sum[3] = {0.0, 0.0, 0.0};
+    } h;
+    static_assert(sizeof(h) == kBytes, "bounds layout");
+    cudaMemcpyAsync(b, &h, kBytes, cudaMemcpyHostToDevice, s);
+    launch(k_cg_bounds<AXIS>, std::min(2 * sm_count(), (n + 255) / 256), 256, 0, s, (const float4*)bvh->tris, n, b,
+           reinterpret_cast<double*>(b + 4));
+    e = cudaMemcpyAsync(&h, b, kBytes, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaFreeAsync(b, s);
     if (e != cudaSuccess) return e;
-    cg.u0 = dec_ord(hb[0]);
-    cg.u1 = dec_ord(hb[1]);
-    cg.v0 = dec_ord(hb[2]);
-    cg.v1 = dec_ord(hb[3]);
-    // About four cells per triangle, shaped like the projected bounds.
-    const double target = std::min(std::max(4.0 * n, 1.0), (double)(1 << 24));
-    const double w = (double)cg.u1 - cg.u0, h = (double)cg.v1 - cg.v0;
+    cg.u0 = dec_ord(h.b[0]);
+    cg.u1 = dec_ord(h.b[1]);
+    cg.v0 = dec_ord(h.b[2]);
+    cg.v1 = dec_ord(h.b[3]);
+    const double w = (double)cg.u1 - cg.u0, hh = (double)cg.v1 - cg.v0;
+    const double target = grid_cells(n, w, hh, h.sum);
     int gu = 1, gv = 1;
-    if (w > 0 && h > 0) {
-        gu = (int)std::lround(std::sqrt(target * w / h));
+    if (w > 0 && hh > 0) {
+        gu = (int)std::lround(std::sqrt(target * w / hh));
         gu = std::min(std::max(gu, 1), 8192);
         gv = (int)std::min(std::max(std::lround(target / gu), 1L), 8192L);
     } else if (w > 0) {
         gu = (int)std::min(target, 8192.0);
-    } else if (h > 0) {
+    } else if (hh > 0) {
         gv = (int)std::min(target, 8192.0);
     }
     cg.gu = gu;
     cg.gv = gv;
     cg.su = w > 0 ? (float)gu / (float)w : 0.0f;
-    cg.sv = h > 0 ? (float)gv / (float)h : 0.0f;
+    cg.sv = hh > 0 ? (float)gv / (float)hh : 0.0f;
     const size_t ncell = (size_t)gu * gv;
     uint32_t* count = nullptr;
     e = dmalloc((void**)&count, ncell * sizeof(uint32_t), s);
@@ -255,7 +343,6 @@ cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e == cudaSuccess) e = dmalloc((void**)&cg.list, (size_t)std::max<uint32_t>(total, 1) * 4, s);
     if (e == cudaSuccess) {
-        cudaMemsetAsync(count, 0, ncell * sizeof(uint32_t), s);
         launch(k_cg_cells<AXIS, true>, grid, 256, 0, s, (const float4*)bvh->tris, n, gvw, count, cg.list);
         e = cudaGetLastError();
     }
