@@ -48,8 +48,7 @@ struct BatchQuery {
     uint64_t n;
     uint64_t first_chunk;
     unsigned int* status;
-    int use_grid;  // axis-aligned point-in-mesh through the handle's column grid
-    GridView grid;
+    GridView grid;  // axis-aligned point-in-mesh: the handle's column grid
 };
 
 __device__ __forceinline__ int find_query(const BatchQuery* __restrict__ q, int nq, uint64_t chunk) {
@@ -62,86 +61,96 @@ __device__ __forceinline__ int find_query(const BatchQuery* __restrict__ q, int 
     return lo;
 }
 
+// One warp's shared memory: a chunk is grid queries, rays or edges (stacks and crossings in
+// one column per lane), so the three share it.
+template <int STACK>
+union BatchWarp {
+    GridWarpSlots grid;
+    HitSmem<32, STACK> rays;
+    EdgeSmem<32, STACK> edges;
+};
+
+template <int STACK>
+__device__ __forceinline__ BatchWarp<STACK>& batch_warp() {
+    extern __shared__ __align__(16) unsigned char batch_smem[];
+    return reinterpret_cast<BatchWarp<STACK>*>(batch_smem)[threadIdx.x >> 5];
+}
+
+__device__ __forceinline__ void batch_spill(const BatchQuery& Q, int qi, uint64_t i, uint2* __restrict__ ovf,
+                                            unsigned long long* __restrict__ ovf_count) {
+    const unsigned long long slot = atomicAdd(ovf_count, 1ull);
+    if (slot < kOverflowCap) ovf[slot] = make_uint2((uint32_t)qi, (uint32_t)i);
+    else atomicOr(Q.status, ST_HIT_OVERFLOW);
+}
+
+// The three kinds of chunk are functions of their own: inlined into one kernel they
+// spilled 1.2 KB of registers a thread at 168 registers.
+
+// Warp-cooperative rounds of 32 points: every lane takes part in each round.
 template <int AXIS, int STACK>
-__device__ __forceinline__ void batch_pim_ray(const BatchQuery& Q, int qi, uint64_t i, uint2* __restrict__ ovf,
-                                              unsigned long long* __restrict__ ovf_count) {
-    const Ray r = make_ray(Q.pts[3 * i], Q.pts[3 * i + 1], Q.pts[3 * i + 2], Q.dx, Q.dy, Q.dz, kEps, kTmax);
-    HitList hl;
-    unsigned int tests = 0;
-    const bool ok = pim_collect<AXIS, STACK>(Q.nodes, Q.max_steps, Q.tris, r, hl, tests);
-    add_tests(tests);
-    if (!ok) {
-        atomicOr(Q.status, ST_STACK_OVERFLOW);
-        return;
+__device__ __noinline__ void batch_grid(const BatchQuery& Q, int qi, uint64_t r0, uint64_t r1, uint2* ovf,
+                                        unsigned long long* ovf_count) {
+    GridWarpSlots& sl = batch_warp<STACK>().grid;
+    for (uint64_t base = r0; base < r1; base += 32) {
+        const uint64_t i = base + (threadIdx.x & 31);
+        const bool valid = i < r1;
+        float p[3] = {0.0f, 0.0f, 0.0f};
+        if (valid) {
+            p[0] = Q.pts[3 * i];
+            p[1] = Q.pts[3 * i + 1];
+            p[2] = Q.pts[3 * i + 2];
+        }
+        pim_grid_warp<AXIS>(Q.grid, Q.tris, p, valid, valid, i, Q.obj, Q.in, sl,
+                            [&]() { batch_spill(Q, qi, i, ovf, ovf_count); });
+        __syncwarp();
     }
-    if (hl.ovf) {
-        const unsigned long long slot = atomicAdd(ovf_count, 1ull);
-        if (slot < kOverflowCap) ovf[slot] = make_uint2((uint32_t)qi, (uint32_t)i);
-        else atomicOr(Q.status, ST_HIT_OVERFLOW);
-        return;
+}
+
+// Point-in-mesh rays of any direction: BVH traversal, one lane per ray.
+template <int STACK>
+__device__ __noinline__ void batch_rays(const BatchQuery& Q, int qi, uint64_t r0, uint64_t r1, uint2* ovf,
+                                        unsigned long long* ovf_count) {
+    const HitColumn col = batch_warp<STACK>().rays.column(threadIdx.x & 31);
+    for (uint64_t i = r0 + (threadIdx.x & 31); i < r1; i += 32) {
+        const Ray r = make_ray(Q.pts[3 * i], Q.pts[3 * i + 1], Q.pts[3 * i + 2], Q.dx, Q.dy, Q.dz, kEps, kTmax);
+        int n;
+        const bool ok = pim_column<-1, STACK>(col, Q.nodes, Q.max_steps, Q.tris, r, n);
+        if (!ok) atomicOr(Q.status, ST_STACK_OVERFLOW);
+        else if (n > kHits) batch_spill(Q, qi, i, ovf, ovf_count);
+        else write_result(column_chain(col, n), i, Q.obj, Q.in);
     }
-    write_result(hl.finish(), i, Q.obj, Q.in);
 }
 
 template <int STACK>
-__global__ void __launch_bounds__(kBT) k_batch(const BatchQuery* __restrict__ q, int nq, uint64_t total_chunks,
+__device__ __noinline__ void batch_edges(const BatchQuery& Q, int qi, uint64_t r0, uint64_t r1, uint2* ovf,
+                                         unsigned long long* ovf_count) {
+    const EdgeColumn col = batch_warp<STACK>().edges.column(threadIdx.x & 31);
+    const EdgePayload p{Q.starts, Q.ends, Q.offsets, Q.counts, Q.sources};
+    for (uint64_t i = r0 + (threadIdx.x & 31); i < r1; i += 32)
+        if (!edge_ray_fast<STACK>(col, p, i, Q.nodes, Q.max_steps, Q.tris, Q.swap, Q.table))
+            batch_spill(Q, qi, i, ovf, ovf_count);
+}
+
+template <int STACK>
+__global__ void __launch_bounds__(kBT, 4) k_batch(const BatchQuery* __restrict__ q, int nq, uint64_t total_chunks,
                                                int chunk, unsigned long long* __restrict__ next,
                                                uint2* __restrict__ ovf, unsigned long long* __restrict__ ovf_count) {
-    __shared__ GridWarpSlots slots[kBT / 32];
-    __shared__ EdgeSmem<kBT, STACK> esm;  // edge rays' stacks and crossings, one column per thread
-    const int lane = threadIdx.x & 31;
-    GridWarpSlots& sl = slots[threadIdx.x >> 5];
     for (;;) {
         unsigned long long c = 0;
-        if (lane == 0) c = atomicAdd(next, 1ull);
+        if ((threadIdx.x & 31) == 0) c = atomicAdd(next, 1ull);
         c = __shfl_sync(0xffffffffu, c, 0);
         if (c >= total_chunks) return;
         const int qi = find_query(q, nq, c);
         const BatchQuery& Q = q[qi];
         const uint64_t r0 = (c - Q.first_chunk) * (uint64_t)chunk;
         const uint64_t r1 = min(r0 + (uint64_t)chunk, Q.n);
-        if (Q.kind == 0 && Q.use_grid) {
-            // Warp-cooperative rounds of 32 points: every lane takes part in each round.
-            for (uint64_t base = r0; base < r1; base += 32) {
-                const uint64_t i = base + lane;
-                const bool valid = i < r1;
-                float p[3] = {0.0f, 0.0f, 0.0f};
-                if (valid) {
-                    p[0] = Q.pts[3 * i];
-                    p[1] = Q.pts[3 * i + 1];
-                    p[2] = Q.pts[3 * i + 2];
-                }
-                auto spill = [&]() {
-                    const unsigned long long slot = atomicAdd(ovf_count, 1ull);
-                    if (slot < kOverflowCap) ovf[slot] = make_uint2((uint32_t)qi, (uint32_t)i);
-                    else atomicOr(Q.status, ST_HIT_OVERFLOW);
-                };
-                if (Q.axis == 0) pim_grid_warp<0>(Q.grid, Q.tris, p, valid, valid, i, Q.obj, Q.in, sl, spill);
-                else if (Q.axis == 1) pim_grid_warp<1>(Q.grid, Q.tris, p, valid, valid, i, Q.obj, Q.in, sl, spill);
-                else pim_grid_warp<2>(Q.grid, Q.tris, p, valid, valid, i, Q.obj, Q.in, sl, spill);
-                __syncwarp();
-            }
-            continue;
-        }
-        for (uint64_t i = r0 + lane; i < r1; i += 32) {
-            if (Q.kind == 1) {
-                const EdgePayload p{Q.starts, Q.ends, Q.offsets, Q.counts, Q.sources};
-                if (!edge_ray_fast<STACK>(esm.column(threadIdx.x), p, i, Q.nodes, Q.max_steps, Q.tris, Q.swap,
-                                          Q.table)) {
-                    const unsigned long long slot = atomicAdd(ovf_count, 1ull);
-                    if (slot < kOverflowCap) ovf[slot] = make_uint2((uint32_t)qi, (uint32_t)i);
-                    else atomicOr(Q.status, ST_HIT_OVERFLOW);
-                }
-            } else if (Q.axis == 0) {
-                batch_pim_ray<0, STACK>(Q, qi, i, ovf, ovf_count);
-            } else if (Q.axis == 1) {
-                batch_pim_ray<1, STACK>(Q, qi, i, ovf, ovf_count);
-            } else if (Q.axis == 2) {
-                batch_pim_ray<2, STACK>(Q, qi, i, ovf, ovf_count);
-            } else {
-                batch_pim_ray<-1, STACK>(Q, qi, i, ovf, ovf_count);
-            }
-        }
+        // Axis-aligned point queries always have a grid (queries of empty meshes have no chunk).
+        if (Q.kind == 1) batch_edges<STACK>(Q, qi, r0, r1, ovf, ovf_count);
+        else if (Q.axis == 0) batch_grid<0, STACK>(Q, qi, r0, r1, ovf, ovf_count);
+        else if (Q.axis == 1) batch_grid<1, STACK>(Q, qi, r0, r1, ovf, ovf_count);
+        else if (Q.axis == 2) batch_grid<2, STACK>(Q, qi, r0, r1, ovf, ovf_count);
+        else batch_rays<STACK>(Q, qi, r0, r1, ovf, ovf_count);
+        __syncwarp();
     }
 }
 
@@ -237,6 +246,11 @@ void release_device(rs_batch* b) {
     b->dirty = true;
 }
 
+template <int STACK>
+constexpr size_t batch_smem_bytes() {
+    return (kBT / 32) * sizeof(BatchWarp<STACK>);
+}
+
 int commit(rs_batch* b, cudaStream_t s) {
     if (!b->dirty) return RS_OK;
     release_device(b);
@@ -273,9 +287,7 @@ int commit(rs_batch* b, cudaStream_t s) {
             if (q.axis >= 0 && h->n_tris > 0) {
                 const int g = ensure_grid(h, q.axis, s);
                 if (g != RS_OK) return g;
-                const rs_column_grid& cg = h->cgrid[q.axis];
-                q.use_grid = 1;
-                q.grid = GridView{cg.u0, cg.v0, cg.su, cg.sv, cg.u1, cg.v1, cg.gu, cg.gv, cg.start, cg.list};
+                q.grid = grid_view(h->cgrid[q.axis]);
             }
         } else {
             q.axis = -1;
@@ -303,8 +315,8 @@ int commit(rs_batch* b, cudaStream_t s) {
     }
     b->total_chunks = chunks;
     int per_sm = 0;
-    if (b->stack == 32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<32>, kBT, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<64>, kBT, 0);
+    if (b->stack == 32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<32>, kBT, batch_smem_bytes<32>());
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<64>, kBT, batch_smem_bytes<64>());
     b->grid = std::max(1, per_sm) * sm_count();
     b->dirty = false;
     return RS_OK;
@@ -333,12 +345,12 @@ cudaError_t enqueue(rs_batch* b, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     if (b->total_chunks) {
         if (b->stack == 32) {
-            launch(k_batch<32>, b->grid, kBT, 0, s, (const BatchQuery*)b->d_q, nq, b->total_chunks, b->chunk,
+            launch(k_batch<32>, b->grid, kBT, batch_smem_bytes<32>(), s, (const BatchQuery*)b->d_q, nq, b->total_chunks, b->chunk,
                    b->d_counters, b->d_ovf, b->d_counters + 1);
             if (b->d_ovf) launch(k_batch_fallback<32>, fallback_grid(b), kBT, 0, s, (const BatchQuery*)b->d_q,
                                  (const uint2*)b->d_ovf, (const unsigned long long*)b->d_counters + 1);
         } else {
-            launch(k_batch<64>, b->grid, kBT, 0, s, (const BatchQuery*)b->d_q, nq, b->total_chunks, b->chunk,
+            launch(k_batch<64>, b->grid, kBT, batch_smem_bytes<64>(), s, (const BatchQuery*)b->d_q, nq, b->total_chunks, b->chunk,
                    b->d_counters, b->d_ovf, b->d_counters + 1);
             if (b->d_ovf) launch(k_batch_fallback<64>, fallback_grid(b), kBT, 0, s, (const BatchQuery*)b->d_q,
                                  (const uint2*)b->d_ovf, (const unsigned long long*)b->d_counters + 1);

@@ -7,14 +7,15 @@
 #include "rs_device.cuh"
 
 // Column grid for rays along +e_axis: a uniform grid over the two other axes whose
-// cells list (in leaf order) every triangle whose projected box touches the cell.
+// cells list every triangle whose projected box touches the cell.
 struct rs_column_grid {
     int built = 0;
     float u0 = 0, v0 = 0, su = 0, sv = 0;  // cell(x) = clamp(floor((x - u0) * su), 0, gu - 1)
     float u1 = 0, v1 = 0;                  // projected bounds of all triangles
+    float w0 = 0, sw = 0, w1 = 0;          // bounds along the axis; sw = 256 / (w1 - w0)
     int gu = 1, gv = 1;
     uint32_t* start = nullptr;             // gu*gv + 1 offsets into list
-    uint32_t* list = nullptr;              // leaf-order triangle indices
+    uint2* list = nullptr;                 // entries (GridView in rs_query_core.cuh)
     uint64_t nlist = 0;
 };
 

@@ -53,12 +53,17 @@ __device__ __forceinline__ bool box_filter(const float* __restrict__ box, const 
 }
 
 
+// BVH traversal per ray: a 32-entry stack and the crossings in shared memory (28 KB a block of
+// 128 threads); deeper or longer rays go to the fallback.
+constexpr int kPimT = 128;
+constexpr int kPimStack = 32;
+
 template <int AXIS, bool FILTER>
-__global__ void __launch_bounds__(kT) k_pim(const float* __restrict__ pts, uint64_t n, float dx, float dy, float dz,
+__global__ void __launch_bounds__(kPimT) k_pim(const float* __restrict__ pts, uint64_t n, float dx, float dy, float dz,
                                             const BNode* __restrict__ nodes, uint32_t max_steps,
                                             const float4* __restrict__ tris, const float* __restrict__ box,
                                             int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
-                                            unsigned int* __restrict__ status, uint32_t* __restrict__ ovf_list,
+                                            uint32_t* __restrict__ ovf_list,
                                             unsigned long long* __restrict__ ovf_count) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -67,30 +72,22 @@ __global__ void __launch_bounds__(kT) k_pim(const float* __restrict__ pts, uint6
         write_result(Chain{}, i, out_obj, out_in);
         return;
     }
-    HitList hl;
-    unsigned int tests = 0;
-    const bool ok = pim_collect<AXIS, kStack>(nodes, max_steps, tris, r, hl, tests);
-    add_tests(tests);
-    if (!ok) {
-        atomicOr(status, ST_STACK_OVERFLOW);
-        return;
-    }
-    if (hl.ovf) {
+    __shared__ HitSmem<kPimT, kPimStack> sm;
+    const HitColumn col = sm.column(threadIdx.x);
+    int n_hits;
+    const bool ok = pim_column<AXIS, kPimStack>(col, nodes, max_steps, tris, r, n_hits);
+    if (!ok || n_hits > kHits) {  // the fallback's deeper stack and longer list take it
         ovf_list[atomicAdd(ovf_count, 1ull)] = (uint32_t)i;
         return;
     }
-    write_result(hl.finish(), i, out_obj, out_in);
+    write_result(column_chain(col, n_hits), i, out_obj, out_in);
 }
 
-// Warp-cooperative column-grid query.  Each warp owns 32 points; their candidate
-// lists are flattened into one (point, triangle) work list with a warp scan, so every
-// lane tests one candidate per round however unevenly the candidates are spread over
-// the points (points outside the projected bounds contribute none).  Crossings go to
-// per-point slots in shared memory; each lane then sorts and counts its own point's.
+// Column-grid query, 32 points a warp (pim_grid_warp).
 constexpr int kWarps = kT / 32;
 
 template <int AXIS, bool FILTER>
-__global__ void __launch_bounds__(kT) k_pim_grid(const float* __restrict__ pts, uint64_t n, GridView g,
+__global__ void __launch_bounds__(kT, 4) k_pim_grid(const float* __restrict__ pts, uint64_t n, GridView g,
                                                  const float4* __restrict__ tris, const float* __restrict__ box,
                                                  int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
                                                  uint32_t* __restrict__ ovf_list,
@@ -133,18 +130,31 @@ __global__ void __launch_bounds__(kT) k_pim_fallback(const float* __restrict__ p
 
 // --- column grid build ---------------------------------------------------------------
 
+// Box of triangle k: across the ray axis (u, v) and along it.
+struct TriBox {
+    float ul, uh, vl, vh, wl, wh;
+    bool nan;  // a coordinate is not a number
+};
+
 template <int AXIS>
-__device__ __forceinline__ void tri_uv_box(const float4* __restrict__ tris, int k, float& ul, float& uh, float& vl,
-                                           float& vh) {
+__device__ __forceinline__ TriBox tri_box(const float4* __restrict__ tris, int k) {
     const float4 a = __ldg(&tris[3 * (size_t)k]), b = __ldg(&tris[3 * (size_t)k + 1]),
                  c = __ldg(&tris[3 * (size_t)k + 2]);
     const float au = AXIS == 0 ? a.y : (AXIS == 1 ? a.z : a.x), av = AXIS == 0 ? a.z : (AXIS == 1 ? a.x : a.y);
     const float bu = AXIS == 0 ? b.y : (AXIS == 1 ? b.z : b.x), bv = AXIS == 0 ? b.z : (AXIS == 1 ? b.x : b.y);
     const float cu = AXIS == 0 ? c.y : (AXIS == 1 ? c.z : c.x), cv = AXIS == 0 ? c.z : (AXIS == 1 ? c.x : c.y);
-    ul = fminf(fminf(au, bu), cu);
-    uh = fmaxf(fmaxf(au, bu), cu);
-    vl = fminf(fminf(av, bv), cv);
-    vh = fmaxf(fmaxf(av, bv), cv);
+    const float aw = AXIS == 0 ? a.x : (AXIS == 1 ? a.y : a.z), bw = AXIS == 0 ? b.x : (AXIS == 1 ? b.y : b.z);
+    const float cw = AXIS == 0 ? c.x : (AXIS == 1 ? c.y : c.z);
+    TriBox r;
+    r.ul = fminf(fminf(au, bu), cu);
+    r.uh = fmaxf(fmaxf(au, bu), cu);
+    r.vl = fminf(fminf(av, bv), cv);
+    r.vh = fmaxf(fmaxf(av, bv), cv);
+    r.wl = fminf(fminf(aw, bw), cw);
+    r.wh = fmaxf(fmaxf(aw, bw), cw);
+    r.nan = isnan(au) || isnan(av) || isnan(aw) || isnan(bu) || isnan(bv) || isnan(bw) || isnan(cu) || isnan(cv) ||
+            isnan(cw);
+    return r;
 }
 
 __device__ __forceinline__ int ford(float f) {
@@ -152,61 +162,46 @@ __device__ __forceinline__ int ford(float f) {
     return i >= 0 ? i : i ^ 0x7fffffff;
 }
 
-// Projected bounds of all triangles (b: ordered ints) and the sums of their boxes' widths,
-// heights and areas (finite ones), which choose the cell size.
+// Bounds of all triangles (b: ordered ints: u, v, w ranges) and the sums of their projected
+// boxes' widths, heights and areas (finite ones), which choose the cell size.
 template <int AXIS>
 __global__ void k_cg_bounds(const float4* __restrict__ tris, int n, int* __restrict__ b, double* __restrict__ sums) {
-    float ul = INFINITY, uh = -INFINITY, vl = INFINITY, vh = -INFINITY;
-    float sw = 0.0f, sh = 0.0f, sa = 0.0f;  // a thread sums a few dozen boxes: the sizing needs no more digits
+    // [0..5] minima of u, -u, v, -v, w, -w, then the three sums (a thread sums a few dozen
+    // boxes: the sizing needs no more digits).
+    float v[9] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, 0.0f, 0.0f, 0.0f};
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        float a0, a1, a2, a3;
-        tri_uv_box<AXIS>(tris, k, a0, a1, a2, a3);
-        ul = fminf(ul, a0);
-        uh = fmaxf(uh, a1);
-        vl = fminf(vl, a2);
-        vh = fmaxf(vh, a3);
-        const float w = a1 - a0, h = a3 - a2;
+        const TriBox t = tri_box<AXIS>(tris, k);
+        // A coordinate that is not a number may be crossed at any height: no height limit then.
+        const float m[6] = {t.ul, -t.uh, t.vl, -t.vh, t.wl, t.nan ? -INFINITY : -t.wh};
+#pragma unroll
+        for (int q = 0; q < 6; ++q) v[q] = fminf(v[q], m[q]);
+        const float w = t.uh - t.ul, h = t.vh - t.vl;
         if (w * h < INFINITY) {
-            sw += w;
-            sh += h;
-            sa += w * h;
+            v[6] += w;
+            v[7] += h;
+            v[8] += w * h;
         }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        ul = fminf(ul, __shfl_xor_sync(0xffffffffu, ul, o));
-        uh = fmaxf(uh, __shfl_xor_sync(0xffffffffu, uh, o));
-        vl = fminf(vl, __shfl_xor_sync(0xffffffffu, vl, o));
-        vh = fmaxf(vh, __shfl_xor_sync(0xffffffffu, vh, o));
-        sw += __shfl_xor_sync(0xffffffffu, sw, o);
-        sh += __shfl_xor_sync(0xffffffffu, sh, o);
-        sa += __shfl_xor_sync(0xffffffffu, sa, o);
-    }
-    __shared__ float red[7][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) {
-        const float v[7] = {ul, uh, vl, vh, sw, sh, sa};
+    for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int q = 0; q < 7; ++q) red[q][warp] = v[q];
-    }
+        for (int q = 0; q < 9; ++q) {
+            const float y = __shfl_xor_sync(0xffffffffu, v[q], o);
+            v[q] = q < 6 ? fminf(v[q], y) : v[q] + y;
+        }
+    __shared__ float red[9][8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < 9; ++q) red[q][warp] = v[q];
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-        ul = fminf(ul, red[0][w]);
-        uh = fmaxf(uh, red[1][w]);
-        vl = fminf(vl, red[2][w]);
-        vh = fmaxf(vh, red[3][w]);
-        sw += red[4][w];
-        sh += red[5][w];
-        sa += red[6][w];
-    }
-    atomicMin(&b[0], ford(ul));
-    atomicMax(&b[1], ford(uh));
-    atomicMin(&b[2], ford(vl));
-    atomicMax(&b[3], ford(vh));
-    atomicAdd(&sums[0], (double)sw);
-    atomicAdd(&sums[1], (double)sh);
-    atomicAdd(&sums[2], (double)sa);
+    if (threadIdx.x >= 9) return;
+    const int q = threadIdx.x;
+    float x = red[q][0];
+    for (int w = 1; w < 8; ++w) x = q < 6 ? fminf(x, red[q][w]) : x + red[q][w];
+    if (q >= 6) atomicAdd(&sums[q - 6], (double)x);
+    else if (q & 1) atomicMax(&b[q], ford(-x));
+    else atomicMin(&b[q], ford(x));
 }
 
 // Counts (FILL false) or lists (FILL true, count holding each cell's length) the cells that
@@ -215,19 +210,29 @@ __global__ void k_cg_bounds(const float4* __restrict__ tris, int n, int* __restr
 // takes its slots from the cell's end, and the counts are back at zero after it.
 template <int AXIS, bool FILL>
 __global__ void __launch_bounds__(256) k_cg_cells(const float4* __restrict__ tris, int n, GridView g,
-                                                  uint32_t* __restrict__ count, uint32_t* __restrict__ list) {
+                                                  uint32_t* __restrict__ count, uint2* __restrict__ list) {
     const int lane = threadIdx.x & 31;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t cells = 0, first = 0, width = 1;
+    uint32_t cells = 0, width = 1;
+    int cu0 = 0, cv0 = 0;
+    float ful = 0.0f, fuh = 0.0f, fvl = 0.0f, fvh = 0.0f;  // the box in cell units
+    uint32_t high = 0;
     if (k < n) {
-        float ul, uh, vl, vh;
-        tri_uv_box<AXIS>(tris, k, ul, uh, vl, vh);
-        const int cu0 = cell_of(ul, g.u0, g.su, g.gu), cu1 = cell_of(uh, g.u0, g.su, g.gu);
-        const int cv0 = cell_of(vl, g.v0, g.sv, g.gv), cv1 = cell_of(vh, g.v0, g.sv, g.gv);
+        const TriBox t = tri_box<AXIS>(tris, k);
+        const int cu1 = cell_of(t.uh, g.u0, g.su, g.gu), cv1 = cell_of(t.vh, g.v0, g.sv, g.gv);
+        cu0 = cell_of(t.ul, g.u0, g.su, g.gu);
+        cv0 = cell_of(t.vl, g.v0, g.sv, g.gv);
         if (cu1 >= cu0 && cv1 >= cv0) {
             width = (uint32_t)(cu1 - cu0 + 1);
             cells = width * (uint32_t)(cv1 - cv0 + 1);
-            first = (uint32_t)(cv0 * g.gu + cu0);
+        }
+        if (FILL) {
+            // A triangle with a coordinate that is not a number covers its cells whole.
+            ful = t.nan ? -INFINITY : cell_units(t.ul, g.u0, g.su);
+            fuh = t.nan ? INFINITY : cell_units(t.uh, g.u0, g.su);
+            fvl = t.nan ? -INFINITY : cell_units(t.vl, g.v0, g.sv);
+            fvh = t.nan ? INFINITY : cell_units(t.vh, g.v0, g.sv);
+            high = t.nan ? 255u : height_units(g, t.wh);
         }
     }
     uint32_t inc = cells;  // 32 rectangles of at most 2^26 cells fit
@@ -245,14 +250,23 @@ __global__ void __launch_bounds__(256) k_cg_cells(const float4* __restrict__ tri
             const uint32_t pc = __shfl_sync(0xffffffffu, pre, owner + step);
             if (pc <= j) owner += step;
         }
-        const uint32_t of = __shfl_sync(0xffffffffu, first, owner), ow = __shfl_sync(0xffffffffu, width, owner);
-        const uint32_t op = __shfl_sync(0xffffffffu, pre, owner);
+        const int ou = __shfl_sync(0xffffffffu, cu0, owner), ov = __shfl_sync(0xffffffffu, cv0, owner);
+        const uint32_t ow = __shfl_sync(0xffffffffu, width, owner), op = __shfl_sync(0xffffffffu, pre, owner);
+        const uint32_t r = j - op, row = r / ow;
+        const int cu = ou + (int)(r - row * ow), cv = ov + (int)row;
+        const size_t c = (size_t)cv * g.gu + cu;
+        if (!FILL) {
+            if (j < total) atomicAdd(&count[c], 1u);
+            continue;
+        }
         const int ok = __shfl_sync(0xffffffffu, k, owner);
+        const float a0 = __shfl_sync(0xffffffffu, ful, owner), a1 = __shfl_sync(0xffffffffu, fuh, owner);
+        const float a2 = __shfl_sync(0xffffffffu, fvl, owner), a3 = __shfl_sync(0xffffffffu, fvh, owner);
+        const uint32_t oh = __shfl_sync(0xffffffffu, high, owner);
         if (j < total) {
-            const uint32_t r = (uint32_t)(j - op), row = r / ow;
-            const uint32_t c = of + row * (uint32_t)g.gu + (r - row * ow);
-            if (FILL) list[g.start[c] + atomicSub(&count[c], 1u) - 1u] = (uint32_t)ok;
-            else atomicAdd(&count[c], 1u);
+            const uint32_t y = unit_in_cell(a0, cu) | unit_in_cell(a1, cu) << 6 | unit_in_cell(a2, cv) << 12 |
+                               unit_in_cell(a3, cv) << 18 | oh << 24;
+            list[g.start[c] + atomicSub(&count[c], 1u) - 1u] = make_uint2((uint32_t)ok, y);
         }
     }
 }
@@ -292,18 +306,18 @@ template <int AXIS>
 cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
     rs_column_grid& cg = bvh->cgrid[AXIS];
     const int n = (int)bvh->n_tris;
-    int* b = nullptr;  // four ordered ints, then three sums
-    constexpr size_t kBytes = 4 * sizeof(int) + 3 * sizeof(double);
+    int* b = nullptr;  // six ordered ints, then three sums
+    constexpr size_t kBytes = 6 * sizeof(int) + 3 * sizeof(double);
     cudaError_t e = dmalloc((void**)&b, kBytes, s);
     if (e != cudaSuccess) return e;
     struct {
-        int b[4] = {0x7fffffff, (int)0x80000000, 0x7fffffff, (int)0x80000000};
+        int b[6] = {0x7fffffff, (int)0x80000000, 0x7fffffff, (int)0x80000000, 0x7fffffff, (int)0x80000000};
         double sum[3] = {0.0, 0.0, 0.0};
     } h;
     static_assert(sizeof(h) == kBytes, "bounds layout");
     cudaMemcpyAsync(b, &h, kBytes, cudaMemcpyHostToDevice, s);
     launch(k_cg_bounds<AXIS>, std::min(2 * sm_count(), (n + 255) / 256), 256, 0, s, (const float4*)bvh->tris, n, b,
-           reinterpret_cast<double*>(b + 4));
+           reinterpret_cast<double*>(b + 6));
     e = cudaMemcpyAsync(&h, b, kBytes, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     cudaFreeAsync(b, s);
@@ -312,6 +326,10 @@ cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
     cg.u1 = dec_ord(h.b[1]);
     cg.v0 = dec_ord(h.b[2]);
     cg.v1 = dec_ord(h.b[3]);
+    cg.w0 = dec_ord(h.b[4]);
+    cg.w1 = dec_ord(h.b[5]);
+    const double depth = (double)cg.w1 - cg.w0;
+    cg.sw = depth > 0 ? (float)(256.0 / depth) : 0.0f;
     const double w = (double)cg.u1 - cg.u0, hh = (double)cg.v1 - cg.v0;
     const double target = grid_cells(n, w, hh, h.sum);
     int gu = 1, gv = 1;
@@ -333,15 +351,15 @@ cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
     e = dmalloc((void**)&count, ncell * sizeof(uint32_t), s);
     if (e == cudaSuccess) e = dmalloc((void**)&cg.start, (ncell + 1) * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    GridView gvw{cg.u0, cg.v0, cg.su, cg.sv, cg.u1, cg.v1, gu, gv, cg.start, nullptr};
+    const GridView gvw = grid_view(cg);
     cudaMemsetAsync(count, 0, ncell * sizeof(uint32_t), s);
     const unsigned grid = (unsigned)((n + 255) / 256);
-    launch(k_cg_cells<AXIS, false>, grid, 256, 0, s, (const float4*)bvh->tris, n, gvw, count, (uint32_t*)nullptr);
+    launch(k_cg_cells<AXIS, false>, grid, 256, 0, s, (const float4*)bvh->tris, n, gvw, count, (uint2*)nullptr);
     e = exclusive_scan_u32(count, cg.start, ncell, cg.start + ncell, s);
     uint32_t total = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&total, cg.start + ncell, sizeof(total), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess) e = dmalloc((void**)&cg.list, (size_t)std::max<uint32_t>(total, 1) * 4, s);
+    if (e == cudaSuccess) e = dmalloc((void**)&cg.list, (size_t)std::max<uint32_t>(total, 1) * sizeof(uint2), s);
     if (e == cudaSuccess) {
         launch(k_cg_cells<AXIS, true>, grid, 256, 0, s, (const float4*)bvh->tris, n, gvw, count, cg.list);
         e = cudaGetLastError();
@@ -355,26 +373,64 @@ cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
 
 template <int AXIS, bool FILTER>
 cudaError_t launch_pim(const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz,
-                       const float* box, int32_t* obj, uint8_t* in, unsigned int* status, uint32_t* ovf_list,
+                       const float* box, int32_t* obj, uint8_t* in, uint32_t* ovf_list,
                        unsigned long long* ovf_count, cudaStream_t s) {
-    const unsigned grid = (unsigned)((n + kT - 1) / kT);
     constexpr int GA = AXIS < 0 ? 0 : AXIS;
     const int ptok = prof_begin(P_PIM, s);
     if (AXIS >= 0 && bvh->cgrid[GA].built) {
-        const rs_column_grid& cg = bvh->cgrid[GA];
-        GridView g{cg.u0, cg.v0, cg.su, cg.sv, cg.u1, cg.v1, cg.gu, cg.gv, cg.start, cg.list};
-        launch(k_pim_grid<GA, FILTER>, grid, kT, 0, s, pts, n, g, (const float4*)bvh->tris, box, obj, in, ovf_list,
+        const GridView g = grid_view(bvh->cgrid[GA]);
+        launch(k_pim_grid<GA, FILTER>, (unsigned)((n + kT - 1) / kT), kT, 0, s, pts, n, g, (const float4*)bvh->tris, box, obj, in, ovf_list,
                ovf_count);
     } else {
-        launch(k_pim<AXIS, FILTER>, grid, kT, 0, s, pts, n, dx, dy, dz, bvh->nodes, max_steps(bvh),
-               (const float4*)bvh->tris, box, obj, in, status, ovf_list, ovf_count);
+        launch(k_pim<AXIS, FILTER>, (unsigned)((n + kPimT - 1) / kPimT), kPimT, 0, s, pts, n, dx, dy, dz, bvh->nodes,
+               max_steps(bvh), (const float4*)bvh->tris, box, obj, in, ovf_list, ovf_count);
     }
     prof_end(P_PIM, s, ptok);
-    // One thread per possible overflow entry (the count is only known on the device);
-    // threads past it return at once.
-    launch(k_pim_fallback<AXIS>, (unsigned)((n + kT - 1) / kT), kT, 0, s, pts, dx, dy, dz, bvh->nodes, max_steps(bvh),
-           (const float4*)bvh->tris, obj, in, status, ovf_list, ovf_count);
     return cudaGetLastError();
+}
+
+// Launches the query, waits for it, and resolves the rays it left in ovf_list (their count
+// is known then, so a query without any pays for no second launch).  meta: status word,
+// overflow count, both zero before the call.
+template <int AXIS>
+int run_pim_axis(const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz, bool filter,
+                 const float* box, int32_t* obj, uint8_t* in, unsigned long long* meta, uint32_t* ovf,
+                 cudaStream_t s) {
+    unsigned int* status = reinterpret_cast<unsigned int*>(meta);
+    cudaError_t e = filter ? launch_pim<AXIS, true>(bvh, pts, n, dx, dy, dz, box, obj, in, ovf, meta + 1, s)
+                           : launch_pim<AXIS, false>(bvh, pts, n, dx, dy, dz, box, obj, in, ovf, meta + 1, s);
+    unsigned long long h[2] = {0, 0};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, meta, sizeof(h), cudaMemcpyDeviceToHost, s);
+    cudaError_t e2 = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess && h[1]) {
+        launch(k_pim_fallback<AXIS>, (unsigned)((h[1] + kT - 1) / kT), kT, 0, s, pts, dx, dy, dz, bvh->nodes,
+               max_steps(bvh), (const float4*)bvh->tris, obj, in, status, (const uint32_t*)ovf,
+               (const unsigned long long*)(meta + 1));
+        e = cudaMemcpyAsync(h, meta, sizeof(h), cudaMemcpyDeviceToHost, s);
+        e2 = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = e2;
+    }
+    prof_collect();
+    return e == cudaSuccess ? status_from_bits((uint32_t)h[0]) : to_status(e);
+}
+
+int pim_axis(float dx, float dy, float dz) {
+    const bool zx = dx == 0.0f, zy = dy == 0.0f, zz = dz == 0.0f;
+    if (dz == 1.0f && zx && zy) return 2;
+    if (dx == 1.0f && zy && zz) return 0;
+    if (dy == 1.0f && zx && zz) return 1;
+    return -1;
+}
+
+int run_pim(int axis, const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz, bool filter,
+            const float* box, int32_t* obj, uint8_t* in, unsigned long long* meta, uint32_t* ovf, cudaStream_t s) {
+    switch (axis) {
+        case 0: return run_pim_axis<0>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, ovf, s);
+        case 1: return run_pim_axis<1>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, ovf, s);
+        case 2: return run_pim_axis<2>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, ovf, s);
+        default: return run_pim_axis<-1>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, ovf, s);
+    }
 }
 
 BoxMesh make_box(const rs_bvh* bvh) {
@@ -409,11 +465,7 @@ int pim_impl(const rs_bvh* cbvh, const float* pts, uint64_t n, float dx, float d
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         return to_status(e);
     }
-    const bool zx = dx == 0.0f, zy = dy == 0.0f, zz = dz == 0.0f;
-    int axis = -1;
-    if (dz == 1.0f && zx && zy) axis = 2;
-    else if (dx == 1.0f && zy && zz) axis = 0;
-    else if (dy == 1.0f && zx && zz) axis = 1;
+    const int axis = pim_axis(dx, dy, dz);
     if (axis >= 0) {
         st = ensure_grid(bvh, axis, s);
         if (st != RS_OK) return st;
@@ -428,33 +480,14 @@ int pim_impl(const rs_bvh* cbvh, const float* pts, uint64_t n, float dx, float d
         return to_status(e);
     }
     cudaMemsetAsync(meta, 0, 2 * sizeof(unsigned long long), s);
-    unsigned int* status = reinterpret_cast<unsigned int*>(meta);
     static_assert(sizeof(BoxMesh) == 108 * sizeof(float), "box mesh layout");
     BoxMesh hbox = filter ? make_box(bvh) : BoxMesh{};
     float* box = reinterpret_cast<float*>(meta + 2);
     if (filter) cudaMemcpyAsync(box, &hbox, sizeof(BoxMesh), cudaMemcpyHostToDevice, s);
-    if (axis == 2) {
-        e = filter ? launch_pim<2, true>(bvh, pts, n, dx, dy, dz, box, obj, in, status, ovf, meta + 1, s)
-                   : launch_pim<2, false>(bvh, pts, n, dx, dy, dz, box, obj, in, status, ovf, meta + 1, s);
-    } else if (axis == 0) {
-        e = filter ? launch_pim<0, true>(bvh, pts, n, dx, dy, dz, box, obj, in, status, ovf, meta + 1, s)
-                   : launch_pim<0, false>(bvh, pts, n, dx, dy, dz, box, obj, in, status, ovf, meta + 1, s);
-    } else if (axis == 1) {
-        e = filter ? launch_pim<1, true>(bvh, pts, n, dx, dy, dz, box, obj, in, status, ovf, meta + 1, s)
-                   : launch_pim<1, false>(bvh, pts, n, dx, dy, dz, box, obj, in, status, ovf, meta + 1, s);
-    } else {
-        e = filter ? launch_pim<-1, true>(bvh, pts, n, dx, dy, dz, box, obj, in, status, ovf, meta + 1, s)
-                   : launch_pim<-1, false>(bvh, pts, n, dx, dy, dz, box, obj, in, status, ovf, meta + 1, s);
-    }
-    unsigned long long hmeta[2] = {0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hmeta, meta, sizeof(hmeta), cudaMemcpyDeviceToHost, s);
+    st = run_pim(axis, bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, ovf, s);
     cudaFreeAsync(meta, s);
     cudaFreeAsync(ovf, s);
-    cudaError_t e2 = cudaStreamSynchronize(s);
-    prof_collect();
-    if (e == cudaSuccess) e = e2;
-    if (e != cudaSuccess) return to_status(e);
-    return status_from_bits((uint32_t)hmeta[0]);
+    return st;
 }
 
 __global__ void k_hit_flags(const int32_t* __restrict__ obj, uint64_t n, uint32_t* __restrict__ flags) {
@@ -572,31 +605,10 @@ extern "C" int rs_pim_noalloc(const rs_bvh* bvh, const float* d_points, uint64_t
         e = cudaMemcpyAsync(box, &hbox, sizeof(BoxMesh), cudaMemcpyHostToDevice, s);
         if (e != cudaSuccess) return to_status(e);
     }
-    unsigned int* status = reinterpret_cast<unsigned int*>(meta);
-    const bool zx = dx == 0.0f, zy = dy == 0.0f, zz = dz == 0.0f;
     // The column grid is used when it already exists; it is never built here, because
     // building it allocates.  Without it the BVH path gives the same results.
-    const bool f = filtered != 0;
-    if (dz == 1.0f && zx && zy) {
-        e = f ? launch_pim<2, true>(bvh, d_points, n, dx, dy, dz, box, d_obj, d_inside, status, ovf, meta + 1, s)
-              : launch_pim<2, false>(bvh, d_points, n, dx, dy, dz, box, d_obj, d_inside, status, ovf, meta + 1, s);
-    } else if (dx == 1.0f && zy && zz) {
-        e = f ? launch_pim<0, true>(bvh, d_points, n, dx, dy, dz, box, d_obj, d_inside, status, ovf, meta + 1, s)
-              : launch_pim<0, false>(bvh, d_points, n, dx, dy, dz, box, d_obj, d_inside, status, ovf, meta + 1, s);
-    } else if (dy == 1.0f && zx && zz) {
-        e = f ? launch_pim<1, true>(bvh, d_points, n, dx, dy, dz, box, d_obj, d_inside, status, ovf, meta + 1, s)
-              : launch_pim<1, false>(bvh, d_points, n, dx, dy, dz, box, d_obj, d_inside, status, ovf, meta + 1, s);
-    } else {
-        e = f ? launch_pim<-1, true>(bvh, d_points, n, dx, dy, dz, box, d_obj, d_inside, status, ovf, meta + 1, s)
-              : launch_pim<-1, false>(bvh, d_points, n, dx, dy, dz, box, d_obj, d_inside, status, ovf, meta + 1, s);
-    }
-    unsigned long long hmeta[2] = {0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hmeta, meta, sizeof(hmeta), cudaMemcpyDeviceToHost, s);
-    cudaError_t e2 = cudaStreamSynchronize(s);
-    prof_collect();
-    if (e == cudaSuccess) e = e2;
-    if (e != cudaSuccess) return to_status(e);
-    return status_from_bits((uint32_t)hmeta[0]);
+    return run_pim(pim_axis(dx, dy, dz), bvh, d_points, n, dx, dy, dz, filtered != 0, box, d_obj, d_inside, meta, ovf,
+                   s);
 }
 
 extern "C" int rs_pim(const rs_bvh* bvh, const float* d_points, uint64_t n, float dx, float dy, float dz,

@@ -4,6 +4,7 @@
 #include <climits>
 
 #include "rs_device.cuh"
+#include "rs_engine.h"
 
 namespace rs {
 namespace {
@@ -114,6 +115,14 @@ struct HitList {
             }
         }
     }
+    // finish() of a list of at most two.
+    __device__ __forceinline__ Chain finish2() const {
+        Chain c;
+        const bool swap = n == 2 && hit_less(t[1], id[1], t[0], id[0]);
+        if (n >= 1) c.step(swap ? t[1] : t[0], swap ? obj[1] : obj[0]);
+        if (n == 2) c.step(swap ? t[0] : t[1], swap ? obj[0] : obj[1]);
+        return c;
+    }
     __device__ __forceinline__ Chain finish() {
         sort();
         Chain c;
@@ -131,127 +140,288 @@ __device__ __forceinline__ void write_result(const Chain& ch, uint64_t i, int32_
     if (out_in) out_in[i] = inside ? 1 : 0;
 }
 
+// Column grid of +e_AXIS rays: cells over the two other axes (u, v), each listing the
+// triangles whose projected box touches it.  A list entry is 8 bytes: x = the leaf-ordered
+// triangle, y = its box in the cell's own units, rounded outwards -- bits 0-5 and 6-11 the
+// u range in 64ths of the cell, 12-17 and 18-23 the v range, 24-31 its highest point along
+// the ray axis in 256ths of the mesh's extent.  The same monotone formulas give a query
+// point's cell and units, so an entry whose ranges miss the point's units, or whose highest
+// point lies below them, is a triangle that the ray cannot cross.
 struct GridView {
     float u0, v0, su, sv, u1, v1;
+    float w0, sw, w1;
     int gu, gv;
     const uint32_t* start;
-    const uint32_t* list;
+    const uint2* list;
 };
+
+inline GridView grid_view(const rs_column_grid& c) {
+    return GridView{c.u0, c.v0, c.su, c.sv, c.u1, c.v1, c.w0, c.sw, c.w1, c.gu, c.gv, c.start, c.list};
+}
+
+__device__ __forceinline__ float cell_units(float x, float x0, float s) { return __fmul_rn(__fsub_rn(x, x0), s); }
 
 // Monotone cell index: identical for triangle boxes and query points.
 __device__ __forceinline__ int cell_of(float x, float x0, float s, int g) {
-    float f = floorf(__fmul_rn(__fsub_rn(x, x0), s));
+    float f = floorf(cell_units(x, x0, s));
     f = fminf(fmaxf(f, 0.0f), (float)(g - 1));
     return (int)f;
 }
 
-// Candidates of a point from the column grid of the +e_AXIS direction (a crossed
-// triangle's projected box contains the point; all boxes lie in [u0,u1]x[v0,v1]).
+// 64ths within cell c of a coordinate whose cell_units are f: monotone in f, clamped to the
+// cell.  f - c is exact for f inside the cell.
+__device__ __forceinline__ uint32_t unit_in_cell(float f, int c) {
+    return (uint32_t)fminf(fmaxf(__fmul_rn(__fsub_rn(f, (float)c), 64.0f), 0.0f), 63.0f);
+}
+
+__device__ __forceinline__ uint32_t height_units(const GridView& g, float w) {
+    return (uint32_t)fminf(fmaxf(cell_units(w, g.w0, g.sw), 0.0f), 255.0f);
+}
+
+__device__ __forceinline__ bool entry_may_hit(uint32_t e, uint32_t pu, uint32_t pv, uint32_t pw) {
+    return (e & 63u) <= pu && ((e >> 6) & 63u) >= pu && ((e >> 12) & 63u) <= pv && ((e >> 18) & 63u) >= pv &&
+           (e >> 24) >= pw;
+}
+
+// A point's cell list and its units (u | v << 8 | w << 16).
 template <int AXIS>
-__device__ __forceinline__ void grid_cell(const GridView& g, const float* p, uint32_t& begin, uint32_t& count) {
+__device__ __forceinline__ void grid_cell(const GridView& g, const float* p, uint32_t& begin, uint32_t& count,
+                                          uint32_t& units) {
     constexpr int U = (AXIS + 1) % 3, V = (AXIS + 2) % 3;
     begin = 0;
     count = 0;
-    if (p[U] >= g.u0 && p[U] <= g.u1 && p[V] >= g.v0 && p[V] <= g.v1) {
-        const int c = cell_of(p[V], g.v0, g.sv, g.gv) * g.gu + cell_of(p[U], g.u0, g.su, g.gu);
+    units = 0;
+    // A crossed triangle's box contains the point in u and v, and no triangle lies above w1.
+    if (p[U] >= g.u0 && p[U] <= g.u1 && p[V] >= g.v0 && p[V] <= g.v1 && !(p[AXIS] > g.w1)) {
+        const int cu = cell_of(p[U], g.u0, g.su, g.gu), cv = cell_of(p[V], g.v0, g.sv, g.gv);
+        const int c = cv * g.gu + cu;
         begin = __ldg(&g.start[c]);
         count = __ldg(&g.start[c + 1]) - begin;
+        units = unit_in_cell(cell_units(p[U], g.u0, g.su), cu) | unit_in_cell(cell_units(p[V], g.v0, g.sv), cv) << 8 |
+                height_units(g, p[AXIS]) << 16;
     }
 }
 
-// Shared-memory crossing slots of one warp for pim_grid_warp.
+// One warp's shared memory for pim_grid_warp: crossing slots (kHits a point, or 32 * kHits of
+// one point), the points, the work lists' owners and a ring of candidates to test.
 struct GridWarpSlots {
     float t[kHits][32];
     uint32_t id[kHits][32];
     int32_t obj[kHits][32];
     int n[32];
+    float p[3][32];
+    uint4 rec[32];      // of the k-th point with candidates: list offset, units, lane
+    uint2 ring[64];     // triangle, lane of its point
 };
+constexpr int kDenseHits = 32 * kHits;
+// Candidates a point from which a warp takes its points one at a time: the lists then fill
+// whole rounds by themselves, and rays through that many boxes often cross more than kHits
+// triangles.
+constexpr uint32_t kDenseCandidates = 48;
+
+// The advance rule on nh crossings that a warp holds, by repeated minima: the next counted
+// crossing is the nearest at or beyond the threshold.  Distances are positive, so their bits
+// order like them.  The same Chain in every lane.
+__device__ __forceinline__ Chain dense_chain(const float* ht, const uint32_t* hid, const int32_t* hobj, int nh,
+                                             int lane) {
+    Chain ch;
+    for (;;) {
+        uint32_t best = 0xffffffffu;
+        for (int h = lane; h < nh; h += 32) {
+            const float t = ht[h];
+            if (t >= ch.thr && t < kTmax) best = min(best, __float_as_uint(t));
+        }
+        best = __reduce_min_sync(0xffffffffu, best);
+        if (best == 0xffffffffu) return ch;
+        const float t = __uint_as_float(best);
+        int32_t obj = -1;
+        if (ch.count == 0) {  // the object of the smallest id at that distance
+            uint32_t low = 0xffffffffu;
+            for (int h = lane; h < nh; h += 32)
+                if (ht[h] == t && hid[h] <= low) {
+                    low = hid[h];
+                    obj = hobj[h];
+                }
+            const uint32_t lowest = __reduce_min_sync(0xffffffffu, low);
+            obj = __shfl_sync(0xffffffffu, obj, __ffs(__ballot_sync(0xffffffffu, low == lowest)) - 1);
+        }
+        ch.step(t, obj);
+        if (ch.count == kPimMaxIters) return ch;
+    }
+}
 
 // Warp-cooperative column-grid query of the warp's 32 points (all lanes call it; lanes
 // without a point pass valid = false, lanes whose point was filtered out keep = false).
-// The candidate lists are flattened into one (point, triangle) work list with a warp
-// scan, so every lane tests one candidate per round however unevenly candidates are
-// spread over the points.  Crossings go to per-point slots in shared memory; each lane
-// then sorts and counts its own point's, or calls overflow() when it has more than
-// kHits of them.
+// Bound by instruction issue, so the work is cut rather than the bytes: of the 5 candidates
+// that a point of the level-4 sphere finds in its cell, 1.5 pass the 8-byte entry's ranges,
+// and only those are loaded and tested exactly.
+//  * The cells' lists are flattened into one work list, 32 entries a round; the owner of an
+//    entry follows from one OR-reduction of the round's list heads.  Entries that pass are
+//    queued in a ring and tested 32 at a time, every lane with a triangle.  Crossings go to
+//    the points' slots, and each lane walks its own in (t, id) order.
+//  * A point with more than kHits crossings, and every point of a warp whose lists are long,
+//    is taken by the whole warp: up to kDenseHits crossings, walked by repeated minima.
+//    Beyond that overflow() takes the point.
 template <int AXIS, class Ovf>
 __device__ __forceinline__ void pim_grid_warp(const GridView& g, const float4* __restrict__ tris, const float* p,
                                               bool valid, bool keep, uint64_t i, int32_t* __restrict__ out_obj,
                                               uint8_t* __restrict__ out_in, GridWarpSlots& sl, Ovf&& overflow) {
+    constexpr unsigned int kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
+    const unsigned int below = (1u << lane) - 1u;
     const float dx = AXIS == 0 ? 1.0f : 0.0f, dy = AXIS == 1 ? 1.0f : 0.0f, dz = AXIS == 2 ? 1.0f : 0.0f;
-    uint32_t b = 0, cnt = 0;
-    if (keep) grid_cell<AXIS>(g, p, b, cnt);
-    sl.n[lane] = 0;
-    // Warp exclusive scan of the candidate counts.
-    uint32_t inc = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    const uint32_t pre = inc - cnt;
-    const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
-    __syncwarp();
-    add_tests(lane == 0 ? total : 0u);
-    for (uint32_t base = 0; base < total; base += 32) {
-        const uint32_t j = base + lane;
-        // Owner of work item j: the last lane whose prefix is <= j.
-        int owner = 0;
-#pragma unroll
-        for (int step = 16; step >= 1; step >>= 1) {
-            const uint32_t pc = __shfl_sync(0xffffffffu, pre, owner + step);
-            if (pc <= j) owner += step;
-        }
-        const uint32_t ob = __shfl_sync(0xffffffffu, b, owner);
-        const uint32_t opre = __shfl_sync(0xffffffffu, pre, owner);
-        const float ox = __shfl_sync(0xffffffffu, p[0], owner);
-        const float oy = __shfl_sync(0xffffffffu, p[1], owner);
-        const float oz = __shfl_sync(0xffffffffu, p[2], owner);
-        if (j < total) {
-            const int k = (int)__ldg(&g.list[ob + (j - opre)]);
-            float a[3], bb[3], cc[3];
-            uint32_t tid;
-            int32_t obj;
-            load_tri(tris, k, a, bb, cc, tid, obj);
-            const Ray r = make_ray(ox, oy, oz, dx, dy, dz, kEps, kTmax);
-            float t;
-            if (hit_triangle<AXIS>(r, a, bb, cc, t)) {
-                const int slot = atomicAdd(&sl.n[owner], 1);
-                if (slot < kHits) {
-                    sl.t[slot][owner] = t;
-                    sl.id[slot][owner] = tid;
-                    sl.obj[slot][owner] = obj;
-                }
-            }
-        }
-    }
-    __syncwarp();
-    if (!valid) return;
-    const int nh = sl.n[lane];
-    if (nh > kHits) {
-        overflow();
+    uint32_t b = 0, cnt = 0, units = 0;
+    if (keep) grid_cell<AXIS>(g, p, b, cnt, units);
+    const unsigned int listed = __ballot_sync(kAll, cnt != 0);
+    if (listed == 0) {
+        if (valid) write_result(Chain{}, i, out_obj, out_in);
         return;
     }
-    HitList hl;
+    uint32_t inc = cnt;  // warp prefix sum of the candidate counts
 #pragma unroll
-    for (int q = 0; q < kHits; ++q)
-        if (q < nh) {
-            hl.t[q] = sl.t[q][lane];
-            hl.id[q] = sl.id[q][lane];
-            hl.obj[q] = sl.obj[q][lane];
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kAll, inc, o);
+        if (lane >= o) inc += y;
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) sl.p[q][lane] = p[q];
+    sl.n[lane] = 0;
+    float* ht = &sl.t[0][0];
+    uint32_t* hid = &sl.id[0][0];
+    int32_t* hobj = &sl.obj[0][0];
+    uint32_t tests = 0;
+    // First all points at once (owner -1), unless their lists are long, then the points that
+    // the whole warp takes, one by one.
+    uint32_t total = __shfl_sync(kAll, inc, 31);
+    uint32_t start = cnt ? inc - cnt : ~0u;  // where this lane's list starts in the work list
+    unsigned int dense = 0;
+    int owner = -1;
+    if (cnt) sl.rec[__popc(listed & below)] = make_uint4(b - start, units, (uint32_t)lane, 0u);
+    if (total >= 32u * kDenseCandidates) {
+        dense = listed;
+        if (valid && cnt == 0) write_result(Chain{}, i, out_obj, out_in);
+        total = 0;
+    }
+    __syncwarp();
+    for (;;) {
+        uint32_t head = 0, queued = 0, owners = 0;
+        for (uint32_t base = 0; base < total || queued; base += 32) {
+            if (base < total) {
+                const uint32_t j = base + lane;
+                // Bit q of heads: a list starts at entry base + q.
+                const unsigned int heads = __reduce_or_sync(kAll, start - base < 32u ? 1u << (start - base) : 0u);
+                const uint4 rec = sl.rec[owners + __popc(heads & (below | 1u << lane)) - 1u];
+                owners += __popc(heads);
+                uint2 e = make_uint2(0u, 0u);
+                bool pass = false;
+                if (j < total) {
+                    e = __ldg(&g.list[rec.x + j]);
+                    pass = entry_may_hit(e.y, rec.y & 255u, (rec.y >> 8) & 255u, rec.y >> 16);
+                }
+                const unsigned int m = __ballot_sync(kAll, pass);
+                if (pass) sl.ring[(head + queued + __popc(m & below)) & 63u] = make_uint2(e.x, rec.z);
+                queued += __popc(m);
+                __syncwarp();
+                if (queued < 32u && base + 32u < total) continue;
+            }
+            // Exact test of up to 32 queued candidates.
+            const uint32_t m = min(queued, 32u);
+            if ((uint32_t)lane < m) {
+                const uint2 e = sl.ring[(head + lane) & 63u];
+                float a[3], bb[3], cc[3];
+                uint32_t tid;
+                int32_t obj;
+                load_tri(tris, (int)e.x, a, bb, cc, tid, obj);
+                const Ray r = make_ray(sl.p[0][e.y], sl.p[1][e.y], sl.p[2][e.y], dx, dy, dz, kEps, kTmax);
+                float t;
+                if (hit_triangle<AXIS>(r, a, bb, cc, t)) {
+                    const int k = atomicAdd(&sl.n[e.y], 1);
+                    if (k < (owner < 0 ? kHits : kDenseHits)) {
+                        const int at = owner < 0 ? k * 32 + (int)e.y : k;
+                        ht[at] = t;
+                        hid[at] = tid;
+                        hobj[at] = obj;
+                    }
+                }
+            }
+            tests += m;
+            head += m;
+            queued -= m;
+            __syncwarp();
         }
-    hl.n = nh;
-    write_result(hl.finish(), i, out_obj, out_in);
+        if (owner < 0) {
+            const int nh = sl.n[lane];
+            const int most = __reduce_max_sync(kAll, nh);
+            if (total) {
+                dense = __ballot_sync(kAll, nh > kHits);
+                if (valid && nh <= kHits) {
+                    HitList hl;
+#pragma unroll
+                    for (int q = 0; q < kHits; ++q)
+                        if (q < nh) {
+                            hl.t[q] = sl.t[q][lane];
+                            hl.id[q] = sl.id[q][lane];
+                            hl.obj[q] = sl.obj[q][lane];
+                        }
+                    hl.n = nh;
+                    write_result(most <= 2 ? hl.finish2() : hl.finish(), i, out_obj, out_in);
+                }
+            }
+        } else {
+            const int nh = sl.n[owner];
+            if (nh > kDenseHits) {
+                if (lane == owner) overflow();
+            } else {
+                const Chain ch = dense_chain(ht, hid, hobj, nh, lane);
+                if (lane == owner) write_result(ch, i, out_obj, out_in);
+            }
+        }
+        if (dense == 0) break;
+        owner = __ffs(dense) - 1;
+        dense &= dense - 1;
+        total = __shfl_sync(kAll, cnt, owner);
+        start = lane == 0 ? 0u : ~0u;
+        __syncwarp();  // the slots are read: free for the next point
+        if (lane == owner) {
+            sl.rec[0] = make_uint4(b, units, (uint32_t)lane, 0u);
+            sl.n[lane] = 0;
+        }
+        __syncwarp();
+    }
+    add_tests(lane == 0 ? tests : 0u);
 }
 
-// Every crossing of ray r with t in [1e-6, 1e16] into hl (BVH traversal).  Returns false
-// on an exhausted traversal budget or stack.
+// One thread's shared-memory column for pim_column: element k of an array at base[k * stride].
+struct HitColumn {
+    int* stack;
+    float* t;
+    uint32_t* id;
+    int32_t* obj;
+    int stride;
+};
+
+// Shared memory of pim_column for T threads.
+template <int T, int STACK>
+struct HitSmem {
+    int stack[STACK][T];
+    float t[kHits][T];
+    uint32_t id[kHits][T];
+    int32_t obj[kHits][T];
+    __device__ __forceinline__ HitColumn column(int tid) {
+        return HitColumn{&stack[0][tid], &t[0][tid], &id[0][tid], &obj[0][tid], T};
+    }
+};
+
+// Crossings of ray r with t in [1e-6, 1e16] by BVH traversal, stack and up to kHits crossings
+// in the thread's shared-memory column (a register list appends through kHits predicated
+// moves, and spilled).  n receives their number, which may exceed kHits; false on an
+// exhausted traversal budget or stack.
 template <int AXIS, int STACK>
-__device__ __forceinline__ bool pim_collect(const BNode* __restrict__ nodes, uint32_t max_steps,
-                                            const float4* __restrict__ tris, const Ray& r, HitList& hl,
-                                            unsigned int& tests) {
-    return traverse<AXIS, STACK>(nodes, max_steps, r, [&](int first, int cnt) {
+__device__ __forceinline__ bool pim_column(const HitColumn& col, const BNode* __restrict__ nodes, uint32_t max_steps,
+                                           const float4* __restrict__ tris, const Ray& r, int& n) {
+    unsigned int tests = 0;
+    n = 0;
+    const bool ok = traverse_with<AXIS, STACK>(col.stack, col.stride, nodes, max_steps, r, [&](int first, int cnt) {
         tests += (unsigned int)cnt;
         for (int k = first; k < first + cnt; ++k) {
             float a[3], b[3], c[3];
@@ -259,9 +429,31 @@ __device__ __forceinline__ bool pim_collect(const BNode* __restrict__ nodes, uin
             int32_t obj;
             load_tri(tris, k, a, b, c, tid, obj);
             float t;
-            if (hit_triangle<AXIS>(r, a, b, c, t)) hl.add(t, tid, obj);
+            if (!hit_triangle<AXIS>(r, a, b, c, t)) continue;
+            if (n < kHits) {
+                col.t[n * col.stride] = t;
+                col.id[n * col.stride] = tid;
+                col.obj[n * col.stride] = obj;
+            }
+            ++n;
         }
     });
+    add_tests(tests);
+    return ok;
+}
+
+// The advance rule on the n <= kHits crossings of a column.
+__device__ __forceinline__ Chain column_chain(const HitColumn& col, int n) {
+    HitList hl;
+#pragma unroll
+    for (int q = 0; q < kHits; ++q)
+        if (q < n) {
+            hl.t[q] = col.t[q * col.stride];
+            hl.id[q] = col.id[q * col.stride];
+            hl.obj[q] = col.obj[q * col.stride];
+        }
+    hl.n = n;
+    return n <= 2 ? hl.finish2() : hl.finish();
 }
 
 // Exact fallback for a ray with more than kHits crossings: each round re-traverses the
