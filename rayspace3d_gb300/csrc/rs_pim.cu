@@ -32,20 +32,45 @@ namespace rs {
 namespace {
 
 constexpr int kT = 256;
+
+// Bounds of all vertices, and the box of 12 triangles over them that the filter's parity is
+// defined by (BoundingBox::createBoxMesh, query/src/geometry/BoundingBox.cpp:12-50): three
+// corners a triangle, bits 0, 1 and 2 of a corner choose the maximum in x, y and z.
+struct BoxBounds {
+    float mn[3], mx[3];
+    int finite;
+};
+
+__constant__ unsigned char kBoxCorners[12][3] = {{0, 3, 1}, {0, 2, 3}, {4, 5, 7}, {4, 7, 6}, {0, 1, 5}, {0, 5, 4},
+                                                 {2, 7, 3}, {2, 6, 7}, {0, 4, 6}, {0, 6, 2}, {1, 3, 7}, {1, 7, 5}};
+
+// Whether the ray's parity against the box is odd.
 template <int AXIS>
-__device__ __forceinline__ bool box_filter(const float* __restrict__ box, const Ray& r) {
+__device__ __forceinline__ bool box_filter(const BoxBounds& box, const Ray& r) {
+    if (AXIS >= 0 && box.finite && isfinite(r.o[0]) && isfinite(r.o[1]) && isfinite(r.o[2])) {
+        // In closed form (12 exact triangle tests took 80 % of a filtered query's time): the
+        // four sides project to segments, which no perturbed point is inside of, and the two
+        // triangles of an end cover its rectangle exactly once, so the ray crosses both ends
+        // when the perturbed point (moved up by delta in u, delta^2 in v) is inside it.  An
+        // end's box is flat, so its t is the rounded difference whatever its triangle.
+        constexpr int W = AXIS >= 0 ? AXIS : 0, U = (W + 1) % 3, V = (W + 2) % 3;
+        if (!(r.o[U] >= box.mn[U] && r.o[U] < box.mx[U] && r.o[V] >= box.mn[V] && r.o[V] < box.mx[V])) return false;
+        Chain ch;
+        const float t0 = __fsub_rn(box.mn[W], r.o[W]), t1 = __fsub_rn(box.mx[W], r.o[W]);
+        if (t0 >= r.tmin && t0 <= r.tmax) ch.step(t0, 0);
+        if (t1 >= r.tmin && t1 <= r.tmax) ch.step(t1, 0);
+        return (ch.count & 1) != 0;
+    }
     HitList hl;
 #pragma unroll 1
     for (int k = 0; k < 12; ++k) {
-        float a[3], b[3], c[3];
+        float v[3][3];
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            a[q] = __ldg(&box[9 * k + q]);
-            b[q] = __ldg(&box[9 * k + 3 + q]);
-            c[q] = __ldg(&box[9 * k + 6 + q]);
-        }
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) v[c][q] = (kBoxCorners[k][c] >> q) & 1 ? box.mx[q] : box.mn[q];
         float t;
-        if (hit_triangle<AXIS>(r, a, b, c, t)) hl.add(t, (uint32_t)k, 0);
+        if (hit_triangle<AXIS>(r, v[0], v[1], v[2], t)) hl.add(t, (uint32_t)k, 0);
     }
     // A ray crosses at most two of the 12 faces under the hit contract.
     const Chain ch = hl.finish();
@@ -61,7 +86,7 @@ constexpr int kPimStack = 32;
 template <int AXIS, bool FILTER>
 __global__ void __launch_bounds__(kPimT) k_pim(const float* __restrict__ pts, uint64_t n, float dx, float dy, float dz,
                                             const BNode* __restrict__ nodes, uint32_t max_steps,
-                                            const float4* __restrict__ tris, const float* __restrict__ box,
+                                            const float4* __restrict__ tris, BoxBounds box,
                                             int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
                                             uint32_t* __restrict__ ovf_list,
                                             unsigned long long* __restrict__ ovf_count) {
@@ -88,7 +113,7 @@ constexpr int kWarps = kT / 32;
 
 template <int AXIS, bool FILTER>
 __global__ void __launch_bounds__(kT, 4) k_pim_grid(const float* __restrict__ pts, uint64_t n, GridView g,
-                                                 const float4* __restrict__ tris, const float* __restrict__ box,
+                                                 const float4* __restrict__ tris, BoxBounds box,
                                                  int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
                                                  uint32_t* __restrict__ ovf_list,
                                                  unsigned long long* __restrict__ ovf_count) {
@@ -373,7 +398,7 @@ cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
 
 template <int AXIS, bool FILTER>
 cudaError_t launch_pim(const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz,
-                       const float* box, int32_t* obj, uint8_t* in, uint32_t* ovf_list,
+                       const BoxBounds& box, int32_t* obj, uint8_t* in, uint32_t* ovf_list,
                        unsigned long long* ovf_count, cudaStream_t s) {
     constexpr int GA = AXIS < 0 ? 0 : AXIS;
     const int ptok = prof_begin(P_PIM, s);
@@ -394,7 +419,7 @@ cudaError_t launch_pim(const rs_bvh* bvh, const float* pts, uint64_t n, float dx
 // overflow count, both zero before the call.
 template <int AXIS>
 int run_pim_axis(const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz, bool filter,
-                 const float* box, int32_t* obj, uint8_t* in, unsigned long long* meta, uint32_t* ovf,
+                 const BoxBounds& box, int32_t* obj, uint8_t* in, unsigned long long* meta, uint32_t* ovf,
                  cudaStream_t s) {
     unsigned int* status = reinterpret_cast<unsigned int*>(meta);
     cudaError_t e = filter ? launch_pim<AXIS, true>(bvh, pts, n, dx, dy, dz, box, obj, in, ovf, meta + 1, s)
@@ -424,7 +449,7 @@ int pim_axis(float dx, float dy, float dz) {
 }
 
 int run_pim(int axis, const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz, bool filter,
-            const float* box, int32_t* obj, uint8_t* in, unsigned long long* meta, uint32_t* ovf, cudaStream_t s) {
+            const BoxBounds& box, int32_t* obj, uint8_t* in, unsigned long long* meta, uint32_t* ovf, cudaStream_t s) {
     switch (axis) {
         case 0: return run_pim_axis<0>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, ovf, s);
         case 1: return run_pim_axis<1>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, ovf, s);
@@ -433,19 +458,14 @@ int run_pim(int axis, const rs_bvh* bvh, const float* pts, uint64_t n, float dx,
     }
 }
 
-BoxMesh make_box(const rs_bvh* bvh) {
-    // BoundingBox::createBoxMesh (query/src/geometry/BoundingBox.cpp:12-50).
-    const float* mn = bvh->vmin;
-    const float* mx = bvh->vmax;
-    const float verts[8][3] = {{mn[0], mn[1], mn[2]}, {mx[0], mn[1], mn[2]}, {mx[0], mx[1], mn[2]},
-                               {mn[0], mx[1], mn[2]}, {mn[0], mn[1], mx[2]}, {mx[0], mn[1], mx[2]},
-                               {mx[0], mx[1], mx[2]}, {mn[0], mx[1], mx[2]}};
-    const int tri[12][3] = {{0, 2, 1}, {0, 3, 2}, {4, 5, 6}, {4, 6, 7}, {0, 1, 5}, {0, 5, 4},
-                            {3, 6, 2}, {3, 7, 6}, {0, 4, 7}, {0, 7, 3}, {1, 2, 6}, {1, 6, 5}};
-    BoxMesh b;
-    for (int t = 0; t < 12; ++t)
-        for (int c = 0; c < 3; ++c)
-            for (int k = 0; k < 3; ++k) b.v[t][3 * c + k] = verts[tri[t][c]][k];
+BoxBounds make_box(const rs_bvh* bvh) {
+    BoxBounds b;
+    b.finite = 1;
+    for (int k = 0; k < 3; ++k) {
+        b.mn[k] = bvh->vmin[k];
+        b.mx[k] = bvh->vmax[k];
+        if (!std::isfinite(b.mn[k]) || !std::isfinite(b.mx[k])) b.finite = 0;
+    }
     return b;
 }
 
@@ -470,9 +490,9 @@ int pim_impl(const rs_bvh* cbvh, const float* pts, uint64_t n, float dx, float d
         st = ensure_grid(bvh, axis, s);
         if (st != RS_OK) return st;
     }
-    unsigned long long* meta = nullptr;  // [0] status, [1] overflow count, then the 12 box triangles
+    unsigned long long* meta = nullptr;  // [0] status, [1] overflow count
     uint32_t* ovf = nullptr;
-    cudaError_t e = dmalloc((void**)&meta, 2 * sizeof(unsigned long long) + sizeof(BoxMesh), s);
+    cudaError_t e = dmalloc((void**)&meta, 2 * sizeof(unsigned long long), s);
     if (e == cudaSuccess) e = dmalloc((void**)&ovf, n * sizeof(uint32_t), s);
     if (e != cudaSuccess) {
         if (meta) cudaFreeAsync(meta, s);
@@ -480,10 +500,7 @@ int pim_impl(const rs_bvh* cbvh, const float* pts, uint64_t n, float dx, float d
         return to_status(e);
     }
     cudaMemsetAsync(meta, 0, 2 * sizeof(unsigned long long), s);
-    static_assert(sizeof(BoxMesh) == 108 * sizeof(float), "box mesh layout");
-    BoxMesh hbox = filter ? make_box(bvh) : BoxMesh{};
-    float* box = reinterpret_cast<float*>(meta + 2);
-    if (filter) cudaMemcpyAsync(box, &hbox, sizeof(BoxMesh), cudaMemcpyHostToDevice, s);
+    const BoxBounds box = filter ? make_box(bvh) : BoxBounds{};
     st = run_pim(axis, bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, ovf, s);
     cudaFreeAsync(meta, s);
     cudaFreeAsync(ovf, s);
@@ -532,8 +549,8 @@ int recheck_pim(int op, unsigned long long* out) { return recheck_op(op, out); }
 // Callers that cannot allocate device memory on their query path -- services whose
 // own allocator has reserved the whole GPU, or hosts with a fixed device-memory budget
 // checked per request -- use rs_pim_noalloc.  It waits for the stream and returns once
-// the results are written.  Its per-call scratch (status word, overflow count, the twelve
-// filter-box triangles and the list of points with more than kHits crossings) lives
+// the results are written.  Its per-call scratch (status word, overflow count and the list
+// of points that the query leaves to the fallback) lives
 // in the fixed array below instead of coming from an allocator.  Host code may not
 // use the array's name as a device address, so its address is looked up with
 // cudaGetSymbolAddress once per device (with that device current) and passed to
@@ -541,7 +558,6 @@ int recheck_pim(int op, unsigned long long* out) { return recheck_op(op, out); }
 // ---------------------------------------------------------------------------
 constexpr uint64_t kNoAllocMaxPoints = 1ull << 20;  // 1,048,576 points per call
 constexpr size_t kNoAllocMetaOffset = 0;            // u64 status, u64 overflow count
-constexpr size_t kNoAllocBoxOffset = 256;           // 108 floats
 constexpr size_t kNoAllocListOffset = 1024;         // u32 per point
 constexpr size_t kNoAllocBytes = kNoAllocListOffset + kNoAllocMaxPoints * sizeof(uint32_t);
 
@@ -594,17 +610,12 @@ extern "C" int rs_pim_noalloc(const rs_bvh* bvh, const float* d_points, uint64_t
     if (e != cudaSuccess) return to_status(e);
     unsigned char* sc = static_cast<unsigned char*>(base);
     unsigned long long* meta = reinterpret_cast<unsigned long long*>(sc + kNoAllocMetaOffset);
-    float* box = reinterpret_cast<float*>(sc + kNoAllocBoxOffset);
     uint32_t* ovf = reinterpret_cast<uint32_t*>(sc + kNoAllocListOffset);
     // The array keeps the previous call's contents: the status word and overflow count
     // must start at zero (the list is written before it is read).
     e = cudaMemsetAsync(meta, 0, 2 * sizeof(unsigned long long), s);
     if (e != cudaSuccess) return to_status(e);
-    if (filtered) {
-        const BoxMesh hbox = make_box(bvh);
-        e = cudaMemcpyAsync(box, &hbox, sizeof(BoxMesh), cudaMemcpyHostToDevice, s);
-        if (e != cudaSuccess) return to_status(e);
-    }
+    const BoxBounds box = filtered ? make_box(bvh) : BoxBounds{};
     // The column grid is used when it already exists; it is never built here, because
     // building it allocates.  Without it the BVH path gives the same results.
     return run_pim(pim_axis(dx, dy, dz), bvh, d_points, n, dx, dy, dz, filtered != 0, box, d_obj, d_inside, meta, ovf,

@@ -14,10 +14,6 @@ constexpr float kEps = 1e-6f;
 constexpr float kTmax = 1e16f;
 constexpr int kFallbackIters = 1 << 16;
 
-struct BoxMesh {
-    float v[12][9];  // 12 triangles x (a,b,c)
-};
-
 __device__ __forceinline__ bool hit_less(float t0, uint32_t i0, float t1, uint32_t i1) {
     return t0 < t1 || (t0 == t1 && i0 < i1);
 }

@@ -71,6 +71,8 @@ def _points(g, n, seed):
     near = g.vertices[rng.integers(0, len(g.vertices), k)]
     pts[:k] = near  # exactly on vertices
     pts[k:2 * k] = near + rng.normal(0, 0.05, (k, 3)).astype(np.float32)
+    b0, b1 = g.vertices.min(0), g.vertices.max(0)  # on the filter box's faces, edges and corners
+    pts[-24:] = np.where(rng.random((24, 3)) < 0.4, b0, np.where(rng.random((24, 3)) < 0.6, b1, pts[-24:]))
     for j, c in enumerate((0.0, 6.0, 12.0, 20.0, 30.0)):  # inside the nested objects
         pts[2 * k + 40 * j:2 * k + 40 * (j + 1)] = c + rng.normal(0, 0.3, (40, 3))
     return pts
