@@ -701,11 +701,25 @@ __global__ void k_first_tri_init(int32_t* __restrict__ first, uint64_t nObj) {
     if (i < nObj) first[i] = INT_MAX;
 }
 
-__global__ void k_first_tri(const int32_t* __restrict__ t2o, uint64_t nF, int32_t* __restrict__ first, uint64_t nObj) {
-    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t >= nF) return;
-    const int32_t o = t2o[t];
-    if (o >= 0 && (uint64_t)o < nObj) atomicMin(&first[o], (int32_t)t);
+// The lowest triangle of every object.  Only the first triangle of a run of one object can be
+// it: with a triangle's atomic each, the 5,500 triangles an object of a 16.5 M-triangle set
+// queued on one word and took 4.5 ms; its 3,000 runs take the pass over t2o.
+constexpr int kFirstPer = 4;  // triangles a thread
+
+__global__ void __launch_bounds__(256) k_first_tri(const int32_t* __restrict__ t2o, uint64_t nF,
+                                                   int32_t* __restrict__ first, uint64_t nObj) {
+    const uint64_t base = blockIdx.x * (uint64_t)(256 * kFirstPer) + threadIdx.x;
+    int32_t o[kFirstPer], before[kFirstPer];
+#pragma unroll
+    for (int k = 0; k < kFirstPer; ++k) {
+        const uint64_t t = base + 256 * (uint64_t)k;
+        o[k] = t < nF ? __ldg(&t2o[t]) : -1;
+        before[k] = t < nF && t > 0 ? __ldg(&t2o[t - 1]) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < kFirstPer; ++k)
+        if (o[k] >= 0 && o[k] != before[k] && (uint64_t)o[k] < nObj)
+            atomicMin(&first[o[k]], (int32_t)(base + 256 * (uint64_t)k));
 }
 
 __global__ void k_max_obj(const int32_t* __restrict__ t2o, uint64_t nF, int* __restrict__ mx) {
@@ -1019,28 +1033,28 @@ struct Tracking {
     uint32_t* candidates;     // [nObj]
 };
 
-template <bool TRACK>
-__global__ void __launch_bounds__(kT) k_containment(const float* __restrict__ V, uint64_t nV,
-                                                    const uint32_t* __restrict__ I,
-                                                    const int32_t* __restrict__ first, uint64_t nObj,
-                                                    const BNode* __restrict__ nodes, uint32_t max_steps,
-                                                    const float4* __restrict__ tris, int swap, PairTable table,
-                                                    Tracking trk) {
-    const uint64_t o = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (o >= nObj) return;
-    if (TRACK) {
-        trk.candidates[o] = 0;
-        for (int q = 0; q < trk.max_targets; ++q) {
-            trk.target_ids[o * trk.max_targets + q] = -1;
-            trk.target_hits[o * trk.max_targets + q] = 0;
-        }
-    }
+// The ray of source object o; false when it has none.
+__device__ __forceinline__ bool containment_ray(const float* __restrict__ V, uint64_t nV,
+                                                const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
+                                                uint64_t o, Ray& r) {
     const int32_t ft = first[o];
-    if (ft == INT_MAX) return;
+    if (ft == INT_MAX) return false;
     const uint32_t vi = I[3 * (uint64_t)ft];
-    if (vi >= nV) return;
-    const Ray r = make_ray(V[3 * (uint64_t)vi], V[3 * (uint64_t)vi + 1], V[3 * (uint64_t)vi + 2], 0.0f, 0.0f, 1.0f,
-                           1e-4f, 1e10f);
+    if (vi >= nV) return false;
+    r = make_ray(V[3 * (uint64_t)vi], V[3 * (uint64_t)vi + 1], V[3 * (uint64_t)vi + 2], 0.0f, 0.0f, 1.0f, 1e-4f, 1e10f);
+    return true;
+}
+
+__device__ __forceinline__ unsigned long long containment_key(uint64_t o, uint32_t target, int swap) {
+    return swap ? (((unsigned long long)target << 32) | (uint32_t)o)
+                : (((unsigned long long)(uint32_t)o << 32) | target);
+}
+
+// One object's ray by one thread, any number of targets.
+template <bool TRACK>
+__device__ __forceinline__ void containment_thread(const Ray& r, uint64_t o, const BNode* __restrict__ nodes,
+                                                   uint32_t max_steps, const float4* __restrict__ tris, int swap,
+                                                   const PairTable& table, const Tracking& trk) {
     // Parity per target object in passes of at most kTargets objects: pass p tracks the
     // kTargets smallest object ids (as uint32) above the largest id of pass p-1.  A list
     // member is inserted at its first crossing and never evicted (evictions only drop the
@@ -1106,9 +1120,7 @@ __global__ void __launch_bounds__(kT) k_containment(const float* __restrict__ V,
         for (int j = 0; j < nt; ++j) {
             mx = max(mx, tgt[j]);
             if (!((par >> j) & 1u)) continue;
-            const unsigned long long key = swap ? (((unsigned long long)tgt[j] << 32) | (uint32_t)o)
-                                                : (((unsigned long long)(uint32_t)o << 32) | tgt[j]);
-            table_insert(table, key);
+            table_insert(table, containment_key(o, tgt[j], swap));
             if (TRACK && out < trk.max_targets) {
                 trk.target_ids[o * trk.max_targets + out] = (int32_t)tgt[j];
                 trk.target_hits[o * trk.max_targets + out] = hits[j];
@@ -1126,6 +1138,140 @@ __global__ void __launch_bounds__(kT) k_containment(const float* __restrict__ V,
         if (candidates) atomicAdd(&table.stats[6], (unsigned long long)candidates);
     }
     if (TRACK) trk.candidates[o] = candidates;
+}
+
+// One thread per object, with the per-source diagnostics.
+__global__ void __launch_bounds__(kT) k_containment_tracked(const float* __restrict__ V, uint64_t nV,
+                                                            const uint32_t* __restrict__ I,
+                                                            const int32_t* __restrict__ first, uint64_t nObj,
+                                                            const BNode* __restrict__ nodes, uint32_t max_steps,
+                                                            const float4* __restrict__ tris, int swap, PairTable table,
+                                                            Tracking trk) {
+    const uint64_t o = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (o >= nObj) return;
+    trk.candidates[o] = 0;
+    for (int q = 0; q < trk.max_targets; ++q) {
+        trk.target_ids[o * trk.max_targets + q] = -1;
+        trk.target_hits[o * trk.max_targets + q] = 0;
+    }
+    Ray r;
+    if (containment_ray(V, nV, I, first, o, r))
+        containment_thread<true>(r, o, nodes, max_steps, tris, swap, table, trk);
+}
+
+// One warp per object: up to 32 nodes a step from a shared-memory stack, as the edge rays of
+// short lists, and the object ids of all crossings in a list; a target is inserted when it
+// occurs an odd number of times.  One thread per object made the join wait on its longest
+// chain of dependent node loads, with one warp for 32 objects.  A ray of more crossings, or
+// a wider traversal, runs the one-thread passes in lane 0.
+constexpr int kContWarps = 4;    // objects per block
+constexpr int kContStack = 256;  // entries of a warp's stack
+constexpr int kContHits = 512;   // crossings a warp keeps
+
+__global__ void __launch_bounds__(32 * kContWarps) k_containment(const float* __restrict__ V, uint64_t nV,
+                                                                 const uint32_t* __restrict__ I,
+                                                                 const int32_t* __restrict__ first, uint64_t nObj,
+                                                                 const BNode* __restrict__ nodes, uint32_t max_steps,
+                                                                 const float4* __restrict__ tris, int swap,
+                                                                 PairTable table) {
+    constexpr unsigned int kAll = 0xffffffffu;
+    __shared__ int s_stack[kContWarps][kContStack];
+    __shared__ uint32_t s_id[kContWarps][kContHits];
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    const unsigned int below = (1u << lane) - 1u;
+    int* stack = s_stack[wi];
+    uint32_t* ids = s_id[wi];
+    for (uint64_t o = blockIdx.x * (uint64_t)kContWarps + wi; o < nObj; o += (uint64_t)gridDim.x * kContWarps) {
+        Ray r;
+        if (!containment_ray(V, nV, I, first, o, r)) continue;  // the same in every lane
+        if (lane == 0) stack[0] = 0;
+        __syncwarp();
+        int sp = 1, nh = 0;
+        uint32_t visits = 0;
+        bool ok = true;
+        unsigned int tests = 0;
+        while (sp > 0) {
+            const int take = min(sp, 32);
+            const int node = lane < take ? stack[sp - take + lane] : -1;
+            __syncwarp();
+            sp -= take;
+            visits += (uint32_t)take;
+            bool h[2] = {false, false};
+            int leaf[2] = {0, 0}, cnt[2] = {0, 0};
+            if (node >= 0) {
+                const float4 na = __ldg(&nodes[node].a), nb = __ldg(&nodes[node].b), nc = __ldg(&nodes[node].c);
+                const int4 nd = __ldg(&nodes[node].d);
+                const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
+                const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
+                float en, ex;
+                h[0] = slab<2>(r, lo0, hi0, r.tmin, r.tmax, en, ex);
+                h[1] = slab<2>(r, lo1, hi1, r.tmin, r.tmax, en, ex);
+                leaf[0] = nd.x;
+                cnt[0] = nd.y;
+                leaf[1] = nd.z;
+                cnt[1] = nd.w;
+            }
+            const bool p0 = h[0] && cnt[0] == 0, p1 = h[1] && cnt[1] == 0;
+            const unsigned b0 = __ballot_sync(kAll, p0), b1 = __ballot_sync(kAll, p1);
+            const int pushed = __popc(b0) + __popc(b1);
+            if (visits > max_steps || sp + pushed > kContStack) {
+                ok = false;
+                break;
+            }
+            int pos = sp + __popc(b0 & below) + __popc(b1 & below);
+            if (p0) stack[pos++] = leaf[0];
+            if (p1) stack[pos] = leaf[1];
+            sp += pushed;
+            // Triangles of the leaves hit: the first child's, then the second's.
+            const int n0 = h[0] ? cnt[0] : 0, n1 = h[1] ? cnt[1] : 0;
+            tests += (unsigned int)(n0 + n1);
+            const int rounds = __reduce_max_sync(kAll, n0 + n1);
+            for (int k = 0; k < rounds; ++k) {
+                bool hit = false;
+                uint32_t tid;
+                int32_t obj = 0;
+                if (k < n0 + n1) {
+                    float a[3], b[3], c[3], t;
+                    load_tri(tris, k < n0 ? leaf[0] + k : leaf[1] + (k - n0), a, b, c, tid, obj);
+                    hit = hit_triangle<2>(r, a, b, c, t);
+                }
+                const unsigned m = __ballot_sync(kAll, hit);
+                const int at = nh + __popc(m & below);
+                if (hit && at < kContHits) ids[at] = (uint32_t)obj;
+                nh += __popc(m);
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+        if (!ok || nh > kContHits) {
+            if (lane == 0) containment_thread<false>(r, o, nodes, max_steps, tris, swap, table, Tracking{});
+            __syncwarp();
+            continue;
+        }
+        add_tests(tests);
+        unsigned int distinct = 0;
+        for (int a = lane; a < nh; a += 32) {
+            const uint32_t id = ids[a];
+            int before = 0, all = 0;
+            for (int b = 0; b < nh; ++b) {
+                const bool same = ids[b] == id;
+                all += same;
+                before += same && b < a;
+            }
+            if (before) continue;  // its first occurrence decides
+            ++distinct;
+            if (all & 1) table_insert(table, containment_key(o, id, swap));
+        }
+        if (table.stats) {
+            distinct = __reduce_add_sync(kAll, distinct);
+            if (lane == 0) {
+                atomicAdd(&table.stats[4], 1ull);
+                if (nh) atomicAdd(&table.stats[5], (unsigned long long)nh);
+                if (distinct) atomicAdd(&table.stats[6], (unsigned long long)distinct);
+            }
+        }
+        __syncwarp();
+    }
 }
 
 }  // namespace
@@ -1557,6 +1703,37 @@ extern "C" int rs_triangle_join(const rs_bvh* target, const float* d_vertices, u
     return r;
 }
 
+namespace rs {
+// Queues the containment rays of source objects 0..nObj-1 (trk nullable).
+static cudaError_t containment_async(const rs_bvh* target, const float* V, uint64_t nV, const uint32_t* I, uint64_t nF,
+                              const int32_t* t2o, uint64_t nObj, int swap, rs_pairset* ps, const Tracking* trk,
+                              cudaStream_t s) {
+    if (nObj == 0 || nF == 0 || target->n_tris == 0) return cudaSuccess;
+    int32_t* first = nullptr;
+    cudaError_t e = dmalloc((void**)&first, nObj * sizeof(int32_t), s);
+    if (e != cudaSuccess) return e;
+    launch(k_first_tri_init, (unsigned)((nObj + 255) / 256), 256, 0, s, first, nObj);
+    launch(k_first_tri, (unsigned)((nF + 256 * kFirstPer - 1) / (256 * kFirstPer)), 256, 0, s, t2o, nF, first, nObj);
+    const int ptok = prof_begin(P_CONTAINMENT, s);
+    if (trk)
+        launch(k_containment_tracked, (unsigned)((nObj + kT - 1) / kT), kT, 0, s, V, nV, I, (const int32_t*)first, nObj,
+               (const BNode*)target->nodes, max_steps(target), (const float4*)target->tris, swap, table_view(ps), *trk);
+    else
+        launch(k_containment, (unsigned)std::min<uint64_t>((nObj + kContWarps - 1) / kContWarps, 16ull * sm_count()),
+               32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first, nObj, (const BNode*)target->nodes,
+               max_steps(target), (const float4*)target->tris, swap, table_view(ps));
+    prof_end(P_CONTAINMENT, s, ptok);
+    e = cudaGetLastError();
+    cudaFreeAsync(first, s);
+    return e;
+}
+
+// Of every object of a built set.
+cudaError_t containment_async(const rs_bvh* target, const rs_bvh* src, int swap, rs_pairset* ps, cudaStream_t s) {
+    return containment_async(target, src->V, src->nV, src->I, src->nF, src->t2o, src->n_obj, swap, ps, nullptr, s);
+}
+}  // namespace rs
+
 static int containment_impl(const rs_bvh* target, const float* d_src_vertices, uint64_t src_nV,
                             const uint32_t* d_src_indices, uint64_t src_nF, const int32_t* d_src_tri2obj, int swap,
                             rs_pairset* ps, const Tracking* trk, uint64_t trk_capacity, cudaStream_t s) {
@@ -1565,44 +1742,23 @@ static int containment_impl(const rs_bvh* target, const float* d_src_vertices, u
     const int st = bvh_use(target, s);
     if (st != RS_OK) return st;
     int* dmx = nullptr;
-    int32_t* first = nullptr;
     int hmx = -1;
     cudaError_t e = dmalloc((void**)&dmx, sizeof(int), s);
     if (e == cudaSuccess) {
         cudaMemsetAsync(dmx, 0xff, sizeof(int), s);
-        launch(k_max_obj, 2 * sm_count(), 256, 0, s, d_src_tri2obj, src_nF, dmx);
+        launch(k_max_obj, (unsigned)std::min<uint64_t>((src_nF + 1023) / 1024, 8ull * sm_count()), 256, 0, s,
+               d_src_tri2obj, src_nF, dmx);
         e = cudaMemcpyAsync(&hmx, dmx, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
+    if (dmx) cudaFreeAsync(dmx, s);
     // Objects 0..max id (the reference sizes its launch by the number of distinct ids,
     // which is the same for the contiguous ids preprocess_dataset writes).
     const uint64_t nObj = hmx >= 0 ? (uint64_t)hmx + 1 : 0;
-    if (trk && nObj > trk_capacity) {
-        if (dmx) cudaFreeAsync(dmx, s);
-        cudaStreamSynchronize(s);
-        return RS_ERR_OUTPUT_OVERFLOW;
-    }
-    if (e == cudaSuccess && nObj) {
-        e = dmalloc((void**)&first, nObj * sizeof(int32_t), s);
-        if (e == cudaSuccess) {
-            launch(k_first_tri_init, (unsigned)((nObj + 255) / 256), 256, 0, s, first, nObj);
-            launch(k_first_tri, (unsigned)((src_nF + 255) / 256), 256, 0, s, d_src_tri2obj, src_nF, first, nObj);
-            const unsigned grid = (unsigned)((nObj + kT - 1) / kT);
-            const int ptok = prof_begin(P_CONTAINMENT, s);
-            if (trk)
-                launch(k_containment<true>, grid, kT, 0, s, d_src_vertices, src_nV, d_src_indices, (const int32_t*)first,
-                       nObj, (const BNode*)target->nodes, max_steps(target), (const float4*)target->tris, swap,
-                       table_view(ps), *trk);
-            else
-                launch(k_containment<false>, grid, kT, 0, s, d_src_vertices, src_nV, d_src_indices, (const int32_t*)first,
-                       nObj, (const BNode*)target->nodes, max_steps(target), (const float4*)target->tris, swap,
-                       table_view(ps), Tracking{0, nullptr, nullptr, nullptr});
-            prof_end(P_CONTAINMENT, s, ptok);
-            e = cudaGetLastError();
-        }
-    }
-    if (dmx) cudaFreeAsync(dmx, s);
-    if (first) cudaFreeAsync(first, s);
+    if (trk && nObj > trk_capacity) return RS_ERR_OUTPUT_OVERFLOW;
+    if (e == cudaSuccess)
+        e = containment_async(target, d_src_vertices, src_nV, d_src_indices, src_nF, d_src_tri2obj, nObj, swap, ps, trk,
+                              s);
     return table_status(ps, s, e);
 }
 

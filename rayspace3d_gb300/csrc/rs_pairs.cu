@@ -18,6 +18,7 @@
 
 namespace rs {
 PairTable table_view(rs_pairset* ps);
+cudaError_t containment_async(const rs_bvh* target, const rs_bvh* src, int swap, rs_pairset* ps, cudaStream_t s);
 cudaError_t edge_join_async(const rs_bvh* target, const float* d_starts, const float* d_ends,
                             const int32_t* d_offsets, const int32_t* d_counts, const int32_t* d_sources, uint64_t nE,
                             int swap, rs_pairset* ps, cudaStream_t s, const EdgeCull& cull);
@@ -366,8 +367,8 @@ static int overlap_join_impl(const rs_bvh* A, const float* d_startsA, const floa
     };
     for (int attempt = 0; attempt < 8; ++attempt) {
         // Order of executeHashQuery (raytracer_intersection_estimated_main.cpp:107-158): overlap A->B,
-        // overlap B->A, containment A->B, containment B->A.  The two edge directions are queued
-        // back to back and checked with one status read.
+        // overlap B->A, containment A->B, containment B->A, queued back to back and checked with
+        // one status read.
         ps->known_count = -1;
         cudaError_t e = cudaMemsetAsync(ps->slots, 0xff, ps->capacity * sizeof(unsigned long long), s);
         if (e == cudaSuccess) e = cudaMemsetAsync(ps->meta, 0, kMetaWords * sizeof(unsigned long long), s);
@@ -388,11 +389,11 @@ static int overlap_join_impl(const rs_bvh* A, const float* d_startsA, const floa
             if (e == cudaSuccess && b2a)
                 e = edge_join_async(A, d_startsB, d_endsB, d_offsetsB, d_countsB, d_sourcesB, nEB, 1, ps, s, cullB);
         }
-        int st = table_status(ps, s, e);
         if (with_containment) {
-            if (st == RS_OK && a2b) st = rs_containment(B, A->V, A->nV, A->I, A->nF, A->t2o, 0, ps, stream);
-            if (st == RS_OK && b2a) st = rs_containment(A, B->V, B->nV, B->I, B->nF, B->t2o, 1, ps, stream);
+            if (e == cudaSuccess && a2b) e = containment_async(B, A, 0, ps, s);
+            if (e == cudaSuccess && b2a) e = containment_async(A, B, 1, ps, s);
         }
+        const int st = table_status(ps, s, e);
         if (st != RS_ERR_TABLE_FULL) {
             release();
             return st;
