@@ -91,10 +91,18 @@ struct WarpEdgeSmem {
 // and push the inner children hit; crossings go to a shared-memory list.  Visits the nodes
 // the one-thread traversal visits (the same slab tests over the same [tmin, tmax]), so it
 // finds the same crossings; the lanes rank them by (t, id) (triangle ids are distinct, so
-// ranks are too) and lane 0 walks them with the table's hit rule.  Returns false, having
-// inserted nothing, when there are more than HITS crossings or the stack or the step
-// budget runs out.
-template <int STACK, int HITS>
+// ranks are too) and lane 0 walks them with the table's hit rule.
+//
+// A step pops no more nodes than the stack has room to replace twice over, so a wide
+// traversal turns into a depth-first one instead of running out of stack: an edge of a
+// large object in a dense cluster overlaps thousands of boxes, and the one-thread loop that
+// used to take such an edge kept a whole join waiting (17 ms of 57).  With RANGES, an edge
+// of more than HITS crossings is walked in ranges of t: the list's middle crossing ends the
+// range and the traversal restarts on it, until a range's crossings fit; the next range
+// begins above it.  Returns false when there are more than HITS crossings (RANGES: at one
+// and the same t) or the step budget or the stack runs out; pairs of ranges walked before
+// that are in the table, where the one-thread loop's start from the beginning finds them.
+template <int STACK, int HITS, bool RANGES>
 __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload& p, uint64_t i,
                               const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris,
                               int swap, const PairTable& table, int start = 0) {
@@ -108,51 +116,55 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
     if (!segment_ray_of(p.starts[3 * i], p.starts[3 * i + 1], p.starts[3 * i + 2], p.ends[3 * i], p.ends[3 * i + 1],
                         p.ends[3 * i + 2], r))
         return true;
-    if (lane == 0) stack[0] = start;
-    __syncwarp();
-    int sp = 1, nh = 0;
-    uint32_t visits = 0;
-    bool ok = true;
+    const float tmax = r.tmax;
+    float above = -INFINITY;  // crossings up to here are walked
+    EdgeWalk w;
+    int32_t last = INT_MIN;
     unsigned int tests = 0;
-    while (sp > 0) {
-        const int take = min(sp, 32);
-        const int node = lane < take ? stack[sp - take + lane] : -1;
+    for (;;) {
+        if (lane == 0) stack[0] = start;
         __syncwarp();
-        sp -= take;
-        visits += (uint32_t)take;
-        if (visits > max_steps) {
-            ok = false;
-            break;
-        }
-        bool h[2] = {false, false};
-        int first[2] = {0, 0}, cnt[2] = {0, 0};
-        if (node >= 0) {
-            const float4 na = __ldg(&nodes[node].a), nb = __ldg(&nodes[node].b), nc = __ldg(&nodes[node].c);
-            const int4 nd = __ldg(&nodes[node].d);
-            const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
-            const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
-            float e, x;
-            h[0] = slab<-1>(r, lo0, hi0, r.tmin, r.tmax, e, x);
-            h[1] = slab<-1>(r, lo1, hi1, r.tmin, r.tmax, e, x);
-            first[0] = nd.x;
-            cnt[0] = nd.y;
-            first[1] = nd.z;
-            cnt[1] = nd.w;
-        }
-#pragma unroll
-        for (int side = 0; side < 2; ++side) {
-            const int mine = (h[side] && cnt[side] > 0) ? cnt[side] : 0;
-            tests += (unsigned int)mine;
-            const int rounds = __reduce_max_sync(0xffffffffu, mine);
+        int sp = 1, nh = 0;
+        uint32_t visits = 0;
+        bool ok = true;
+        while (sp > 0) {
+            const int take = min(min(sp, 32), max(STACK - sp, 1));
+            const int node = lane < take ? stack[sp - take + lane] : -1;
+            __syncwarp();
+            sp -= take;
+            visits += (uint32_t)take;
+            if (visits > max_steps) {
+                ok = false;
+                break;
+            }
+            bool h[2] = {false, false};
+            int first[2] = {0, 0}, cnt[2] = {0, 0};
+            if (node >= 0) {
+                const float4 na = __ldg(&nodes[node].a), nb = __ldg(&nodes[node].b), nc = __ldg(&nodes[node].c);
+                const int4 nd = __ldg(&nodes[node].d);
+                const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
+                const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
+                float e, x;
+                h[0] = slab<-1>(r, lo0, hi0, r.tmin, r.tmax, e, x);
+                h[1] = slab<-1>(r, lo1, hi1, r.tmin, r.tmax, e, x);
+                first[0] = nd.x;
+                cnt[0] = nd.y;
+                first[1] = nd.z;
+                cnt[1] = nd.w;
+            }
+            // Triangles of the leaves hit: the first child's, then the second's.
+            const int n0 = h[0] ? cnt[0] : 0, n1 = h[1] ? cnt[1] : 0;
+            tests += (unsigned int)(n0 + n1);
+            const int rounds = __reduce_max_sync(0xffffffffu, n0 + n1);
             for (int k = 0; k < rounds; ++k) {
                 bool hit = false;
                 float t = 0.0f;
                 uint32_t tid = 0;
                 int32_t obj = 0;
-                if (k < mine) {
+                if (k < n0 + n1) {
                     float a[3], b[3], c[3];
-                    load_tri(tris, first[side] + k, a, b, c, tid, obj);
-                    hit = hit_triangle<-1>(r, a, b, c, t);
+                    load_tri(tris, k < n0 ? first[0] + k : first[1] + (k - n0), a, b, c, tid, obj);
+                    hit = hit_triangle<-1>(r, a, b, c, t) && (!RANGES || t > above);
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, hit);
                 if (hit) {
@@ -165,46 +177,58 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
                 }
                 nh += __popc(m);
             }
+            if (nh > HITS) break;
+            const bool p0 = h[0] && cnt[0] == 0, p1 = h[1] && cnt[1] == 0;
+            const unsigned b0 = __ballot_sync(0xffffffffu, p0), b1 = __ballot_sync(0xffffffffu, p1);
+            const int total = __popc(b0) + __popc(b1);
+            if (sp + total > STACK) {
+                ok = false;
+                break;
+            }
+            int pos = sp + __popc(b0 & lt) + __popc(b1 & lt);
+            if (p0) stack[pos++] = first[0];
+            if (p1) stack[pos] = first[1];
+            __syncwarp();
+            sp += total;
         }
-        const bool p0 = h[0] && cnt[0] == 0, p1 = h[1] && cnt[1] == 0;
-        const unsigned b0 = __ballot_sync(0xffffffffu, p0), b1 = __ballot_sync(0xffffffffu, p1);
-        const int total = __popc(b0) + __popc(b1);
-        if (sp + total > STACK) {
-            ok = false;
-            break;
-        }
-        int pos = sp + __popc(b0 & lt) + __popc(b1 & lt);
-        if (p0) stack[pos++] = first[0];
-        if (p1) stack[pos] = first[1];
         __syncwarp();
-        sp += total;
+        if (!ok) return false;
+        if (!RANGES && nh > HITS) return false;
+        const int kept = min(nh, HITS);
+        for (int a = lane; a < kept; a += 32) {
+            const float t = ht[a];
+            const uint32_t id = hid[a];
+            int rank = 0;
+            for (int b = 0; b < kept; ++b) rank += hit_less(ht[b], hid[b], t, id) ? 1 : 0;
+            w_sm.t2[rank] = t;
+            w_sm.id2[rank] = id;
+            w_sm.obj2[rank] = hobj[a];
+        }
+        __syncwarp();
+        if (RANGES && nh > HITS) {
+            const float mid = w_sm.t2[HITS / 2];
+            if (!(mid < r.tmax)) return false;
+            r.tmax = mid;
+            continue;
+        }
+        if (lane == 0) {
+            const int32_t* src = p.sources + p.offsets[i];
+            const int nsrc = p.counts[i];
+            for (int a = 0; a < nh && !w.done; ++a) {
+                if (!w.take(w_sm.t2[a], table.max_hits, table.next_float)) continue;
+                if (w_sm.obj2[a] == last) continue;
+                last = w_sm.obj2[a];
+                insert_sources(table, src, nsrc, last, swap);
+            }
+        }
+        if (!RANGES || r.tmax == tmax || __shfl_sync(0xffffffffu, (int)w.done, 0)) break;
+        above = r.tmax;
+        r.tmin = fmaxf(r.tmin, above);
+        r.tmax = tmax;
+        __syncwarp();
     }
     add_tests(tests);
-    __syncwarp();
-    if (!ok || nh > HITS) return false;
-    for (int a = lane; a < nh; a += 32) {
-        const float t = ht[a];
-        const uint32_t id = hid[a];
-        int rank = 0;
-        for (int b = 0; b < nh; ++b) rank += hit_less(ht[b], hid[b], t, id) ? 1 : 0;
-        w_sm.t2[rank] = t;
-        w_sm.id2[rank] = id;
-        w_sm.obj2[rank] = hobj[a];
-    }
-    __syncwarp();
-    if (lane == 0) {
-        EdgeWalk w;
-        int32_t last = INT_MIN;
-        const int32_t* src = p.sources + p.offsets[i];
-        const int nsrc = p.counts[i];
-        for (int a = 0; a < nh && !w.done; ++a) {
-            if (!w.take(w_sm.t2[a], table.max_hits, table.next_float)) continue;
-            if (w_sm.obj2[a] == last) continue;
-            last = w_sm.obj2[a];
-            insert_sources(table, src, nsrc, last, swap);
-        }
-        count_edge(table, w.n);
-    }
+    if (lane == 0) count_edge(table, w.n);
     __syncwarp();
     return true;
 }
@@ -222,17 +246,17 @@ __global__ void __launch_bounds__(32 * kWarpRayWarps) k_edge_rays_warp(
         const uint32_t e = live[j];
         const int start = live_entry ? (int)live_entry[j] : 0;
         if (e >= n_direct) continue;
-        if (!edge_ray_warp<kWarpRayStack, kWarpRayHits>(sm[wi], p, e, nodes, max_steps, tris, swap, table, start) &&
+        if (!edge_ray_warp<kWarpRayStack, kWarpRayHits, false>(sm[wi], p, e, nodes, max_steps, tris, swap, table, start) &&
             (threadIdx.x & 31) == 0)
             deferred[atomicAdd(n_def, 1u)] = e;
     }
 }
 
 // Long path over the deferred edges, one warp per edge: the warp collects every crossing
-// of the edge in one traversal (up to kLongWarpHits; the reference's walk takes at most
-// --overlap-max-iterations of them) instead of one thread re-traversing per chunk of 16;
-// an edge with more crossings, or a wider traversal than the warp's stack, runs the
-// one-thread chunked loop (segment_long) in lane 0.
+// of the edge in one traversal (or, beyond kLongWarpHits, in a traversal per range of t; the
+// reference's walk takes at most --overlap-max-iterations of them) instead of one thread
+// re-traversing per chunk of 16, which is left for more than kLongWarpHits crossings at one
+// distance (segment_long, in lane 0).
 constexpr int kLongWarps = 4;
 constexpr int kLongWarpStack = 256;
 constexpr int kLongWarpHits = 256;
@@ -248,7 +272,7 @@ __global__ void __launch_bounds__(32 * kLongWarps) k_edge_long_warp(EdgePayload 
     const unsigned int nw = gridDim.x * kLongWarps;
     for (unsigned int j = blockIdx.x * kLongWarps + wi; j < n; j += nw) {  // warp-uniform
         const uint32_t e = deferred[j];
-        if (!edge_ray_warp<kLongWarpStack, kLongWarpHits>(sm[wi], p, e, nodes, max_steps, tris, swap, table) &&
+        if (!edge_ray_warp<kLongWarpStack, kLongWarpHits, true>(sm[wi], p, e, nodes, max_steps, tris, swap, table) &&
             (threadIdx.x & 31) == 0)
             edge_ray_long(p, e, nodes, max_steps, tris, swap, table);
         __syncwarp();
