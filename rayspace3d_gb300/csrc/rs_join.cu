@@ -36,30 +36,23 @@ constexpr uint64_t kBinMaxEdges = 1ull << 27;
 // cost more than the coherence saves.
 constexpr unsigned int kBinMinLive = 1u << 16;
 
-// Live lists of at most kWarpRayMax edges are traced one warp per edge (k_edge_rays_warp),
-// longer ones one thread per edge (k_edge_rays): with few rays the join waits on the
-// longest chain of dependent node loads, which a warp shortens to the tree's depth plus
-// its node count over 32.
-constexpr unsigned int kWarpRayMax = 4096;
-constexpr int kWarpRayWarps = 8;   // warps per block
-constexpr int kWarpRayStack = 128; // entries of a warp's stack
-constexpr int kWarpRayHits = 16;   // crossings a warp keeps; an edge with more is deferred
+// Edge rays over the edges order[0..*n_order) of a payload of n_direct edges (or over all of
+// them when order is null), in packets that the warps of a resident grid take from *next; a
+// packet has as many edges as give every warp one (32 at most), since the lists of a few
+// thousand edges wait on their longest packet.  The edges it defers go to
+// deferred[0..*n_def).  entry (nullable): the node each listed edge's traversal starts from.
+constexpr int kPacketWarps = 4;
 
-// Fast path over the edges order[0..*n_order) of a payload of n_direct edges (or over all
-// of them when order is null); the edges it defers go to deferred[0..*n_def).
-// entry / order_entry (nullable): the node each listed edge's traversal starts from.
-__global__ void __launch_bounds__(kT) k_edge_rays(EdgePayload p, const uint32_t* __restrict__ order,
-                                                  const uint32_t* __restrict__ live,
-                                                  const unsigned int* __restrict__ n_order, uint64_t n_direct,
-                                                  const BNode* __restrict__ nodes, uint32_t max_steps,
-                                                  const float4* __restrict__ tris, int swap, PairTable table,
-                                                  uint32_t* __restrict__ deferred, unsigned int* __restrict__ n_def,
-                                                  const uint32_t* __restrict__ order_entry,
-                                                  const uint32_t* __restrict__ live_entry) {
-    __shared__ EdgeSmem<kT, kFastStack> sm;
-    const EdgeColumn col = sm.column(threadIdx.x);
+__global__ void __launch_bounds__(32 * kPacketWarps) k_edge_rays(
+    EdgePayload p, const uint32_t* __restrict__ order, const uint32_t* __restrict__ live,
+    const unsigned int* __restrict__ n_order, uint64_t n_direct, const BNode* __restrict__ nodes, uint32_t max_steps,
+    const float4* __restrict__ tris, int swap, PairTable table, uint32_t* __restrict__ deferred,
+    unsigned int* __restrict__ n_def, const uint32_t* __restrict__ order_entry,
+    const uint32_t* __restrict__ live_entry, unsigned int* __restrict__ next) {
+    __shared__ EdgePacket packets[kPacketWarps];
+    EdgePacket& sm = packets[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
     const uint64_t n = live ? (uint64_t)*n_order : n_direct;
-    if (live && n <= kWarpRayMax) return;  // k_edge_rays_warp traces short live lists
     // The cell-ordered list when the job was binned and is long enough, else the live list.
     const uint32_t* entry = nullptr;
     if (live) {
@@ -67,12 +60,22 @@ __global__ void __launch_bounds__(kT) k_edge_rays(EdgePayload p, const uint32_t*
         entry = binned ? order_entry : live_entry;
         order = binned ? order : live;
     }
-    for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t e = order ? order[j] : (uint32_t)j;
-        const int start = entry ? (int)entry[j] : 0;
-        if (e >= n_direct) continue;  // never, for a list of this payload's edges
-        if (!edge_ray_fast<kFastStack>(col, p, e, nodes, max_steps, tris, swap, table, start))
-            deferred[atomicAdd(n_def, 1u)] = e;  // the deferred paths start from the root
+    const uint64_t warps = (uint64_t)gridDim.x * kPacketWarps;
+    const uint32_t size = (uint32_t)min((n + warps - 1) / warps, (uint64_t)32);
+    for (;;) {
+        unsigned int k = 0;
+        if (lane == 0) k = atomicAdd(next, 1u);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        const uint64_t base = (uint64_t)k * size;
+        if (base >= n) return;
+        const uint64_t j = base + lane;
+        bool valid = (uint32_t)lane < size && j < n;
+        const uint32_t e = !valid ? 0u : order ? order[j] : (uint32_t)j;
+        const int start = valid && entry ? (int)entry[j] : 0;
+        valid = valid && e < n_direct;  // always, for a list of this payload's edges
+        if (edge_packet(sm, p, valid, e, start, nodes, max_steps, tris, swap, table))
+            deferred[atomicAdd(n_def, 1u)] = e;
+        __syncwarp();
     }
 }
 
@@ -231,25 +234,6 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
     if (lane == 0) count_edge(table, w.n);
     __syncwarp();
     return true;
-}
-
-__global__ void __launch_bounds__(32 * kWarpRayWarps) k_edge_rays_warp(
-    EdgePayload p, const uint32_t* __restrict__ live, const unsigned int* __restrict__ n_live, uint64_t n_direct,
-    const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris, int swap, PairTable table,
-    uint32_t* __restrict__ deferred, unsigned int* __restrict__ n_def, const uint32_t* __restrict__ live_entry) {
-    __shared__ WarpEdgeSmem<kWarpRayStack, kWarpRayHits> sm[kWarpRayWarps];
-    const unsigned int n = *n_live;
-    if (n > kWarpRayMax) return;  // the one-thread kernel traces this list
-    const int wi = threadIdx.x >> 5;
-    const unsigned int nw = gridDim.x * kWarpRayWarps;
-    for (unsigned int j = blockIdx.x * kWarpRayWarps + wi; j < n; j += nw) {  // warp-uniform
-        const uint32_t e = live[j];
-        const int start = live_entry ? (int)live_entry[j] : 0;
-        if (e >= n_direct) continue;
-        if (!edge_ray_warp<kWarpRayStack, kWarpRayHits, false>(sm[wi], p, e, nodes, max_steps, tris, swap, table, start) &&
-            (threadIdx.x & 31) == 0)
-            deferred[atomicAdd(n_def, 1u)] = e;
-    }
 }
 
 // Long path over the deferred edges, one warp per edge: the warp collects every crossing
@@ -1330,6 +1314,16 @@ namespace rs {
 // Launches one edge-ray direction without waiting for it (status lands in the table's meta word).
 cudaError_t edge_jobs_async(EdgeJob* job, int n_jobs, rs_pairset* ps, cudaStream_t s);
 
+// Blocks of k_edge_rays for at most n edges: one resident wave.
+static unsigned packet_grid(uint64_t n) {
+    static const int per_sm = [] {
+        int b = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_edge_rays, 32 * kPacketWarps, 0);
+        return std::max(b, 1);
+    }();
+    return (unsigned)std::min<uint64_t>((n + kPacketWarps - 1) / kPacketWarps, (uint64_t)per_sm * sm_count());
+}
+
 // Every edge of a payload, in payload order (no broad phase), in chunks of 2^31 edges so
 // that edge ids fit the 32-bit deferred list (a chunk's payload pointers are offset; the
 // offsets still index the whole sources array).
@@ -1340,19 +1334,18 @@ static cudaError_t edge_all_async(const rs_bvh* target, EdgePayload p, uint64_t 
     uint32_t* deferred = nullptr;
     unsigned int* n_def = nullptr;
     cudaError_t e = dmalloc((void**)&deferred, std::max<uint64_t>(cap, 1) * sizeof(uint32_t), s);
-    if (e == cudaSuccess) e = dmalloc((void**)&n_def, sizeof(unsigned int), s);
+    if (e == cudaSuccess) e = dmalloc((void**)&n_def, 2 * sizeof(unsigned int), s);  // deferred, next packet
     const PairTable table = table_view(ps);
     const int ptok = prof_begin(P_EDGE_JOIN, s);
     for (uint64_t base = 0; base < nE && e == cudaSuccess; base += kChunk) {
         const uint64_t n = std::min(kChunk, nE - base);
         const EdgePayload q{p.starts + 3 * base, p.ends + 3 * base, p.offsets + base, p.counts + base, p.sources};
-        e = cudaMemsetAsync(n_def, 0, sizeof(unsigned int), s);
+        e = cudaMemsetAsync(n_def, 0, 2 * sizeof(unsigned int), s);
         if (e != cudaSuccess) break;
-        const unsigned grid = (unsigned)std::min<uint64_t>((n + kT - 1) / kT, 8ull * sm_count());
-        launch(k_edge_rays, grid, kT, 0, s, q, (const uint32_t*)nullptr, (const uint32_t*)nullptr,
+        launch(k_edge_rays, packet_grid(n), 32 * kPacketWarps, 0, s, q, (const uint32_t*)nullptr, (const uint32_t*)nullptr,
                (const unsigned int*)nullptr, n,
                (const BNode*)target->nodes, max_steps(target), (const float4*)target->tris, swap, table, deferred,
-               n_def, (const uint32_t*)nullptr, (const uint32_t*)nullptr);
+               n_def, (const uint32_t*)nullptr, (const uint32_t*)nullptr, n_def + 1);
         launch(k_edge_long_warp, (unsigned)std::min<uint64_t>((n + kLongWarps - 1) / kLongWarps, 4ull * sm_count()),
                32 * kLongWarps, 0, s, q, (const uint32_t*)deferred, (const unsigned int*)n_def,
                (const BNode*)target->nodes, max_steps(target), (const float4*)target->tris, swap, table);
@@ -1393,7 +1386,7 @@ cudaError_t edge_join_async(const rs_bvh* target, const float* d_starts, const f
 // job's on a side stream) and its deferred edges.  Each job's nE < 2^32 and its cull flags
 // set.
 cudaError_t edge_jobs_async(EdgeJob* job, int n_jobs, rs_pairset* ps, cudaStream_t s) {
-    // One zeroed block: n_live[2], n_def[2], the cell counts of the binned jobs, then (slab
+    // One zeroed block: n_live[2], n_def[2], next packet[2], the cell counts of the binned jobs, then (slab
     // mode) each job's slab flags.
     uint32_t* zeroed = nullptr;
     EdgeJob jobs[2] = {};
@@ -1408,7 +1401,7 @@ cudaError_t edge_jobs_async(EdgeJob* job, int n_jobs, rs_pairset* ps, cudaStream
         slab = slab && jobs[d].xindex && jobs[d].sbox && jobs[d].part;
     }
     auto a256 = [](size_t b) { return (b + 255) & ~size_t(255); };
-    const size_t cbytes = a256((4 + (size_t)n_bin * kCells) * sizeof(uint32_t));
+    const size_t cbytes = a256((6 + (size_t)n_bin * kCells) * sizeof(uint32_t));
     size_t zbytes = cbytes;
     for (int d = 0; d < n_jobs && slab; ++d) {
         jobs[d].n_slab = (jobs[d].nE + kSlab - 1) / kSlab;
@@ -1424,7 +1417,7 @@ cudaError_t edge_jobs_async(EdgeJob* job, int n_jobs, rs_pairset* ps, cudaStream
     }
     cudaError_t e = dmalloc((void**)&zeroed, total, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(zeroed, 0, zbytes, s);
-    uint32_t* next_cells = zeroed + 4;
+    uint32_t* next_cells = zeroed + 6;
     char* next_flags = reinterpret_cast<char*>(zeroed) + cbytes;
     char* next = reinterpret_cast<char*>(zeroed) + a256(zbytes);
     for (int d = 0; d < n_jobs && e == cudaSuccess; ++d) {
@@ -1490,15 +1483,10 @@ cudaError_t edge_jobs_async(EdgeJob* job, int n_jobs, rs_pairset* ps, cudaStream
         for (int d = 0; d < n_jobs; ++d) {
             const EdgeJob& j = jobs[d];
             cudaStream_t st = d == 1 && side ? side : s;
-            launch(k_edge_rays_warp,
-                   (unsigned)std::min<uint64_t>((std::min<uint64_t>(j.nE, kWarpRayMax) + kWarpRayWarps - 1) /
-                                                    kWarpRayWarps, 4ull * sm_count()),
-                   32 * kWarpRayWarps, 0, st, j.p, (const uint32_t*)j.live, (const unsigned int*)j.n_live, j.nE,
-                   j.nodes, j.max_steps, j.tris, j.swap, table, j.rank, j.n_def, (const uint32_t*)j.live_entry);
-            launch(k_edge_rays, (unsigned)std::min<uint64_t>((j.nE + kT - 1) / kT, 8ull * sm_count()), kT, 0, st, j.p,
-                   (const uint32_t*)j.order, (const uint32_t*)j.live, (const unsigned int*)j.n_live, j.nE, j.nodes,
-                   j.max_steps, j.tris, j.swap, table, j.rank, j.n_def, (const uint32_t*)j.order_entry,
-                   (const uint32_t*)j.live_entry);
+            launch(k_edge_rays, packet_grid(j.nE), 32 * kPacketWarps, 0, st, j.p, (const uint32_t*)j.order,
+                   (const uint32_t*)j.live, (const unsigned int*)j.n_live, j.nE, j.nodes, j.max_steps, j.tris, j.swap,
+                   table, j.rank, j.n_def, (const uint32_t*)j.order_entry, (const uint32_t*)j.live_entry,
+                   zeroed + 4 + d);
             launch(k_edge_long_warp,
                    (unsigned)std::min<uint64_t>((j.nE + kLongWarps - 1) / kLongWarps, 4ull * sm_count()),
                    32 * kLongWarps, 0, st, j.p, (const uint32_t*)j.rank, (const unsigned int*)j.n_def, j.nodes,

@@ -759,6 +759,188 @@ __device__ __forceinline__ void edge_ray_long(const EdgePayload& p, uint64_t i, 
     segment_long(r, p.sources + p.offsets[i], p.counts[i], nodes, max_steps, tris, swap, table);
 }
 
+// ---------------------------------------------------------------------------
+// Edge packets: up to 32 edges by one warp, every lane busy.  One thread per edge ran 9 of 32
+// lanes an instruction (the edges of a warp visit different numbers of nodes and reach their
+// leaves at different steps) and left whole joins waiting on the thread with the longest
+// traversal.  Here the warp's (node, edge) pairs lie on one shared-memory stack and its
+// (leaf, edge) pairs in a ring: each step pops up to 32 nodes of any of the edges and tests
+// both children of each, and 32 leaves at a time are tested once there are so many.  The
+// visits, and so the crossings, are those of one traversal per edge.
+// ---------------------------------------------------------------------------
+constexpr int kPacketStack = 512;  // (node, edge) pairs
+constexpr int kPacketRing = 128;   // (leaf, edge) pairs: below 32 before a step, which adds at most 64
+constexpr int kPacketHits = 8;     // crossings kept per edge
+
+struct EdgePacket {
+    float4 o[32];    // origin, tmax
+    float4 d[32];    // direction
+    float4 inv[32];  // 1 / direction as make_ray defines it
+    int node[kPacketStack];
+    uint2 leaf[kPacketRing];  // first triangle; count << 5 | edge
+    float t[kPacketHits][32];
+    uint32_t id[kPacketHits][32];
+    int32_t obj[kPacketHits][32];
+    int n[32];
+    unsigned char own[kPacketStack];
+};
+
+// The edge of every lane (valid false: none), traversed from node `start`.  True for a lane
+// whose edge has to be traced by the long path: more than kPacketHits crossings, or the
+// packet ran out of stack or steps; nothing is inserted for it.
+__device__ __forceinline__ bool edge_packet(EdgePacket& sm, const EdgePayload& p, bool valid, uint64_t i, int start,
+                                            const BNode* __restrict__ nodes, uint32_t max_steps,
+                                            const float4* __restrict__ tris, int swap, const PairTable& table) {
+    constexpr unsigned int kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned int below = (1u << lane) - 1u;
+    {
+        Ray r;
+        if (valid)
+            valid = segment_ray_of(p.starts[3 * i], p.starts[3 * i + 1], p.starts[3 * i + 2], p.ends[3 * i],
+                                   p.ends[3 * i + 1], p.ends[3 * i + 2], r);
+        if (valid) {
+            sm.o[lane] = make_float4(r.o[0], r.o[1], r.o[2], r.tmax);
+            sm.d[lane] = make_float4(r.d[0], r.d[1], r.d[2], 0.0f);
+            sm.inv[lane] = make_float4(r.inv[0], r.inv[1], r.inv[2], 0.0f);
+        }
+    }
+    sm.n[lane] = 0;
+    const unsigned int traced = __ballot_sync(kAll, valid);
+    if (valid) {
+        const int at = __popc(traced & below);
+        sm.node[at] = start;
+        sm.own[at] = (unsigned char)lane;
+    }
+    __syncwarp();
+    int sp = __popc(traced);
+    uint32_t head = 0, queued = 0, steps = 0;
+    unsigned int tests = 0;
+    bool ok = true;
+    auto ray_of = [&](int e) {
+        const float4 o = sm.o[e], inv = sm.inv[e];
+        Ray r;
+        r.o[0] = o.x; r.o[1] = o.y; r.o[2] = o.z;
+        r.inv[0] = inv.x; r.inv[1] = inv.y; r.inv[2] = inv.z;
+        r.tmin = kEps;
+        r.tmax = o.w;
+        return r;
+    };
+    while (sp > 0 || queued > 0) {
+        if (queued >= 32u || sp == 0) {
+            const uint32_t m = min(queued, 32u);
+            const uint2 leaf = (uint32_t)lane < m ? sm.leaf[(head + lane) & (kPacketRing - 1)] : make_uint2(0u, 0u);
+            head += m;
+            queued -= m;
+            const int cnt = (int)(leaf.y >> 5), e = (int)(leaf.y & 31u);
+            tests += (unsigned int)cnt;
+            const int rounds = __reduce_max_sync(kAll, cnt);
+            for (int k = 0; k < rounds; ++k) {
+                if (k >= cnt) continue;
+                float a[3], b[3], c[3], t;
+                uint32_t tid;
+                int32_t obj;
+                load_tri(tris, (int)leaf.x + k, a, b, c, tid, obj);
+                Ray r = ray_of(e);
+                const float4 d = sm.d[e];
+                r.d[0] = d.x; r.d[1] = d.y; r.d[2] = d.z;
+                if (!hit_triangle<-1>(r, a, b, c, t)) continue;
+                const int slot = atomicAdd(&sm.n[e], 1);
+                if (slot < kPacketHits) {
+                    sm.t[slot][e] = t;
+                    sm.id[slot][e] = tid;
+                    sm.obj[slot][e] = obj;
+                }
+            }
+            __syncwarp();
+            continue;
+        }
+        // No more nodes than the stack has room to replace twice over.
+        const int take = min(min(sp, 32), max(kPacketStack - sp, 1));
+        sp -= take;
+        if (++steps > max_steps) {  // a step visits a node, and no edge visits one twice
+            ok = false;
+            break;
+        }
+        bool h0 = false, h1 = false;
+        int e = 0;
+        int4 nd = make_int4(0, 0, 0, 0);
+        if (lane < take) {
+            const int node = sm.node[sp + lane];
+            e = sm.own[sp + lane];
+            const float4 na = __ldg(&nodes[node].a), nb = __ldg(&nodes[node].b), nc = __ldg(&nodes[node].c);
+            nd = __ldg(&nodes[node].d);
+            const Ray r = ray_of(e);
+            const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
+            const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
+            float en, ex;
+            h0 = slab<-1>(r, lo0, hi0, r.tmin, r.tmax, en, ex);
+            h1 = slab<-1>(r, lo1, hi1, r.tmin, r.tmax, en, ex);
+        }
+        __syncwarp();  // popped entries are read before they are overwritten
+        const bool l0 = h0 && nd.y > 0, l1 = h1 && nd.w > 0;
+        const unsigned int ml0 = __ballot_sync(kAll, l0), ml1 = __ballot_sync(kAll, l1);
+        if (ml0 | ml1) {
+            const uint32_t at = head + queued;
+            if (l0) sm.leaf[(at + __popc(ml0 & below)) & (kPacketRing - 1)] = make_uint2((uint32_t)nd.x, (uint32_t)nd.y << 5 | (uint32_t)e);
+            if (l1)
+                sm.leaf[(at + __popc(ml0) + __popc(ml1 & below)) & (kPacketRing - 1)] =
+                    make_uint2((uint32_t)nd.z, (uint32_t)nd.w << 5 | (uint32_t)e);
+            queued += __popc(ml0) + __popc(ml1);
+        }
+        const bool p0 = h0 && nd.y <= 0, p1 = h1 && nd.w <= 0;
+        const unsigned int mp0 = __ballot_sync(kAll, p0), mp1 = __ballot_sync(kAll, p1);
+        const int pushed = __popc(mp0) + __popc(mp1);
+        if (sp + pushed > kPacketStack) {
+            ok = false;
+            break;
+        }
+        if (p0) {
+            const int at = sp + __popc(mp0 & below);
+            sm.node[at] = nd.x;
+            sm.own[at] = (unsigned char)e;
+        }
+        if (p1) {
+            const int at = sp + __popc(mp0) + __popc(mp1 & below);
+            sm.node[at] = nd.z;
+            sm.own[at] = (unsigned char)e;
+        }
+        sp += pushed;
+        __syncwarp();
+    }
+    __syncwarp();
+    add_tests(tests);
+    if (!valid) return false;
+    const int n = sm.n[lane];
+    if (!ok || n > kPacketHits) return true;
+    // The crossings in (t, id) order, each the least above the one before.
+    EdgeWalk w;
+    int32_t last = INT_MIN;
+    float ct = -INFINITY;
+    uint32_t cid = 0;
+    for (int k = 0; k < n && !w.done; ++k) {
+        float bt = INFINITY;
+        uint32_t bid = 0xffffffffu;
+        int32_t bobj = -1;
+        for (int j = 0; j < n; ++j) {
+            const float t = sm.t[j][lane];
+            const uint32_t id = sm.id[j][lane];
+            if ((k == 0 || hit_less(ct, cid, t, id)) && hit_less(t, id, bt, bid)) {
+                bt = t;
+                bid = id;
+                bobj = sm.obj[j][lane];
+            }
+        }
+        ct = bt;
+        cid = bid;
+        if (!w.take(bt, table.max_hits, table.next_float) || bobj == last) continue;
+        last = bobj;
+        insert_sources(table, p.sources + p.offsets[i], p.counts[i], bobj, swap);
+    }
+    count_edge(table, w.n);
+    return false;
+}
+
 // Record r = 3 t + e: edge e of triangle t of a source mesh, in the triangle's own
 // orientation (v0v1, v1v2, v2v0), with the triangle's object as its one source -- the
 // legacy per-triangle overlap (mesh_overlap.cu:126-179), which traces shared edges once

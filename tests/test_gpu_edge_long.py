@@ -1,5 +1,5 @@
-"""Edges with long crossing lists and wide traversals (the warp-per-edge path's lists,
-ranges of t and stack): 255 to 700 crossings of one edge, hundreds of crossings at one
+"""Edges with long crossing lists and wide traversals: lists of a few and of many edges with
+as many crossings as a packet keeps and one more, and, on the warp-per-edge path, 255 to 700 crossings of one edge, hundreds of crossings at one
 distance, and edges of large objects through a dense cluster.  Pair sets equal the CPU
 oracle's."""
 import numpy as np
@@ -45,7 +45,14 @@ def _large(n):
     return synth.make_geometry(V, I, T)
 
 
-CASES = {"256": lambda: (_rod(4.0), _slabs(128)), "255": lambda: (_rod(4.0), _half(128)),
+def _rods(k):
+    """k rods side by side through the same slabs: a list of 18 k edges of 8 or 9 crossings."""
+    return synth.box_set([(np.array([0.001 * j, 0.03, -0.5]), np.array([0.001 * j + 0.0004, 0.11, 4.0]))
+                          for j in range(k)])
+
+
+CASES = {"8 crossings": lambda: (_rods(1), _slabs(4)), "9 crossings": lambda: (_rods(1), _half(5)),
+         "594 edges": lambda: (_rods(33), _half(5)), "3600 edges": lambda: (_rods(200), _slabs(4)), "256": lambda: (_rod(4.0), _slabs(128)), "255": lambda: (_rod(4.0), _half(128)),
          "258": lambda: (_rod(4.0), _slabs(129)), "700": lambda: (_rod(8.0), _slabs(350)),
          "equal": lambda: (_rod(4.0), _coincident(300)), "cluster": lambda: (_large(60), _cluster(6000))}
 
