@@ -8,9 +8,9 @@
 // counter and trace its rays with the same per-ray bodies as the single-query kernels
 // (rs_query_core.cuh), so queries of very uneven sizes share the GPU without a launch
 // or a tail per query.  Axis-aligned point-in-mesh queries read the handle's column
-// grid (built at the first submit), others traverse the BVH.  Points whose rays cross
-// more than 8 triangles, and edges with more than 4 crossings or a deep traversal, go to
-// one overflow list that a second launch resolves exactly.  The launches of an unchanged
+// grid (built at the first submit), others traverse the BVH in ray packets.  Rays and edges
+// that cross more than 8 triangles (axis-aligned points: 256) go to one overflow list that a
+// second launch resolves exactly.  The launches of an unchanged
 // batch are captured once as a CUDA graph and replayed.  rs_batch_autotune times the
 // batch over BVH leaf sizes, chunk sizes and traversal stack depths and keeps the best.
 #include <algorithm>
@@ -61,19 +61,15 @@ __device__ __forceinline__ int find_query(const BatchQuery* __restrict__ q, int 
     return lo;
 }
 
-// One warp's shared memory: a chunk is grid queries, rays or edges (stacks and crossings in
-// one column per lane), so the three share it.
-template <int STACK>
+// One warp's shared memory: a chunk is grid queries or ray packets, so the two share it.
 union BatchWarp {
     GridWarpSlots grid;
-    HitSmem<32, STACK> rays;
-    EdgeSmem<32, STACK> edges;
+    RayPacket rays;
 };
 
-template <int STACK>
-__device__ __forceinline__ BatchWarp<STACK>& batch_warp() {
+__device__ __forceinline__ BatchWarp& batch_warp() {
     extern __shared__ __align__(16) unsigned char batch_smem[];
-    return reinterpret_cast<BatchWarp<STACK>*>(batch_smem)[threadIdx.x >> 5];
+    return reinterpret_cast<BatchWarp*>(batch_smem)[threadIdx.x >> 5];
 }
 
 __device__ __forceinline__ void batch_spill(const BatchQuery& Q, int qi, uint64_t i, uint2* __restrict__ ovf,
@@ -87,10 +83,10 @@ __device__ __forceinline__ void batch_spill(const BatchQuery& Q, int qi, uint64_
 // spilled 1.2 KB of registers a thread at 168 registers.
 
 // Warp-cooperative rounds of 32 points: every lane takes part in each round.
-template <int AXIS, int STACK>
+template <int AXIS>
 __device__ __noinline__ void batch_grid(const BatchQuery& Q, int qi, uint64_t r0, uint64_t r1, uint2* ovf,
                                         unsigned long long* ovf_count) {
-    GridWarpSlots& sl = batch_warp<STACK>().grid;
+    GridWarpSlots& sl = batch_warp().grid;
     for (uint64_t base = r0; base < r1; base += 32) {
         const uint64_t i = base + (threadIdx.x & 31);
         const bool valid = i < r1;
@@ -106,33 +102,38 @@ __device__ __noinline__ void batch_grid(const BatchQuery& Q, int qi, uint64_t r0
     }
 }
 
-// Point-in-mesh rays of any direction: BVH traversal, one lane per ray.
-template <int STACK>
+// Point-in-mesh rays of any direction: BVH traversal in packets.
 __device__ __noinline__ void batch_rays(const BatchQuery& Q, int qi, uint64_t r0, uint64_t r1, uint2* ovf,
                                         unsigned long long* ovf_count) {
-    const HitColumn col = batch_warp<STACK>().rays.column(threadIdx.x & 31);
-    for (uint64_t i = r0 + (threadIdx.x & 31); i < r1; i += 32) {
-        const Ray r = make_ray(Q.pts[3 * i], Q.pts[3 * i + 1], Q.pts[3 * i + 2], Q.dx, Q.dy, Q.dz, kEps, kTmax);
-        int n;
-        const bool ok = pim_column<-1, STACK>(col, Q.nodes, Q.max_steps, Q.tris, r, n);
-        if (!ok) atomicOr(Q.status, ST_STACK_OVERFLOW);
-        else if (n > kHits) batch_spill(Q, qi, i, ovf, ovf_count);
-        else write_result(column_chain(col, n), i, Q.obj, Q.in);
+    RayPacket& sm = batch_warp().rays;
+    for (uint64_t base = r0; base < r1; base += 32) {
+        const uint64_t i = base + (threadIdx.x & 31);
+        const bool valid = i < r1;
+        Ray r;
+        if (valid) r = make_ray(Q.pts[3 * i], Q.pts[3 * i + 1], Q.pts[3 * i + 2], Q.dx, Q.dy, Q.dz, kEps, kTmax);
+        const bool ok = packet_trace<-1>(sm, r, valid, 0, Q.nodes, Q.max_steps, Q.tris);
+        if (valid) {
+            const int n = sm.n[threadIdx.x & 31];
+            if (!ok || n > kPacketHits) batch_spill(Q, qi, i, ovf, ovf_count);
+            else write_result(packet_chain(sm, Q.tris, n), i, Q.obj, Q.in);
+        }
+        __syncwarp();
     }
 }
 
-template <int STACK>
 __device__ __noinline__ void batch_edges(const BatchQuery& Q, int qi, uint64_t r0, uint64_t r1, uint2* ovf,
                                          unsigned long long* ovf_count) {
-    const EdgeColumn col = batch_warp<STACK>().edges.column(threadIdx.x & 31);
+    RayPacket& sm = batch_warp().rays;
     const EdgePayload p{Q.starts, Q.ends, Q.offsets, Q.counts, Q.sources};
-    for (uint64_t i = r0 + (threadIdx.x & 31); i < r1; i += 32)
-        if (!edge_ray_fast<STACK>(col, p, i, Q.nodes, Q.max_steps, Q.tris, Q.swap, Q.table))
+    for (uint64_t base = r0; base < r1; base += 32) {
+        const uint64_t i = base + (threadIdx.x & 31);
+        if (edge_packet(sm, p, i < r1, i, 0, Q.nodes, Q.max_steps, Q.tris, Q.swap, Q.table))
             batch_spill(Q, qi, i, ovf, ovf_count);
+        __syncwarp();
+    }
 }
 
-template <int STACK>
-__global__ void __launch_bounds__(kBT, 4) k_batch(const BatchQuery* __restrict__ q, int nq, uint64_t total_chunks,
+__global__ void __launch_bounds__(kBT, 6) k_batch(const BatchQuery* __restrict__ q, int nq, uint64_t total_chunks,
                                                int chunk, unsigned long long* __restrict__ next,
                                                uint2* __restrict__ ovf, unsigned long long* __restrict__ ovf_count) {
     for (;;) {
@@ -145,11 +146,11 @@ __global__ void __launch_bounds__(kBT, 4) k_batch(const BatchQuery* __restrict__
         const uint64_t r0 = (c - Q.first_chunk) * (uint64_t)chunk;
         const uint64_t r1 = min(r0 + (uint64_t)chunk, Q.n);
         // Axis-aligned point queries always have a grid (queries of empty meshes have no chunk).
-        if (Q.kind == 1) batch_edges<STACK>(Q, qi, r0, r1, ovf, ovf_count);
-        else if (Q.axis == 0) batch_grid<0, STACK>(Q, qi, r0, r1, ovf, ovf_count);
-        else if (Q.axis == 1) batch_grid<1, STACK>(Q, qi, r0, r1, ovf, ovf_count);
-        else if (Q.axis == 2) batch_grid<2, STACK>(Q, qi, r0, r1, ovf, ovf_count);
-        else batch_rays<STACK>(Q, qi, r0, r1, ovf, ovf_count);
+        if (Q.kind == 1) batch_edges(Q, qi, r0, r1, ovf, ovf_count);
+        else if (Q.axis == 0) batch_grid<0>(Q, qi, r0, r1, ovf, ovf_count);
+        else if (Q.axis == 1) batch_grid<1>(Q, qi, r0, r1, ovf, ovf_count);
+        else if (Q.axis == 2) batch_grid<2>(Q, qi, r0, r1, ovf, ovf_count);
+        else batch_rays(Q, qi, r0, r1, ovf, ovf_count);
         __syncwarp();
     }
 }
@@ -246,10 +247,7 @@ void release_device(rs_batch* b) {
     b->dirty = true;
 }
 
-template <int STACK>
-constexpr size_t batch_smem_bytes() {
-    return (kBT / 32) * sizeof(BatchWarp<STACK>);
-}
+constexpr size_t kBatchSmem = (kBT / 32) * sizeof(BatchWarp);
 
 int commit(rs_batch* b, cudaStream_t s) {
     if (!b->dirty) return RS_OK;
@@ -315,19 +313,18 @@ int commit(rs_batch* b, cudaStream_t s) {
     }
     b->total_chunks = chunks;
     int per_sm = 0;
-    if (b->stack == 32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<32>, kBT, batch_smem_bytes<32>());
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<64>, kBT, batch_smem_bytes<64>());
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch, kBT, kBatchSmem);
     b->grid = std::max(1, per_sm) * sm_count();
     b->dirty = false;
     return RS_OK;
 }
 
-// One fallback thread per possible overflow entry, up to the list's capacity (the count
-// is only known on the device; threads past it return at once).
+// Fallback blocks: a resident grid at most (the entries' number is only known on the device;
+// one thread per possible entry took 20 us to find none).
 unsigned fallback_grid(const rs_batch* b) {
     uint64_t rays = 0;
     for (const rs_batch_item& it : b->items) rays += it.n;
-    return (unsigned)std::max<uint64_t>(1, (std::min(rays, kOverflowCap) + kBT - 1) / kBT);
+    return (unsigned)std::min<uint64_t>((std::min(rays, kOverflowCap) + kBT - 1) / kBT + 1, 8ull * sm_count());
 }
 
 // The launches of one submit: counters, per-query statuses, outputs of queries against
@@ -344,17 +341,14 @@ cudaError_t enqueue(rs_batch* b, cudaStream_t s) {
     }
     if (e != cudaSuccess) return e;
     if (b->total_chunks) {
-        if (b->stack == 32) {
-            launch(k_batch<32>, b->grid, kBT, batch_smem_bytes<32>(), s, (const BatchQuery*)b->d_q, nq, b->total_chunks, b->chunk,
-                   b->d_counters, b->d_ovf, b->d_counters + 1);
-            if (b->d_ovf) launch(k_batch_fallback<32>, fallback_grid(b), kBT, 0, s, (const BatchQuery*)b->d_q,
-                                 (const uint2*)b->d_ovf, (const unsigned long long*)b->d_counters + 1);
-        } else {
-            launch(k_batch<64>, b->grid, kBT, batch_smem_bytes<64>(), s, (const BatchQuery*)b->d_q, nq, b->total_chunks, b->chunk,
-                   b->d_counters, b->d_ovf, b->d_counters + 1);
-            if (b->d_ovf) launch(k_batch_fallback<64>, fallback_grid(b), kBT, 0, s, (const BatchQuery*)b->d_q,
-                                 (const uint2*)b->d_ovf, (const unsigned long long*)b->d_counters + 1);
-        }
+        launch(k_batch, b->grid, kBT, kBatchSmem, s, (const BatchQuery*)b->d_q, nq, b->total_chunks, b->chunk,
+               b->d_counters, b->d_ovf, b->d_counters + 1);
+        if (b->d_ovf && b->stack == 32)
+            launch(k_batch_fallback<32>, fallback_grid(b), kBT, 0, s, (const BatchQuery*)b->d_q,
+                   (const uint2*)b->d_ovf, (const unsigned long long*)b->d_counters + 1);
+        else if (b->d_ovf)
+            launch(k_batch_fallback<64>, fallback_grid(b), kBT, 0, s, (const BatchQuery*)b->d_q,
+                   (const uint2*)b->d_ovf, (const unsigned long long*)b->d_counters + 1);
     }
     return cudaGetLastError();
 }

@@ -456,6 +456,22 @@ struct __align__(16) BNode {
     int4 d;    // idx0 count0 idx1 count1
 };
 
+// A node by two 32-byte loads: with every lane at another node, half the cache lookups of
+// four 16-byte loads.  The node array is 256-byte aligned and read-only in every traversal.
+__device__ __forceinline__ BNode load_node(const BNode* __restrict__ nodes, int i) {
+    BNode n;
+    const BNode* p = nodes + i;
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(n.a.x), "=f"(n.a.y), "=f"(n.a.z), "=f"(n.a.w), "=f"(n.b.x), "=f"(n.b.y), "=f"(n.b.z), "=f"(n.b.w)
+        : "l"(p));
+    float d0, d1, d2, d3;
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(n.c.x), "=f"(n.c.y), "=f"(n.c.z), "=f"(n.c.w), "=f"(d0), "=f"(d1), "=f"(d2), "=f"(d3)
+        : "l"(reinterpret_cast<const char*>(p) + 32));
+    n.d = make_int4(__float_as_int(d0), __float_as_int(d1), __float_as_int(d2), __float_as_int(d3));
+    return n;
+}
+
 constexpr int kStack = 64;
 
 // Visits every leaf whose box passes the slab test and calls on_leaf(first, count)
@@ -472,10 +488,9 @@ __device__ __forceinline__ bool traverse_with(int* stack, int stride, const BNod
     int node = start;  // the root, or a node known to hold every triangle the ray can hit
     for (uint32_t step = 0;; ++step) {
         if (step > max_steps) return false;
-        const float4 na = __ldg(&nodes[node].a);
-        const float4 nb = __ldg(&nodes[node].b);
-        const float4 nc = __ldg(&nodes[node].c);
-        const int4 nd = __ldg(&nodes[node].d);
+        const BNode bn = load_node(nodes, node);
+        const float4 na = bn.a, nb = bn.b, nc = bn.c;
+        const int4 nd = bn.d;
         const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
         const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
         float e0, x0, e1, x1;

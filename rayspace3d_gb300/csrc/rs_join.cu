@@ -43,14 +43,14 @@ constexpr unsigned int kBinMinLive = 1u << 16;
 // deferred[0..*n_def).  entry (nullable): the node each listed edge's traversal starts from.
 constexpr int kPacketWarps = 4;
 
-__global__ void __launch_bounds__(32 * kPacketWarps) k_edge_rays(
+__global__ void __launch_bounds__(32 * kPacketWarps, 6) k_edge_rays(
     EdgePayload p, const uint32_t* __restrict__ order, const uint32_t* __restrict__ live,
     const unsigned int* __restrict__ n_order, uint64_t n_direct, const BNode* __restrict__ nodes, uint32_t max_steps,
     const float4* __restrict__ tris, int swap, PairTable table, uint32_t* __restrict__ deferred,
     unsigned int* __restrict__ n_def, const uint32_t* __restrict__ order_entry,
     const uint32_t* __restrict__ live_entry, unsigned int* __restrict__ next) {
-    __shared__ EdgePacket packets[kPacketWarps];
-    EdgePacket& sm = packets[threadIdx.x >> 5];
+    __shared__ RayPacket packets[kPacketWarps];
+    RayPacket& sm = packets[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const uint64_t n = live ? (uint64_t)*n_order : n_direct;
     // The cell-ordered list when the job was binned and is long enough, else the live list.
@@ -143,8 +143,9 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
             bool h[2] = {false, false};
             int first[2] = {0, 0}, cnt[2] = {0, 0};
             if (node >= 0) {
-                const float4 na = __ldg(&nodes[node].a), nb = __ldg(&nodes[node].b), nc = __ldg(&nodes[node].c);
-                const int4 nd = __ldg(&nodes[node].d);
+                const BNode bn = load_node(nodes, node);
+            const float4 na = bn.a, nb = bn.b, nc = bn.c;
+            const int4 nd = bn.d;
                 const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
                 const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
                 float e, x;
@@ -842,8 +843,9 @@ __global__ void __launch_bounds__(kT) k_cull_flag(CullJob j0, CullJob j1, unsign
             result = 1;
             break;
         }
-        const float4 na = __ldg(&nodes[node].a), nb = __ldg(&nodes[node].b), nc = __ldg(&nodes[node].c);
-        const int4 nd = __ldg(&nodes[node].d);
+        const BNode bn = load_node(nodes, node);
+            const float4 na = bn.a, nb = bn.b, nc = bn.c;
+            const int4 nd = bn.d;
         bool h0 = cull_overlap(na.x, na.y, na.z, na.w, nb.x, nb.y, qlo, qhi);
         bool h1 = cull_overlap(nb.z, nb.w, nc.x, nc.y, nc.z, nc.w, qlo, qhi);
 #pragma unroll 1
@@ -958,8 +960,9 @@ __global__ void __launch_bounds__(32 * kCullWarps) k_cull_query(CullJob j0, Cull
         bool h[2] = {false, false};
         int first[2] = {0, 0}, cnt[2] = {0, 0};
         if (node >= 0) {
-            const float4 na = __ldg(&nodes[node].a), nb = __ldg(&nodes[node].b), nc = __ldg(&nodes[node].c);
-            const int4 nd = __ldg(&nodes[node].d);
+            const BNode bn = load_node(nodes, node);
+            const float4 na = bn.a, nb = bn.b, nc = bn.c;
+            const int4 nd = bn.d;
             h[0] = cull_overlap(na.x, na.y, na.z, na.w, nb.x, nb.y, qlo, qhi);
             h[1] = cull_overlap(nb.z, nb.w, nc.x, nc.y, nc.z, nc.w, qlo, qhi);
             first[0] = nd.x;
@@ -1207,8 +1210,9 @@ __global__ void __launch_bounds__(32 * kContWarps) k_containment(const float* __
             bool h[2] = {false, false};
             int leaf[2] = {0, 0}, cnt[2] = {0, 0};
             if (node >= 0) {
-                const float4 na = __ldg(&nodes[node].a), nb = __ldg(&nodes[node].b), nc = __ldg(&nodes[node].c);
-                const int4 nd = __ldg(&nodes[node].d);
+                const BNode bn = load_node(nodes, node);
+            const float4 na = bn.a, nb = bn.b, nc = bn.c;
+            const int4 nd = bn.d;
                 const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
                 const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
                 float en, ex;

@@ -78,34 +78,32 @@ __device__ __forceinline__ bool box_filter(const BoxBounds& box, const Ray& r) {
 }
 
 
-// BVH traversal per ray: a 32-entry stack and the crossings in shared memory (28 KB a block of
-// 128 threads); deeper or longer rays go to the fallback.
+// BVH traversal in ray packets, for directions without a column grid.  Rays of more
+// crossings than a packet keeps, or of a packet without room, go to the fallback.
 constexpr int kPimT = 128;
-constexpr int kPimStack = 32;
 
 template <int AXIS, bool FILTER>
-__global__ void __launch_bounds__(kPimT) k_pim(const float* __restrict__ pts, uint64_t n, float dx, float dy, float dz,
-                                            const BNode* __restrict__ nodes, uint32_t max_steps,
-                                            const float4* __restrict__ tris, BoxBounds box,
-                                            int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
-                                            uint32_t* __restrict__ ovf_list,
-                                            unsigned long long* __restrict__ ovf_count) {
+__global__ void __launch_bounds__(kPimT, 6) k_pim(const float* __restrict__ pts, uint64_t n, float dx, float dy,
+                                                  float dz, const BNode* __restrict__ nodes, uint32_t max_steps,
+                                                  const float4* __restrict__ tris, BoxBounds box,
+                                                  int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
+                                                  uint32_t* __restrict__ ovf_list,
+                                                  unsigned long long* __restrict__ ovf_count) {
+    __shared__ RayPacket packets[kPimT / 32];
+    RayPacket& sm = packets[threadIdx.x >> 5];
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const Ray r = make_ray(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], dx, dy, dz, kEps, kTmax);
-    if (FILTER && !box_filter<AXIS>(box, r)) {
-        write_result(Chain{}, i, out_obj, out_in);
-        return;
+    const bool valid = i < n;
+    Ray r;
+    bool keep = valid;
+    if (valid) {
+        r = make_ray(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], dx, dy, dz, kEps, kTmax);
+        if (FILTER) keep = box_filter<AXIS>(box, r);
     }
-    __shared__ HitSmem<kPimT, kPimStack> sm;
-    const HitColumn col = sm.column(threadIdx.x);
-    int n_hits;
-    const bool ok = pim_column<AXIS, kPimStack>(col, nodes, max_steps, tris, r, n_hits);
-    if (!ok || n_hits > kHits) {  // the fallback's deeper stack and longer list take it
-        ovf_list[atomicAdd(ovf_count, 1ull)] = (uint32_t)i;
-        return;
-    }
-    write_result(column_chain(col, n_hits), i, out_obj, out_in);
+    const bool ok = packet_trace<AXIS>(sm, r, keep, 0, nodes, max_steps, tris);
+    const int hits = keep ? sm.n[threadIdx.x & 31] : 0;
+    if (!valid) return;
+    if (keep && (!ok || hits > kPacketHits)) ovf_list[atomicAdd(ovf_count, 1ull)] = (uint32_t)i;
+    else write_result(packet_chain(sm, tris, hits), i, out_obj, out_in);
 }
 
 // Column-grid query, 32 points a warp (pim_grid_warp).

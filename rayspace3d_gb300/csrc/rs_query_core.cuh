@@ -387,71 +387,6 @@ __device__ __forceinline__ void pim_grid_warp(const GridView& g, const float4* _
     add_tests(lane == 0 ? tests : 0u);
 }
 
-// One thread's shared-memory column for pim_column: element k of an array at base[k * stride].
-struct HitColumn {
-    int* stack;
-    float* t;
-    uint32_t* id;
-    int32_t* obj;
-    int stride;
-};
-
-// Shared memory of pim_column for T threads.
-template <int T, int STACK>
-struct HitSmem {
-    int stack[STACK][T];
-    float t[kHits][T];
-    uint32_t id[kHits][T];
-    int32_t obj[kHits][T];
-    __device__ __forceinline__ HitColumn column(int tid) {
-        return HitColumn{&stack[0][tid], &t[0][tid], &id[0][tid], &obj[0][tid], T};
-    }
-};
-
-// Crossings of ray r with t in [1e-6, 1e16] by BVH traversal, stack and up to kHits crossings
-// in the thread's shared-memory column (a register list appends through kHits predicated
-// moves, and spilled).  n receives their number, which may exceed kHits; false on an
-// exhausted traversal budget or stack.
-template <int AXIS, int STACK>
-__device__ __forceinline__ bool pim_column(const HitColumn& col, const BNode* __restrict__ nodes, uint32_t max_steps,
-                                           const float4* __restrict__ tris, const Ray& r, int& n) {
-    unsigned int tests = 0;
-    n = 0;
-    const bool ok = traverse_with<AXIS, STACK>(col.stack, col.stride, nodes, max_steps, r, [&](int first, int cnt) {
-        tests += (unsigned int)cnt;
-        for (int k = first; k < first + cnt; ++k) {
-            float a[3], b[3], c[3];
-            uint32_t tid;
-            int32_t obj;
-            load_tri(tris, k, a, b, c, tid, obj);
-            float t;
-            if (!hit_triangle<AXIS>(r, a, b, c, t)) continue;
-            if (n < kHits) {
-                col.t[n * col.stride] = t;
-                col.id[n * col.stride] = tid;
-                col.obj[n * col.stride] = obj;
-            }
-            ++n;
-        }
-    });
-    add_tests(tests);
-    return ok;
-}
-
-// The advance rule on the n <= kHits crossings of a column.
-__device__ __forceinline__ Chain column_chain(const HitColumn& col, int n) {
-    HitList hl;
-#pragma unroll
-    for (int q = 0; q < kHits; ++q)
-        if (q < n) {
-            hl.t[q] = col.t[q * col.stride];
-            hl.id[q] = col.id[q * col.stride];
-            hl.obj[q] = col.obj[q * col.stride];
-        }
-    hl.n = n;
-    return n <= 2 ? hl.finish2() : hl.finish();
-}
-
 // Exact fallback for a ray with more than kHits crossings: each round re-traverses the
 // BVH and takes the smallest (t, id) above the previous one, so the crossings are
 // walked in the same order as the sorted list.
@@ -736,19 +671,6 @@ struct EdgePayload {
     const int32_t* sources;
 };
 
-template <int STACK>
-__device__ __forceinline__ bool edge_ray_fast(const EdgeColumn& col, const EdgePayload& p, uint64_t i,
-                                              const BNode* __restrict__ nodes, uint32_t max_steps,
-                                              const float4* __restrict__ tris, int swap, const PairTable& table,
-                                              int start = 0) {
-    Ray r;
-    if (!segment_ray_of(p.starts[3 * i], p.starts[3 * i + 1], p.starts[3 * i + 2], p.ends[3 * i], p.ends[3 * i + 1],
-                        p.ends[3 * i + 2], r))
-        return true;
-    return segment_fast<STACK>(col, r, p.sources + p.offsets[i], p.counts[i], nodes, max_steps, tris, swap, table,
-                               start);
-}
-
 __device__ __forceinline__ void edge_ray_long(const EdgePayload& p, uint64_t i, const BNode* __restrict__ nodes,
                                               uint32_t max_steps, const float4* __restrict__ tris, int swap,
                                               const PairTable& table) {
@@ -760,49 +682,47 @@ __device__ __forceinline__ void edge_ray_long(const EdgePayload& p, uint64_t i, 
 }
 
 // ---------------------------------------------------------------------------
-// Edge packets: up to 32 edges by one warp, every lane busy.  One thread per edge ran 9 of 32
-// lanes an instruction (the edges of a warp visit different numbers of nodes and reach their
+// Ray packets: up to 32 rays by one warp, every lane busy.  One thread per ray ran 9 of 32
+// lanes an instruction (the rays of a warp visit different numbers of nodes and reach their
 // leaves at different steps) and left whole joins waiting on the thread with the longest
-// traversal.  Here the warp's (node, edge) pairs lie on one shared-memory stack and its
-// (leaf, edge) pairs in a ring: each step pops up to 32 nodes of any of the edges and tests
+// traversal.  Here the warp's (node, ray) pairs lie on one shared-memory stack and its
+// (leaf, ray) pairs in a ring: each step pops up to 32 nodes of any of the rays and tests
 // both children of each, and 32 leaves at a time are tested once there are so many.  The
-// visits, and so the crossings, are those of one traversal per edge.
+// visits, and so the crossings, are those of one traversal per ray.  Bound by the latency of
+// the scattered node loads at 24 warps an SM: 6.6 KB a warp leaves the L1 cache 70 KB, where
+// 32 warps of 64 registers (no spills gained) took 15 % longer and 16 warps 25 %.
 // ---------------------------------------------------------------------------
-constexpr int kPacketStack = 512;  // (node, edge) pairs
-constexpr int kPacketRing = 128;   // (leaf, edge) pairs: below 32 before a step, which adds at most 64
-constexpr int kPacketHits = 8;     // crossings kept per edge
+constexpr int kPacketStack = 384;  // (node, ray) pairs
+constexpr int kPacketRing = 128;   // (leaf, ray) pairs: below 32 before a step, which adds at most 64
+constexpr int kPacketHits = kHits; // crossings kept per ray
 
-struct EdgePacket {
+struct RayPacket {
     float4 o[32];    // origin, tmax
     float4 d[32];    // direction
     float4 inv[32];  // 1 / direction as make_ray defines it
     int node[kPacketStack];
-    uint2 leaf[kPacketRing];  // first triangle; count << 5 | edge
+    uint2 leaf[kPacketRing];  // first triangle; count << 5 | ray
     float t[kPacketHits][32];
-    uint32_t id[kPacketHits][32];
-    int32_t obj[kPacketHits][32];
+    int tri[kPacketHits][32];  // leaf-ordered triangle: its id and object are read at the end
     int n[32];
     unsigned char own[kPacketStack];
 };
 
-// The edge of every lane (valid false: none), traversed from node `start`.  True for a lane
-// whose edge has to be traced by the long path: more than kPacketHits crossings, or the
-// packet ran out of stack or steps; nothing is inserted for it.
-__device__ __forceinline__ bool edge_packet(EdgePacket& sm, const EdgePayload& p, bool valid, uint64_t i, int start,
-                                            const BNode* __restrict__ nodes, uint32_t max_steps,
-                                            const float4* __restrict__ tris, int swap, const PairTable& table) {
+// Traces every lane's ray r (valid false: none; r.tmin 1e-6 for all) from node `start`: sm.n
+// has its number of crossings, sm.t and sm.tri the first kPacketHits found.  False when the
+// packet ran out of stack or steps.
+template <int AXIS>
+__device__ __forceinline__ bool packet_trace(RayPacket& sm, const Ray& mine, bool valid, int start,
+                                             const BNode* __restrict__ nodes, uint32_t max_steps,
+                                             const float4* __restrict__ tris) {
     constexpr unsigned int kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned int below = (1u << lane) - 1u;
-    {
-        Ray r;
-        if (valid)
-            valid = segment_ray_of(p.starts[3 * i], p.starts[3 * i + 1], p.starts[3 * i + 2], p.ends[3 * i],
-                                   p.ends[3 * i + 1], p.ends[3 * i + 2], r);
-        if (valid) {
-            sm.o[lane] = make_float4(r.o[0], r.o[1], r.o[2], r.tmax);
-            sm.d[lane] = make_float4(r.d[0], r.d[1], r.d[2], 0.0f);
-            sm.inv[lane] = make_float4(r.inv[0], r.inv[1], r.inv[2], 0.0f);
+    if (valid) {
+        sm.o[lane] = make_float4(mine.o[0], mine.o[1], mine.o[2], mine.tmax);
+        if (AXIS < 0) {
+            sm.d[lane] = make_float4(mine.d[0], mine.d[1], mine.d[2], 0.0f);
+            sm.inv[lane] = make_float4(mine.inv[0], mine.inv[1], mine.inv[2], 0.0f);
         }
     }
     sm.n[lane] = 0;
@@ -817,13 +737,21 @@ __device__ __forceinline__ bool edge_packet(EdgePacket& sm, const EdgePayload& p
     uint32_t head = 0, queued = 0, steps = 0;
     unsigned int tests = 0;
     bool ok = true;
-    auto ray_of = [&](int e) {
-        const float4 o = sm.o[e], inv = sm.inv[e];
+    auto ray_of = [&](int e, bool direction) {
+        const float4 o = sm.o[e];
+        if (AXIS >= 0)
+            return make_ray(o.x, o.y, o.z, AXIS == 0 ? 1.0f : 0.0f, AXIS == 1 ? 1.0f : 0.0f, AXIS == 2 ? 1.0f : 0.0f,
+                            kEps, o.w);
+        const float4 inv = sm.inv[e];
         Ray r;
         r.o[0] = o.x; r.o[1] = o.y; r.o[2] = o.z;
         r.inv[0] = inv.x; r.inv[1] = inv.y; r.inv[2] = inv.z;
         r.tmin = kEps;
         r.tmax = o.w;
+        if (direction) {
+            const float4 d = sm.d[e];
+            r.d[0] = d.x; r.d[1] = d.y; r.d[2] = d.z;
+        }
         return r;
     };
     while (sp > 0 || queued > 0) {
@@ -841,15 +769,11 @@ __device__ __forceinline__ bool edge_packet(EdgePacket& sm, const EdgePayload& p
                 uint32_t tid;
                 int32_t obj;
                 load_tri(tris, (int)leaf.x + k, a, b, c, tid, obj);
-                Ray r = ray_of(e);
-                const float4 d = sm.d[e];
-                r.d[0] = d.x; r.d[1] = d.y; r.d[2] = d.z;
-                if (!hit_triangle<-1>(r, a, b, c, t)) continue;
+                if (!hit_triangle<AXIS>(ray_of(e, true), a, b, c, t)) continue;
                 const int slot = atomicAdd(&sm.n[e], 1);
                 if (slot < kPacketHits) {
                     sm.t[slot][e] = t;
-                    sm.id[slot][e] = tid;
-                    sm.obj[slot][e] = obj;
+                    sm.tri[slot][e] = (int)leaf.x + k;
                 }
             }
             __syncwarp();
@@ -858,7 +782,7 @@ __device__ __forceinline__ bool edge_packet(EdgePacket& sm, const EdgePayload& p
         // No more nodes than the stack has room to replace twice over.
         const int take = min(min(sp, 32), max(kPacketStack - sp, 1));
         sp -= take;
-        if (++steps > max_steps) {  // a step visits a node, and no edge visits one twice
+        if (++steps > max_steps) {  // a step visits a node, and no ray visits one twice
             ok = false;
             break;
         }
@@ -868,14 +792,15 @@ __device__ __forceinline__ bool edge_packet(EdgePacket& sm, const EdgePayload& p
         if (lane < take) {
             const int node = sm.node[sp + lane];
             e = sm.own[sp + lane];
-            const float4 na = __ldg(&nodes[node].a), nb = __ldg(&nodes[node].b), nc = __ldg(&nodes[node].c);
-            nd = __ldg(&nodes[node].d);
-            const Ray r = ray_of(e);
+            const BNode bn = load_node(nodes, node);
+            const float4 na = bn.a, nb = bn.b, nc = bn.c;
+            nd = bn.d;
+            const Ray r = ray_of(e, false);
             const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
             const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
             float en, ex;
-            h0 = slab<-1>(r, lo0, hi0, r.tmin, r.tmax, en, ex);
-            h1 = slab<-1>(r, lo1, hi1, r.tmin, r.tmax, en, ex);
+            h0 = slab<AXIS>(r, lo0, hi0, r.tmin, r.tmax, en, ex);
+            h1 = slab<AXIS>(r, lo1, hi1, r.tmin, r.tmax, en, ex);
         }
         __syncwarp();  // popped entries are read before they are overwritten
         const bool l0 = h0 && nd.y > 0, l1 = h1 && nd.w > 0;
@@ -910,6 +835,38 @@ __device__ __forceinline__ bool edge_packet(EdgePacket& sm, const EdgePayload& p
     }
     __syncwarp();
     add_tests(tests);
+    return ok;
+}
+
+// The advance rule on the crossings that packet_trace left for this lane (at most
+// kPacketHits).
+__device__ __forceinline__ Chain packet_chain(const RayPacket& sm, const float4* __restrict__ tris, int n) {
+    const int lane = threadIdx.x & 31;
+    HitList hl;
+#pragma unroll
+    for (int q = 0; q < kHits; ++q)
+        if (q < n) {
+            const size_t k = 3 * (size_t)sm.tri[q][lane];
+            hl.t[q] = sm.t[q][lane];
+            hl.id[q] = __float_as_uint(__ldg(&tris[k].w));
+            hl.obj[q] = __float_as_int(__ldg(&tris[k + 1].w));
+        }
+    hl.n = n;
+    return n <= 2 ? hl.finish2() : hl.finish();
+}
+
+// The edge of every lane (valid false: none), traversed from node `start`.  True for a lane
+// whose edge has to be traced by the long path: more than kPacketHits crossings, or the
+// packet ran out of stack or steps; nothing is inserted for it.
+__device__ __forceinline__ bool edge_packet(RayPacket& sm, const EdgePayload& p, bool valid, uint64_t i, int start,
+                                            const BNode* __restrict__ nodes, uint32_t max_steps,
+                                            const float4* __restrict__ tris, int swap, const PairTable& table) {
+    const int lane = threadIdx.x & 31;
+    Ray r;
+    if (valid)
+        valid = segment_ray_of(p.starts[3 * i], p.starts[3 * i + 1], p.starts[3 * i + 2], p.ends[3 * i],
+                               p.ends[3 * i + 1], p.ends[3 * i + 2], r);
+    const bool ok = packet_trace<-1>(sm, r, valid, start, nodes, max_steps, tris);
     if (!valid) return false;
     const int n = sm.n[lane];
     if (!ok || n > kPacketHits) return true;
@@ -921,16 +878,17 @@ __device__ __forceinline__ bool edge_packet(EdgePacket& sm, const EdgePayload& p
     for (int k = 0; k < n && !w.done; ++k) {
         float bt = INFINITY;
         uint32_t bid = 0xffffffffu;
-        int32_t bobj = -1;
+        int bk = 0;
         for (int j = 0; j < n; ++j) {
             const float t = sm.t[j][lane];
-            const uint32_t id = sm.id[j][lane];
+            const uint32_t id = __float_as_uint(__ldg(&tris[3 * (size_t)sm.tri[j][lane]].w));
             if ((k == 0 || hit_less(ct, cid, t, id)) && hit_less(t, id, bt, bid)) {
                 bt = t;
                 bid = id;
-                bobj = sm.obj[j][lane];
+                bk = sm.tri[j][lane];
             }
         }
+        const int32_t bobj = __float_as_int(__ldg(&tris[3 * (size_t)bk + 1].w));
         ct = bt;
         cid = bid;
         if (!w.take(bt, table.max_hits, table.next_float) || bobj == last) continue;
