@@ -69,28 +69,52 @@ __device__ __forceinline__ bool tri_valid(const uint32_t* __restrict__ I, uint64
 
 // Pass 1 (preprocess_dataset.cpp:69-86): object boxes and valid-triangle span.  flags[0]
 // is set when a valid triangle's object is outside [0, n_obj); flags[1] when tri2obj
-// decreases somewhere (objects not stored contiguously).
-__global__ void k_gs_boxes(const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, uint64_t nF,
-                           const int32_t* __restrict__ T, ObjStats* __restrict__ o, uint64_t n_obj,
-                           uint32_t* __restrict__ flags) {
+// decreases somewhere (objects not stored contiguously).  The lanes of a warp that share an
+// object reduce its box first: triangles are stored by object, and eight atomics a triangle
+// queued on their object's words (3.2 M triangles: 410 us against 40).
+__global__ void __launch_bounds__(kGT) k_gs_boxes(const float* __restrict__ V, uint64_t nV,
+                                                  const uint32_t* __restrict__ I, uint64_t nF,
+                                                  const int32_t* __restrict__ T, ObjStats* __restrict__ o,
+                                                  uint64_t n_obj, uint32_t* __restrict__ flags) {
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (t >= nF) return;
-    if (t > 0 && T[t] < T[t - 1]) flags[1] = 1;
-    if (!tri_valid(I, nV, t)) return;
-    const int32_t obj = T[t];
-    if (obj < 0 || (uint64_t)obj >= n_obj) {
+    const int32_t obj = t < nF ? T[t] : -1;
+    if (t > 0 && t < nF && obj < T[t - 1]) flags[1] = 1;
+    bool ok = t < nF && tri_valid(I, nV, t);
+    if (ok && (obj < 0 || (uint64_t)obj >= n_obj)) {
         flags[0] = 1;
-        return;
+        ok = false;
     }
+    int lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+    if (ok) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const float a = V[3 * (uint64_t)I[3 * t] + c], b = V[3 * (uint64_t)I[3 * t + 1] + c],
-                    d = V[3 * (uint64_t)I[3 * t + 2] + c];
-        atomicMin(&o[obj].box[c], g_f2ord(fminf(fminf(a, b), d)));
-        atomicMax(&o[obj].box[3 + c], g_f2ord(fmaxf(fmaxf(a, b), d)));
+        for (int c = 0; c < 3; ++c) {
+            const float a = V[3 * (uint64_t)I[3 * t] + c], b = V[3 * (uint64_t)I[3 * t + 1] + c],
+                        d = V[3 * (uint64_t)I[3 * t + 2] + c];
+            lo[c] = g_f2ord(fminf(fminf(a, b), d));
+            hi[c] = g_f2ord(fmaxf(fmaxf(a, b), d));
+        }
     }
-    atomicMin(&o[obj].first, (uint32_t)t);
-    atomicMax(&o[obj].last, (uint32_t)t);
+    const int lane = threadIdx.x & 31;
+    unsigned int todo = __ballot_sync(0xffffffffu, ok);
+    while (todo) {  // one object at a time; warp-uniform
+        const int32_t one = __shfl_sync(0xffffffffu, obj, __ffs(todo) - 1);
+        const bool in = ok && obj == one;
+        const unsigned int group = __ballot_sync(0xffffffffu, in);
+        todo &= ~group;
+        if (!in) continue;
+        ObjStats& s = o[one];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int l = __reduce_min_sync(group, lo[c]), h = __reduce_max_sync(group, hi[c]);
+            if (lane == __ffs(group) - 1) {
+                atomicMin(&s.box[c], l);
+                atomicMax(&s.box[3 + c], h);
+            }
+        }
+        // Lanes hold consecutive triangles: the group's first and last.
+        if (lane == __ffs(group) - 1) atomicMin(&s.first, (uint32_t)t);
+        if (lane == 31 - __clz(group)) atomicMax(&s.last, (uint32_t)t);
+    }
 }
 
 // The float term of one triangle (:100-113): translate by the box centre, dot(cross(t0,t1), t2),
@@ -113,17 +137,57 @@ __device__ __forceinline__ void box_centre(const ObjStats& s, float c[3]) {
     for (int k = 0; k < 3; ++k) c[k] = __fmul_rn(__fadd_rn(g_ord2f(s.box[k]), g_ord2f(s.box[3 + k])), 0.5f);
 }
 
-// Pass 2 (:88-114), objects stored contiguously: each object's valid triangles in order.
-__global__ void k_gs_volume_span(const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I,
-                                 ObjStats* __restrict__ o, uint64_t n_obj) {
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i >= n_obj || o[i].first == kNone) return;
-    float c[3];
-    box_centre(o[i], c);
+// Pass 2 (:88-114), objects stored contiguously: each object's valid triangles in order.  A
+// block takes 32 objects: its warps compute the terms of kVolChunk triangles of each into
+// shared memory, then one lane per object adds them in order -- the sums are the serial part,
+// but a thread that also loads its object's triangles one after the other waits on each
+// (10,000 objects of 320: 318 us).  A triangle that does not count adds 0.0, which leaves
+// every partial sum as it is (none is -0.0: they start at 0.0).
+constexpr int kVolObjects = 32;
+constexpr int kVolChunk = 128;
+
+__global__ void __launch_bounds__(kGT) k_gs_volume_span(const float* __restrict__ V, uint64_t nV,
+                                                        const uint32_t* __restrict__ I, ObjStats* __restrict__ o,
+                                                        uint64_t n_obj) {
+    __shared__ float term[kVolObjects][kVolChunk + 1];
+    __shared__ uint32_t s_n[kVolObjects], s_first[kVolObjects];
+    __shared__ float s_c[kVolObjects][3];
+    const uint64_t o0 = blockIdx.x * (uint64_t)kVolObjects;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t n = 0;
     double vol = 0.0;
-    for (uint64_t t = o[i].first; t <= o[i].last; ++t)
-        if (tri_valid(I, nV, t)) vol = __dadd_rn(vol, (double)volume_term(V, I, t, c));
-    o[i].volume = vol;
+    if (threadIdx.x < kVolObjects) {
+        const uint64_t i = o0 + threadIdx.x;
+        if (i < n_obj && o[i].first != kNone) {
+            n = o[i].last - o[i].first + 1;
+            s_first[threadIdx.x] = o[i].first;
+            box_centre(o[i], s_c[threadIdx.x]);
+        }
+        s_n[threadIdx.x] = n;
+    }
+    __syncthreads();
+    uint32_t most = 0;
+    for (int k = 0; k < kVolObjects; ++k) most = max(most, s_n[k]);
+    for (uint32_t base = 0; base < most; base += kVolChunk) {
+        for (int k = warp; k < kVolObjects; k += kGT / 32) {
+            const uint32_t nk = s_n[k];
+#pragma unroll
+            for (int q = 0; q < kVolChunk / 32; ++q) {
+                const uint32_t j = base + 32 * q + lane;
+                if (j < nk) {
+                    const uint64_t t = (uint64_t)s_first[k] + j;
+                    term[k][32 * q + lane] = tri_valid(I, nV, t) ? volume_term(V, I, t, s_c[k]) : 0.0f;
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < kVolObjects && n > base) {
+            const uint32_t m = min(n - base, (uint32_t)kVolChunk);
+            for (uint32_t j = 0; j < m; ++j) vol = __dadd_rn(vol, (double)term[threadIdx.x][j]);
+        }
+        __syncthreads();
+    }
+    if (n) o[o0 + threadIdx.x].volume = vol;
 }
 
 // Sort keys (object << 32 | triangle) for the general case; invalid triangles and
@@ -345,7 +409,7 @@ extern "C" int rs_grid_stats(const float* d_vertices, uint64_t nV, const uint32_
     if (e != cudaSuccess) return to_status(e);
     if (hf[0]) return RS_ERR_INVALID;  // an object id outside [0, n_obj)
     if (!hf[1]) {
-        launch(k_gs_volume_span, go, kGT, 0, s, d_vertices, nV, d_indices, o, n_obj);
+        launch(k_gs_volume_span, (unsigned)((n_obj + kVolObjects - 1) / kVolObjects), kGT, 0, s, d_vertices, nV, d_indices, o, n_obj);
     } else {
         uint64_t* keys = nullptr;
         uint32_t* start = nullptr;
