@@ -87,19 +87,15 @@ template <int AXIS>
 __device__ __noinline__ void batch_grid(const BatchQuery& Q, int qi, uint64_t r0, uint64_t r1, uint2* ovf,
                                         unsigned long long* ovf_count) {
     GridWarpSlots& sl = batch_warp().grid;
-    for (uint64_t base = r0; base < r1; base += 32) {
-        const uint64_t i = base + (threadIdx.x & 31);
-        const bool valid = i < r1;
-        float p[3] = {0.0f, 0.0f, 0.0f};
-        if (valid) {
+    grid_points<AXIS>(
+        Q.grid, Q.tris, r0 + (threadIdx.x & 31), r1, 32, Q.obj, Q.in, sl,
+        [&](uint64_t i, float* p) {
             p[0] = Q.pts[3 * i];
             p[1] = Q.pts[3 * i + 1];
             p[2] = Q.pts[3 * i + 2];
-        }
-        pim_grid_warp<AXIS>(Q.grid, Q.tris, p, valid, valid, i, Q.obj, Q.in, sl,
-                            [&]() { batch_spill(Q, qi, i, ovf, ovf_count); });
-        __syncwarp();
-    }
+        },
+        [](const float*) { return true; }, [&](uint32_t i) { batch_spill(Q, qi, i, ovf, ovf_count); });
+    __syncwarp();
 }
 
 // Point-in-mesh rays of any direction: BVH traversal in packets.

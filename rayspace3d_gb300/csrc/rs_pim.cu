@@ -109,28 +109,28 @@ __global__ void __launch_bounds__(kPimT, 6) k_pim(const float* __restrict__ pts,
 
 // Column-grid query, 32 points a warp (pim_grid_warp).
 constexpr int kWarps = kT / 32;
+constexpr int kGridBlocks = 4;  // resident blocks an SM
 
 template <int AXIS, bool FILTER>
-__global__ void __launch_bounds__(kT, 4) k_pim_grid(const float* __restrict__ pts, uint64_t n, GridView g,
+__global__ void __launch_bounds__(kT, kGridBlocks) k_pim_grid(const float* __restrict__ pts, uint64_t n, GridView g,
                                                  const float4* __restrict__ tris, BoxBounds box,
                                                  int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
                                                  uint32_t* __restrict__ ovf_list,
                                                  unsigned long long* __restrict__ ovf_count) {
     __shared__ GridWarpSlots slots[kWarps];
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const bool valid = i < n;
-    float p[3] = {0.0f, 0.0f, 0.0f};
-    if (valid) {
-        p[0] = pts[3 * i];
-        p[1] = pts[3 * i + 1];
-        p[2] = pts[3 * i + 2];
-    }
-    bool keep = valid;
-    if (FILTER && valid)
-        keep = box_filter<AXIS>(box, make_ray(p[0], p[1], p[2], AXIS == 0 ? 1.0f : 0.0f, AXIS == 1 ? 1.0f : 0.0f,
-                                              AXIS == 2 ? 1.0f : 0.0f, kEps, kTmax));
-    pim_grid_warp<AXIS>(g, tris, p, valid, keep, i, out_obj, out_in, slots[threadIdx.x >> 5],
-                        [&]() { ovf_list[atomicAdd(ovf_count, 1ull)] = (uint32_t)i; });
+    grid_points<AXIS>(
+        g, tris, blockIdx.x * (uint64_t)kT + threadIdx.x, n, (uint64_t)gridDim.x * kT, out_obj, out_in,
+        slots[threadIdx.x >> 5],
+        [&](uint64_t i, float* p) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) p[q] = __ldcs(&pts[3 * i + q]);
+        },
+        [&](const float* p) {
+            return !FILTER || box_filter<AXIS>(box, make_ray(p[0], p[1], p[2], AXIS == 0 ? 1.0f : 0.0f,
+                                                             AXIS == 1 ? 1.0f : 0.0f, AXIS == 2 ? 1.0f : 0.0f, kEps,
+                                                             kTmax));
+        },
+        [&](uint32_t i) { ovf_list[atomicAdd(ovf_count, 1ull)] = i; });
 }
 
 // Exact fallback for rays with more than kHits crossings (pim_fallback_ray).
@@ -395,6 +395,11 @@ cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
     return e;
 }
 
+// Blocks of k_pim_grid: one resident wave at most.
+unsigned grid_blocks(uint64_t n) {
+    return (unsigned)std::min<uint64_t>((n + kT - 1) / kT, (uint64_t)kGridBlocks * sm_count());
+}
+
 template <int AXIS, bool FILTER>
 cudaError_t launch_pim(const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz,
                        const BoxBounds& box, int32_t* obj, uint8_t* in, uint32_t* ovf_list,
@@ -403,7 +408,7 @@ cudaError_t launch_pim(const rs_bvh* bvh, const float* pts, uint64_t n, float dx
     const int ptok = prof_begin(P_PIM, s);
     if (AXIS >= 0 && bvh->cgrid[GA].built) {
         const GridView g = grid_view(bvh->cgrid[GA]);
-        launch(k_pim_grid<GA, FILTER>, (unsigned)((n + kT - 1) / kT), kT, 0, s, pts, n, g, (const float4*)bvh->tris, box, obj, in, ovf_list,
+        launch(k_pim_grid<GA, FILTER>, grid_blocks(n), kT, 0, s, pts, n, g, (const float4*)bvh->tris, box, obj, in, ovf_list,
                ovf_count);
     } else {
         launch(k_pim<AXIS, FILTER>, (unsigned)((n + kPimT - 1) / kPimT), kPimT, 0, s, pts, n, dx, dy, dz, bvh->nodes,

@@ -208,6 +208,10 @@ struct GridWarpSlots {
     float p[3][32];
     uint4 rec[32];      // of the k-th point with candidates: list offset, units, lane
     uint2 ring[64];     // triangle, lane of its point
+    // Points with candidates that wait for a full round (grid_points): coordinates, list
+    // begin and length, units, number.
+    float qp[3][64];
+    uint32_t qb[64], qc[64], qu[64], qi[64];
 };
 constexpr int kDenseHits = 32 * kHits;
 // Candidates a point from which a warp takes its points one at a time: the lists then fill
@@ -258,16 +262,16 @@ __device__ __forceinline__ Chain dense_chain(const float* ht, const uint32_t* hi
 //  * A point with more than kHits crossings, and every point of a warp whose lists are long,
 //    is taken by the whole warp: up to kDenseHits crossings, walked by repeated minima.
 //    Beyond that overflow() takes the point.
+// (b, cnt, units: the point's list and units, grid_cell; cnt 0 for a lane with nothing to test.)
 template <int AXIS, class Ovf>
 __device__ __forceinline__ void pim_grid_warp(const GridView& g, const float4* __restrict__ tris, const float* p,
-                                              bool valid, bool keep, uint64_t i, int32_t* __restrict__ out_obj,
-                                              uint8_t* __restrict__ out_in, GridWarpSlots& sl, Ovf&& overflow) {
+                                              bool valid, uint32_t b, uint32_t cnt, uint32_t units, uint64_t i,
+                                              int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
+                                              GridWarpSlots& sl, Ovf&& overflow) {
     constexpr unsigned int kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned int below = (1u << lane) - 1u;
     const float dx = AXIS == 0 ? 1.0f : 0.0f, dy = AXIS == 1 ? 1.0f : 0.0f, dz = AXIS == 2 ? 1.0f : 0.0f;
-    uint32_t b = 0, cnt = 0, units = 0;
-    if (keep) grid_cell<AXIS>(g, p, b, cnt, units);
     const unsigned int listed = __ballot_sync(kAll, cnt != 0);
     if (listed == 0) {
         if (valid) write_result(Chain{}, i, out_obj, out_in);
@@ -385,6 +389,59 @@ __device__ __forceinline__ void pim_grid_warp(const GridView& g, const float4* _
         __syncwarp();
     }
     add_tests(lane == 0 ? tests : 0u);
+}
+
+// Points first, first + stride, ... below end, one per lane and round (first: this lane's
+// point; every lane of a warp runs the same rounds): load(i, p) reads a point, keep(p)
+// filters it.  Points without candidates are answered at once; the others wait in shared
+// memory until they fill a round of pim_grid_warp, which otherwise runs two thirds empty for
+// points spread over a box around the mesh.
+template <int AXIS, class Load, class Keep, class Ovf>
+__device__ __forceinline__ void grid_points(const GridView& g, const float4* __restrict__ tris, uint64_t first,
+                                            uint64_t end, uint64_t stride, int32_t* __restrict__ out_obj,
+                                            uint8_t* __restrict__ out_in, GridWarpSlots& sl, Load&& load, Keep&& keep,
+                                            Ovf&& overflow) {
+    const int lane = threadIdx.x & 31;
+    uint32_t head = 0, waiting = 0;
+    float p[3] = {0.0f, 0.0f, 0.0f};
+    uint64_t i = first;
+    if (i < end) load(i, p);
+    bool more = i - lane < end;  // warp-uniform: lane 0 has the least number of the round
+    while (more || waiting) {
+        if (more) {
+            uint32_t b = 0, cnt = 0, units = 0;
+            const bool valid = i < end;
+            if (valid && keep(p)) grid_cell<AXIS>(g, p, b, cnt, units);
+            if (valid && cnt == 0) write_result(Chain{}, i, out_obj, out_in);
+            const unsigned int m = __ballot_sync(0xffffffffu, cnt != 0);
+            if (cnt) {
+                const uint32_t at = (head + waiting + __popc(m & ((1u << lane) - 1u))) & 63u;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) sl.qp[q][at] = p[q];
+                sl.qb[at] = b;
+                sl.qc[at] = cnt;
+                sl.qu[at] = units;
+                sl.qi[at] = (uint32_t)i;
+            }
+            waiting += __popc(m);
+            i += stride;
+            more = i - lane < end;
+            if (i < end) load(i, p);  // on its way while this round is tested
+            __syncwarp();
+            if (waiting < 32u && more) continue;
+        }
+        const uint32_t take = min(waiting, 32u), at = (head + lane) & 63u;
+        const bool mine = (uint32_t)lane < take;
+        float t[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) t[q] = mine ? sl.qp[q][at] : 0.0f;
+        const uint32_t k = mine ? sl.qi[at] : 0u;
+        pim_grid_warp<AXIS>(g, tris, t, mine, mine ? sl.qb[at] : 0u, mine ? sl.qc[at] : 0u, mine ? sl.qu[at] : 0u, k,
+                            out_obj, out_in, sl, [&]() { overflow(k); });
+        head += take;
+        waiting -= take;
+        __syncwarp();
+    }
 }
 
 // Exact fallback for a ray with more than kHits crossings: each round re-traverses the
