@@ -79,6 +79,14 @@ __device__ __forceinline__ bool box_filter(const BoxBounds& box, const Ray& r) {
 }
 
 
+// Leaves ray i to the fallback.  *left (pinned host memory, nullable) tells the host that
+// there is one, so that a query without any needs no read-back of the count.
+__device__ __forceinline__ void leave_ray(uint32_t* __restrict__ ovf_list, unsigned long long* __restrict__ ovf_count,
+                                          volatile int* left, uint32_t i) {
+    ovf_list[atomicAdd(ovf_count, 1ull)] = i;
+    if (left) *left = 1;
+}
+
 // BVH traversal in ray packets, for directions without a column grid.  Rays of more
 // crossings than a packet keeps, or of a packet without room, go to the fallback.
 constexpr int kPimT = 128;
@@ -89,7 +97,8 @@ __global__ void __launch_bounds__(kPimT, 6) k_pim(const float* __restrict__ pts,
                                                   const float4* __restrict__ tris, BoxBounds box,
                                                   int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
                                                   uint32_t* __restrict__ ovf_list,
-                                                  unsigned long long* __restrict__ ovf_count) {
+                                                  unsigned long long* __restrict__ ovf_count,
+                                                  volatile int* __restrict__ left) {
     __shared__ RayPacket packets[kPimT / 32];
     RayPacket& sm = packets[threadIdx.x >> 5];
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -103,7 +112,7 @@ __global__ void __launch_bounds__(kPimT, 6) k_pim(const float* __restrict__ pts,
     const bool ok = packet_trace<AXIS>(sm, r, keep, 0, nodes, max_steps, tris);
     const int hits = keep ? sm.n[threadIdx.x & 31] : 0;
     if (!valid) return;
-    if (keep && (!ok || hits > kPacketHits)) ovf_list[atomicAdd(ovf_count, 1ull)] = (uint32_t)i;
+    if (keep && (!ok || hits > kPacketHits)) leave_ray(ovf_list, ovf_count, left, (uint32_t)i);
     else write_result(packet_chain(sm, tris, hits), i, out_obj, out_in);
 }
 
@@ -116,7 +125,8 @@ __global__ void __launch_bounds__(kT, kGridBlocks) k_pim_grid(const float* __res
                                                  const float4* __restrict__ tris, BoxBounds box,
                                                  int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
                                                  uint32_t* __restrict__ ovf_list,
-                                                 unsigned long long* __restrict__ ovf_count) {
+                                                 unsigned long long* __restrict__ ovf_count,
+                                                 volatile int* __restrict__ left) {
     __shared__ GridWarpSlots slots[kWarps];
     grid_points<AXIS>(
         g, tris, blockIdx.x * (uint64_t)kT + threadIdx.x, n, (uint64_t)gridDim.x * kT, out_obj, out_in,
@@ -130,7 +140,7 @@ __global__ void __launch_bounds__(kT, kGridBlocks) k_pim_grid(const float* __res
                                                              AXIS == 1 ? 1.0f : 0.0f, AXIS == 2 ? 1.0f : 0.0f, kEps,
                                                              kTmax));
         },
-        [&](uint32_t i) { ovf_list[atomicAdd(ovf_count, 1ull)] = i; });
+        [&](uint32_t i) { leave_ray(ovf_list, ovf_count, left, i); });
 }
 
 // Exact fallback for rays with more than kHits crossings (pim_fallback_ray).
@@ -403,16 +413,16 @@ unsigned grid_blocks(uint64_t n) {
 template <int AXIS, bool FILTER>
 cudaError_t launch_pim(const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz,
                        const BoxBounds& box, int32_t* obj, uint8_t* in, uint32_t* ovf_list,
-                       unsigned long long* ovf_count, cudaStream_t s) {
+                       unsigned long long* ovf_count, volatile int* left, cudaStream_t s) {
     constexpr int GA = AXIS < 0 ? 0 : AXIS;
     const int ptok = prof_begin(P_PIM, s);
     if (AXIS >= 0 && bvh->cgrid[GA].built) {
         const GridView g = grid_view(bvh->cgrid[GA]);
-        launch(k_pim_grid<GA, FILTER>, grid_blocks(n), kT, 0, s, pts, n, g, (const float4*)bvh->tris, box, obj, in, ovf_list,
-               ovf_count);
+        launch(k_pim_grid<GA, FILTER>, grid_blocks(n), kT, 0, s, pts, n, g, (const float4*)bvh->tris, box, obj, in,
+               ovf_list, ovf_count, left);
     } else {
         launch(k_pim<AXIS, FILTER>, (unsigned)((n + kPimT - 1) / kPimT), kPimT, 0, s, pts, n, dx, dy, dz, bvh->nodes,
-               max_steps(bvh), (const float4*)bvh->tris, box, obj, in, ovf_list, ovf_count);
+               max_steps(bvh), (const float4*)bvh->tris, box, obj, in, ovf_list, ovf_count, left);
     }
     prof_end(P_PIM, s, ptok);
     return cudaGetLastError();
@@ -420,18 +430,23 @@ cudaError_t launch_pim(const rs_bvh* bvh, const float* pts, uint64_t n, float dx
 
 // Launches the query, waits for it, and resolves the rays it left in ovf_list (their count
 // is known then, so a query without any pays for no second launch).  meta: status word,
-// overflow count, both zero before the call; h: their host copy (pinned, or of the caller's).
+// overflow count, both zero before the call; h: their host copy.  left: a pinned word, zero
+// before the call, that says whether there is anything to read back (nullable: read back).
 template <int AXIS>
 int run_pim_axis(const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz, bool filter,
                  const BoxBounds& box, int32_t* obj, uint8_t* in, unsigned long long* meta, unsigned long long* h,
-                 uint32_t* ovf, cudaStream_t s) {
+                 volatile int* left, uint32_t* ovf, cudaStream_t s) {
     unsigned int* status = reinterpret_cast<unsigned int*>(meta);
-    cudaError_t e = filter ? launch_pim<AXIS, true>(bvh, pts, n, dx, dy, dz, box, obj, in, ovf, meta + 1, s)
-                           : launch_pim<AXIS, false>(bvh, pts, n, dx, dy, dz, box, obj, in, ovf, meta + 1, s);
+    cudaError_t e = filter ? launch_pim<AXIS, true>(bvh, pts, n, dx, dy, dz, box, obj, in, ovf, meta + 1, left, s)
+                           : launch_pim<AXIS, false>(bvh, pts, n, dx, dy, dz, box, obj, in, ovf, meta + 1, left, s);
     constexpr size_t kWords = 2 * sizeof(unsigned long long);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, meta, kWords, cudaMemcpyDeviceToHost, s);
     cudaError_t e2 = cudaStreamSynchronize(s);
     if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess && (!left || *left)) {
+        e = cudaMemcpyAsync(h, meta, kWords, cudaMemcpyDeviceToHost, s);
+        e2 = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = e2;
+    }
     if (e == cudaSuccess && h[1]) {
         launch(k_pim_fallback<AXIS>, (unsigned)((h[1] + kT - 1) / kT), kT, 0, s, pts, dx, dy, dz, bvh->nodes,
                max_steps(bvh), (const float4*)bvh->tris, obj, in, status, (const uint32_t*)ovf,
@@ -454,12 +469,12 @@ int pim_axis(float dx, float dy, float dz) {
 
 int run_pim(int axis, const rs_bvh* bvh, const float* pts, uint64_t n, float dx, float dy, float dz, bool filter,
             const BoxBounds& box, int32_t* obj, uint8_t* in, unsigned long long* meta, unsigned long long* h,
-            uint32_t* ovf, cudaStream_t s) {
+            volatile int* left, uint32_t* ovf, cudaStream_t s) {
     switch (axis) {
-        case 0: return run_pim_axis<0>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, h, ovf, s);
-        case 1: return run_pim_axis<1>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, h, ovf, s);
-        case 2: return run_pim_axis<2>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, h, ovf, s);
-        default: return run_pim_axis<-1>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, h, ovf, s);
+        case 0: return run_pim_axis<0>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, h, left, ovf, s);
+        case 1: return run_pim_axis<1>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, h, left, ovf, s);
+        case 2: return run_pim_axis<2>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, h, left, ovf, s);
+        default: return run_pim_axis<-1>(bvh, pts, n, dx, dy, dz, filter, box, obj, in, meta, h, left, ovf, s);
     }
 }
 
@@ -475,8 +490,8 @@ BoxBounds make_box(const rs_bvh* bvh) {
 }
 
 // The status word and overflow count of a call, device memory that is zero while it waits in
-// its device's pool, and a pinned copy of it: a call then needs neither an allocation nor a
-// memset for them, and its read-back no staging.  A call has one to itself until it has
+// its device's pool, and pinned words for their copy and run_pim's `left`: a call then needs
+// neither an allocation nor a memset for them, and a copy back only when rays were left.  A call has one to itself until it has
 // synchronised, so calls on other streams and threads have others.
 struct CallWords {
     unsigned long long* dev = nullptr;
@@ -548,8 +563,9 @@ int pim_impl(const rs_bvh* cbvh, const float* pts, uint64_t n, float dx, float d
         return to_status(e);
     }
     const BoxBounds box = filter ? make_box(bvh) : BoxBounds{};
-    words.host[0] = words.host[1] = 0;
-    st = run_pim(axis, bvh, pts, n, dx, dy, dz, filter, box, obj, in, words.dev, words.host, ovf, s);
+    words.host[0] = words.host[1] = words.host[2] = 0;
+    st = run_pim(axis, bvh, pts, n, dx, dy, dz, filter, box, obj, in, words.dev, words.host,
+                 reinterpret_cast<volatile int*>(words.host + 2), ovf, s);
     cudaFreeAsync(ovf, s);
     words_release(device, words, st == RS_OK && words.host[0] == 0 && words.host[1] == 0, s);
     return st;
@@ -764,7 +780,7 @@ extern "C" int rs_pim_noalloc(const rs_bvh* bvh, const float* d_points, uint64_t
     // building it allocates.  Without it the BVH path gives the same results.
     unsigned long long h[2] = {0, 0};
     return run_pim(pim_axis(dx, dy, dz), bvh, d_points, n, dx, dy, dz, filtered != 0, box, d_obj, d_inside, meta, h,
-                   ovf, s);
+                   nullptr, ovf, s);
 }
 
 extern "C" int rs_pim(const rs_bvh* bvh, const float* d_points, uint64_t n, float dx, float dy, float dz,
