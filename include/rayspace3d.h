@@ -112,7 +112,9 @@ int rs_compact_hits(const int32_t* d_obj, uint64_t n, int32_t* d_point_ids, int3
 /* Pair tables (the hash tables of query/src/cuda/mesh_overlap_edges.cu:62-104 and
  * mesh_intersection.cu:108-132).  pow2 != 0: capacity is rounded up to a power of two and
  * slots are hash & (capacity-1); pow2 == 0: slot = hash % capacity (the intersection
- * variant).  A key that finds no slot raises RS_ERR_TABLE_FULL instead of being dropped. */
+ * variant).  A key that finds no slot raises RS_ERR_TABLE_FULL instead of being dropped.
+ * rs_pairset_create returns once the table's clearing is queued on `stream`; every entry
+ * point that takes the table orders its own stream after that. */
 int rs_pairset_create(uint64_t capacity, int pow2, rs_pairset** out, void* stream);
 int rs_pairset_clear(rs_pairset* ps, void* stream);
 int rs_pairset_destroy(rs_pairset* ps);

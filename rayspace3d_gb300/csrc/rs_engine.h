@@ -77,6 +77,11 @@ struct rs_pairset {
     // meta[1] as last read by the host with status ok, while no launch has been given the
     // table since (table_view() resets it); -1 when unknown.
     long long known_count = -1;
+    // Recorded after the allocation and first clearing, which rs_pairset_create only queues:
+    // every entry point orders its stream after it (ps_use).
+    cudaEvent_t ready = nullptr;
+    // Cleared (slots, words, overflow table) and given to no launch since.
+    bool pristine = false;
 };
 
 namespace rs {
@@ -92,6 +97,10 @@ int table_status(rs_pairset* ps, cudaStream_t s, cudaError_t e);
 // its overflow table: new slots with room for all of them, both tables' keys reinserted,
 // the overflow table cleared.
 cudaError_t table_regrow(rs_pairset* ps, uint64_t count, uint64_t over, cudaStream_t s);
+// Orders work queued on stream s after the table's creation.
+cudaError_t ps_use(const rs_pairset* ps, cudaStream_t s);
+// Queues the clearing of a table for a join, unless it is pristine.
+cudaError_t table_clear(rs_pairset* ps, cudaStream_t s);
 // Queues the clearing of the overflow table (and its count) when a launch may have used it.
 cudaError_t over_clear(rs_pairset* ps, cudaStream_t s);
 // Upper bound on the node visits of one traversal of a valid tree.

@@ -1390,6 +1390,7 @@ int recheck_join(int op, unsigned long long* out) { return recheck_op(op, out); 
 
 PairTable table_view(rs_pairset* ps) {
     ps->known_count = -1;  // a launch is about to insert
+    ps->pristine = false;
     PairTable t;
     t.slots = ps->slots;
     t.capacity = ps->capacity;
@@ -1806,7 +1807,8 @@ extern "C" int rs_edge_join(const rs_bvh* target, const float* d_starts, const f
     if (!target || !ps || (nE && (!d_starts || !d_ends || !d_offsets || !d_counts || !d_sources)))
         return RS_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
-    const int st = bvh_use(target, s);
+    int st = bvh_use(target, s);
+    if (st == RS_OK) st = to_status(ps_use(ps, s));
     if (st != RS_OK) return st;
     cudaError_t e = edge_join_async(target, d_starts, d_ends, d_offsets, d_counts, d_sources, nE, swap, ps, s,
                                     EdgeCull{});
@@ -1819,7 +1821,8 @@ extern "C" int rs_triangle_join(const rs_bvh* target, const float* d_vertices, u
     const uint64_t m = 3 * nF;
     if (m == 0 || target->n_tris == 0) return RS_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    const int st = bvh_use(target, s);
+    int st = bvh_use(target, s);
+    if (st == RS_OK) st = to_status(ps_use(ps, s));
     if (st != RS_OK) return st;
     // bad flag and deferred count in one zeroed pair; records as 32-bit ids when they fit
     // (else every record runs the long path in the first kernel).
@@ -1886,7 +1889,8 @@ static int containment_impl(const rs_bvh* target, const float* d_src_vertices, u
                             rs_pairset* ps, const Tracking* trk, uint64_t trk_capacity, cudaStream_t s) {
     if (!target || !ps || (src_nF && (!d_src_vertices || !d_src_indices || !d_src_tri2obj))) return RS_ERR_INVALID;
     if (src_nF == 0 || target->n_tris == 0) return RS_OK;
-    const int st = bvh_use(target, s);
+    int st = bvh_use(target, s);
+    if (st == RS_OK) st = to_status(ps_use(ps, s));
     if (st != RS_OK) return st;
     int* dmx = nullptr;
     int hmx = -1;

@@ -56,6 +56,7 @@ uint64_t next_pow2(uint64_t v) {
 
 cudaError_t alloc_slots(rs_pairset* ps, uint64_t capacity, cudaStream_t s) {
     ps->known_count = -1;
+    ps->pristine = false;
     if (ps->slots) cudaFreeAsync(ps->slots, s);
     ps->slots = nullptr;
     ps->capacity = capacity;
@@ -65,6 +66,14 @@ cudaError_t alloc_slots(rs_pairset* ps, uint64_t capacity, cudaStream_t s) {
 }
 
 namespace {
+// A new table's words: kMetaWords zeros, then empty overflow slots; and its empty slots.
+__global__ void __launch_bounds__(256) k_table_init(unsigned long long* __restrict__ meta,
+                                                    unsigned long long* __restrict__ slots, uint64_t capacity) {
+    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = i0; i < kMetaWords + kOverSlots; i += stride) meta[i] = i < kMetaWords ? 0ull : kEmptyKey;
+    for (uint64_t i = i0; i < capacity; i += stride) slots[i] = kEmptyKey;
+}
+
 // Reinserts the keys of a spilled table's old slots (n_slots) and of its overflow table
 // (n_over slots) into the regrown table, skipping empty slots.
 __global__ void __launch_bounds__(256) k_rehash(PairTable t, const unsigned long long* __restrict__ keys,
@@ -77,6 +86,19 @@ __global__ void __launch_bounds__(256) k_rehash(PairTable t, const unsigned long
     }
 }
 }  // namespace
+
+cudaError_t ps_use(const rs_pairset* ps, cudaStream_t s) {
+    return ps->ready ? cudaStreamWaitEvent(s, ps->ready, 0) : cudaSuccess;
+}
+
+cudaError_t table_clear(rs_pairset* ps, cudaStream_t s) {
+    if (ps->pristine) return cudaSuccess;
+    ps->known_count = -1;
+    cudaError_t e = cudaMemsetAsync(ps->slots, 0xff, ps->capacity * sizeof(unsigned long long), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ps->meta, 0, kMetaWords * sizeof(unsigned long long), s);
+    if (e == cudaSuccess) e = over_clear(ps, s);
+    return e;
+}
 
 cudaError_t over_clear(rs_pairset* ps, cudaStream_t s) {
     if (!ps->over || !ps->over_dirty) return cudaSuccess;
@@ -179,33 +201,43 @@ extern "C" int rs_pairset_create(uint64_t capacity, int pow2, rs_pairset** out, 
     cudaGetDevice(&ps->device);
     ps->pow2 = pow2 ? 1 : 0;
     if (ps->pow2) capacity = next_pow2(capacity);
+    // Two synchronisations and five memsets cost a join up to 90 us here, waiting behind its own
+    // builds: the clearing is queued, in one kernel, and the table's users wait for it.
     cudaError_t e = dmalloc((void**)&ps->meta, (kMetaWords + kOverSlots) * sizeof(unsigned long long), s);
+    if (e == cudaSuccess) e = alloc_slots(ps, capacity, s);
     if (e == cudaSuccess) {
         ps->over = ps->meta + kMetaWords;
-        ps->over_dirty = true;  // cleared below
-        e = over_clear(ps, s);
+        const uint64_t n = std::max<uint64_t>(capacity, kOverSlots);
+        launch(k_table_init, (unsigned)std::min<uint64_t>((n + 1023) / 1024, 8ull * sm_count()), 256, 0, s, ps->meta,
+               ps->slots, capacity);
+        e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = alloc_slots(ps, capacity, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ps->ready, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(ps->ready, s);
     if (e != cudaSuccess) {
+        cudaStreamSynchronize(s);
+        if (ps->ready) cudaEventDestroy(ps->ready);
         if (ps->meta) cudaFree(ps->meta);
         if (ps->slots) cudaFree(ps->slots);
         delete ps;
         return to_status(e);
     }
+    ps->known_count = 0;
+    ps->pristine = true;
     *out = ps;
-    return rs_pairset_clear(ps, stream);
+    return RS_OK;
 }
 
 extern "C" int rs_pairset_clear(rs_pairset* ps, void* stream) {
     if (!ps) return RS_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
-    ps->known_count = -1;
-    cudaError_t e = cudaMemsetAsync(ps->slots, 0xff, ps->capacity * sizeof(unsigned long long), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ps->meta, 0, kMetaWords * sizeof(unsigned long long), s);
-    if (e == cudaSuccess) e = over_clear(ps, s);
+    cudaError_t e = ps_use(ps, s);
+    if (e == cudaSuccess) e = table_clear(ps, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess) ps->known_count = 0;
+    if (e == cudaSuccess) {
+        ps->known_count = 0;
+        ps->pristine = true;
+    }
     return to_status(e);
 }
 
@@ -214,6 +246,10 @@ extern "C" int rs_pairset_destroy(rs_pairset* ps) {
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(ps->device);
+    if (ps->ready) {
+        cudaEventSynchronize(ps->ready);
+        cudaEventDestroy(ps->ready);
+    }
     if (ps->slots) cudaFree(ps->slots);
     if (ps->meta) cudaFree(ps->meta);
     cudaSetDevice(prev);
@@ -229,7 +265,8 @@ extern "C" int rs_pairset_info(const rs_pairset* ps, uint64_t* capacity, uint64_
     } else if (count) {
         cudaStream_t s = (cudaStream_t)stream;
         unsigned long long c = 0;
-        cudaError_t e = cudaMemcpyAsync(&c, ps->meta + 1, sizeof(c), cudaMemcpyDeviceToHost, s);
+        cudaError_t e = ps_use(ps, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&c, ps->meta + 1, sizeof(c), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) return to_status(e);
         *count = c;
@@ -244,7 +281,8 @@ extern "C" int rs_pairset_finalize(rs_pairset* ps, int order, uint64_t* d_keys, 
     if (!ps || !h_count || (capacity && !d_keys)) return RS_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
     *h_count = 0;
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = ps_use(ps, s);
+    if (e != cudaSuccess) return to_status(e);
     // The status and count: from the last read when no launch has touched the table since.
     uint64_t n = 0;
     if (ps->known_count >= 0) {
@@ -263,6 +301,22 @@ extern "C" int rs_pairset_finalize(rs_pairset* ps, int order, uint64_t* d_keys, 
         prof_end(P_FINALIZE, s, ptok);
         if (e == cudaSuccess && !no_wait) e = cudaStreamSynchronize(s);
         if (!no_wait) prof_collect();
+        if (e != cudaSuccess) return to_status(e);
+        *h_count = n;
+        return RS_OK;
+    }
+    if (n <= kTilesTableSort && n <= capacity) {
+        uint64_t* tiles = nullptr;
+        const int ptok = prof_begin(P_FINALIZE, s);
+        e = dmalloc((void**)&tiles, n * sizeof(uint64_t), s);
+        if (e == cudaSuccess)
+            e = table_keys_sorted_tiles(reinterpret_cast<const uint64_t*>(ps->slots), ps->capacity, kEmptyKey,
+                                        order == 1 ? 1 : 0, d_keys, n, tiles, ps->meta + kGatherWord, s);
+        prof_end(P_FINALIZE, s, ptok);
+        if (tiles) cudaFreeAsync(tiles, s);
+        const cudaError_t e2 = cudaStreamSynchronize(s);
+        prof_collect();
+        if (e == cudaSuccess) e = e2;
         if (e != cudaSuccess) return to_status(e);
         *h_count = n;
         return RS_OK;
@@ -328,6 +382,7 @@ static int overlap_join_impl(const rs_bvh* A, const float* d_startsA, const floa
         if (st == RS_OK) st = bvh_ready(B);
         if (st == RS_OK) st = bvh_use(A, s);
         if (st == RS_OK) st = bvh_use(B, s);
+        if (st == RS_OK) st = to_status(ps_use(ps, s));
         if (st != RS_OK) return st;
     }
     // Broad phase once per call (it does not depend on the table, so reruns after growth
@@ -369,10 +424,7 @@ static int overlap_join_impl(const rs_bvh* A, const float* d_startsA, const floa
         // Order of executeHashQuery (raytracer_intersection_estimated_main.cpp:107-158): overlap A->B,
         // overlap B->A, containment A->B, containment B->A, queued back to back and checked with
         // one status read.
-        ps->known_count = -1;
-        cudaError_t e = cudaMemsetAsync(ps->slots, 0xff, ps->capacity * sizeof(unsigned long long), s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(ps->meta, 0, kMetaWords * sizeof(unsigned long long), s);
-        if (e == cudaSuccess) e = over_clear(ps, s);
+        cudaError_t e = table_clear(ps, s);
         // Both directions with their broad phase and no events: one live-edge launch for both,
         // and the two directions' rays concurrently.  Otherwise each direction reads its
         // source edges only after the caller's event for them.
@@ -471,7 +523,8 @@ extern "C" int rs_pairset_counters(const rs_pairset* ps, uint64_t* h_out8, void*
     if (!ps || !h_out8) return RS_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
     unsigned long long m[kMetaWords];
-    cudaError_t e = cudaMemcpyAsync(m, ps->meta, sizeof(m), cudaMemcpyDeviceToHost, s);
+    cudaError_t e = ps_use(ps, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(m, ps->meta, sizeof(m), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return to_status(e);
     for (int k = 0; k < 8; ++k) h_out8[k] = m[2 + k];

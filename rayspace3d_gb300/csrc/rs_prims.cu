@@ -414,8 +414,11 @@ __global__ void __launch_bounds__(kThreads) k_compact_write(const uint64_t* __re
 // Single-block bitonic sort of up to kSmallSort keys in shared memory.
 constexpr int kSmallSort = 4096;
 
-__global__ void __launch_bounds__(1024) k_sort_small(uint64_t* __restrict__ keys, int n, int swap_out) {
+// Block b sorts keys [b * kSmallSort, ...) of total keys.
+__global__ void __launch_bounds__(1024) k_sort_small(uint64_t* __restrict__ keys, uint64_t total, int swap_out) {
     __shared__ uint64_t sh[kSmallSort];
+    keys += (uint64_t)blockIdx.x * kSmallSort;
+    const int n = (int)min(total - (uint64_t)blockIdx.x * kSmallSort, (uint64_t)kSmallSort);
     int m = 1;
     while (m < n) m <<= 1;
     for (int i = threadIdx.x; i < m; i += blockDim.x) sh[i] = i < n ? keys[i] : ~0ull;
@@ -440,6 +443,29 @@ __global__ void __launch_bounds__(1024) k_sort_small(uint64_t* __restrict__ keys
         const uint64_t k = sh[i];
         keys[i] = swap_out ? (k << 32) | (k >> 32) : k;
     }
+}
+
+// Distinct keys in sorted tiles of kSmallSort, merged: a key's place is its place in its own
+// tile plus the number of smaller keys in every other tile, by binary search.
+__global__ void __launch_bounds__(256) k_merge_tiles(const uint64_t* __restrict__ keys, uint64_t n, int swap_out,
+                                                     uint64_t* __restrict__ out) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint64_t k = keys[i], mine = i / kSmallSort, tiles = (n + kSmallSort - 1) / kSmallSort;
+    uint64_t pos = i % kSmallSort;
+    for (uint64_t t = 0; t < tiles; ++t) {
+        if (t == mine) continue;
+        const uint64_t* x = keys + t * kSmallSort;
+        uint32_t lo = 0, len = (uint32_t)min(n - t * kSmallSort, (uint64_t)kSmallSort);
+        while (len > 0) {  // first key of the tile that is not below k
+            const uint32_t half = len >> 1;
+            const bool right = __ldg(&x[lo + half]) < k;
+            lo = right ? lo + half + 1 : lo;
+            len = right ? len - half - 1 : half;
+        }
+        pos += lo;
+    }
+    out[pos] = swap_out ? (k << 32) | (k >> 32) : k;
 }
 
 // The keys of a hash table (slots not equal to `empty`) appended to out in any order,
@@ -471,14 +497,27 @@ cudaError_t table_keys_sorted_small(const uint64_t* slots, uint64_t capacity, ui
     const uint64_t blocks = std::min<uint64_t>((capacity + 255) / 256, 4ull * sm_count());
     launch(k_table_gather, (unsigned)std::max<uint64_t>(blocks, 1), 256, 0, s, slots, capacity, empty, swap, out, n,
            counter);
-    launch(k_sort_small, 1, 1024, 0, s, out, (int)n, swap);
+    launch(k_sort_small, 1, 1024, 0, s, out, n, swap);
+    return cudaGetLastError();
+}
+
+cudaError_t table_keys_sorted_tiles(const uint64_t* slots, uint64_t capacity, uint64_t empty, int swap, uint64_t* out,
+                                    uint64_t n, uint64_t* tmp, unsigned long long* counter, cudaStream_t s) {
+    if (n > kTilesTableSort) return cudaErrorInvalidValue;
+    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s);
+    if (e != cudaSuccess || n == 0) return e;
+    const uint64_t blocks = std::min<uint64_t>((capacity + 255) / 256, 4ull * sm_count());
+    launch(k_table_gather, (unsigned)std::max<uint64_t>(blocks, 1), 256, 0, s, slots, capacity, empty, swap, tmp, n,
+           counter);
+    launch(k_sort_small, (unsigned)((n + kSmallSort - 1) / kSmallSort), 1024, 0, s, tmp, n, 0);
+    launch(k_merge_tiles, (unsigned)((n + 255) / 256), 256, 0, s, (const uint64_t*)tmp, n, swap, out);
     return cudaGetLastError();
 }
 
 cudaError_t sort_u64_any(uint64_t* keys, size_t n, cudaStream_t s) {
     if (n <= 1) return cudaSuccess;
     if (n <= (size_t)kSmallSort) {
-        launch(k_sort_small, 1, 1024, 0, s, keys, (int)n, 0);
+        launch(k_sort_small, 1, 1024, 0, s, keys, (uint64_t)n, 0);
         return cudaGetLastError();
     }
     return radix_sort_u64(keys, nullptr, n, 64, s);

@@ -39,6 +39,14 @@ constexpr uint64_t kSmallTableSort = 4096;
 cudaError_t table_keys_sorted_small(const uint64_t* slots, uint64_t capacity, uint64_t empty, int swap, uint64_t* out,
                                     uint64_t n, unsigned long long* counter, cudaStream_t s);
 
+// The same for n <= kTilesTableSort: tiles of kSmallTableSort keys sorted by a block each in
+// tmp (n keys), then merged by rank.  Three kernels where compaction, half swaps and the
+// eight radix passes of so short a list take sixteen (9,072 keys: 152 us of a join's 2.4 ms,
+// against 45).
+constexpr uint64_t kTilesTableSort = 65536;
+cudaError_t table_keys_sorted_tiles(const uint64_t* slots, uint64_t capacity, uint64_t empty, int swap, uint64_t* out,
+                                    uint64_t n, uint64_t* tmp, unsigned long long* counter, cudaStream_t s);
+
 // Exclusive prefix sums.  `total` (device, nullable) receives the sum of all inputs.
 cudaError_t exclusive_scan_u32(const uint32_t* in, uint32_t* out, size_t n, uint32_t* total, cudaStream_t s);
 cudaError_t exclusive_scan_i32_to_i64(const int32_t* in, int64_t* out, size_t n, int64_t* total, cudaStream_t s);
