@@ -322,7 +322,7 @@ float dec_ord(int i) {
 // most kEntries a triangle, since many small objects over a wide scene would otherwise list
 // every triangle in a hundred cells and more.  Up to kFree entries the build takes no longer
 // than its launches and stays at four cells a triangle.
-constexpr double kEntries = 12.0;
+constexpr double kEntries = 8.0;
 constexpr double kFree = 4194304.0;
 
 double grid_cells(double n, double w, double h, const double* sum) {

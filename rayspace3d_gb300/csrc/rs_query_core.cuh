@@ -225,6 +225,25 @@ constexpr uint32_t kDenseCandidates = 48;
 __device__ __forceinline__ Chain dense_chain(const float* ht, const uint32_t* hid, const int32_t* hobj, int nh,
                                              int lane) {
     Chain ch;
+    if (nh <= 32) {
+        // Crossings that all lie a step or more apart are all counted, in whatever order they
+        // were found, up to the first that a step does not move: almost every ray, and a third
+        // of the instructions of the minima below.
+        const bool mine = lane < nh;
+        const float t = mine ? ht[lane] : INFINITY, nt = __fadd_rn(t, kEps);
+        bool close = mine && !(t >= kEps && t < kTmax);
+        for (int j = 0; j < nh; ++j) {
+            const float o = __shfl_sync(0xffffffffu, t, j);
+            close |= mine && j != lane && o >= t && o < nt;
+        }
+        if (!__any_sync(0xffffffffu, close)) {
+            const uint32_t near = __reduce_min_sync(0xffffffffu, __float_as_uint(t));
+            const unsigned int first = __ballot_sync(0xffffffffu, mine && __float_as_uint(t) == near);
+            ch.count = __any_sync(0xffffffffu, mine && !(nt > t)) ? kPimMaxIters : (uint32_t)nh;
+            if (first) ch.first_obj = hobj[__ffs(first) - 1];
+            return ch;
+        }
+    }
     for (;;) {
         uint32_t best = 0xffffffffu;
         for (int h = lane; h < nh; h += 32) {
