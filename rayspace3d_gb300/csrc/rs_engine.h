@@ -116,7 +116,7 @@ int ensure_grid(const rs_bvh* h, int axis, cudaStream_t s);
 // have a partner; no culling when cand is null.  With partner lists (part != null):
 // cand[o] = the number of partner objects of the other set (0..kPartners) listed in
 // part[o * kPartners ...], or kCandAll when they were not all collected; pbox holds the
-// other set's object boxes (ordered-int min xyz, max xyz), n_pbox of them.  entry
+// other set's object boxes, widened (two float4: min xyz, max xyz), n_pbox of them.  entry
 // (nullable, with part): per source object whose flag is set, the node of the other set's
 // BVH under which lie all triangles its edges' rays can hit; they start there.
 constexpr int kPartners = 8;
@@ -125,11 +125,11 @@ struct EdgeCull {
     const uint8_t* cand = nullptr;
     uint64_t n_obj = 0;
     const int32_t* part = nullptr;
-    const int* pbox = nullptr;
+    const float4* pbox = nullptr;
     uint64_t n_pbox = 0;
     const uint32_t* entry = nullptr;
     // Slab index of the source payload (rs_edge_index; nullable) and the source objects' own
-    // boxes (as pbox): with both, only the payload's slabs that can hold an edge of an object
+    // boxes (ordered-int min xyz, max xyz): with both, only the payload's slabs that can hold an edge of an object
     // with a partner are checked for live edges.
     const long long* xindex = nullptr;
     const int* sbox = nullptr;

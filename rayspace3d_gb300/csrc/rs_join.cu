@@ -355,7 +355,7 @@ struct EdgeJob {
     const uint8_t* cull;  // flag (or partner count) per source object below n_cull
     uint64_t n_cull;
     const int32_t* part;  // partner lists (nullable), as EdgeCull
-    const int* pbox;      // the target set's object boxes
+    const float4* pbox;   // the target set's object boxes, widened
     uint64_t n_pbox;
     uint32_t* live;       // live edges, in arrival order
     uint32_t* rank;       // rank of each live edge within its cell; then the deferred edges
@@ -405,6 +405,32 @@ __device__ __forceinline__ uint32_t edge_cell(const EdgeJob& j, uint64_t i) {
     return code;
 }
 
+// Eight 32-bit values from a 32-byte boundary.
+__device__ __forceinline__ void load_ints8(const int32_t* __restrict__ p, int32_t (&v)[8]) {
+    asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "l"(p));
+}
+
+// Both sets' object boxes widened by their margins, as box_overlaps widens them.
+__global__ void __launch_bounds__(256) k_wide_boxes(const int* __restrict__ boxA, uint64_t nA,
+                                                    const int* __restrict__ boxB, uint64_t nB,
+                                                    float4* __restrict__ out) {
+    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (i >= nA + nB) return;
+    const int* ob = i < nA ? boxA + 6 * i : boxB + 6 * (i - nA);
+    float lo[3], hi[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float l = ord2f(ob[k]), h = ord2f(ob[3 + k]);
+        const float m = cull_margin(l, h);
+        lo[k] = l - m;
+        hi[k] = h + m;
+    }
+    out[2 * i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
+    out[2 * i + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+}
+
 // Whether edge i of job j is live, given its source count ns, its source list sp, and its
 // first source so0 with that object's flag c0 (loaded by the caller).
 __device__ __forceinline__ bool edge_is_live(const EdgeJob& j, uint64_t i, int ns, const int32_t* sp, int32_t so0,
@@ -422,10 +448,18 @@ __device__ __forceinline__ bool edge_is_live(const EdgeJob& j, uint64_t i, int n
             edge_query_box(j.p, i, qlo, qhi);
             have_box = true;
         }
-        const int32_t* pl = j.part + (uint64_t)so * kPartners;
-        for (int k = 0; k < (int)c; ++k) {
-            const int32_t b = pl[k];
-            if (b < 0 || (uint64_t)b >= j.n_pbox || box_overlaps(j.pbox + 6 * (uint64_t)b, qlo, qhi)) return true;
+        // The list and each partner's box by one 32-byte load.
+        int32_t pl[kPartners];
+        load_ints8(j.part + (uint64_t)so * kPartners, pl);
+#pragma unroll
+        for (int k = 0; k < kPartners; ++k) {
+            if (k >= (int)c) break;
+            if (pl[k] < 0 || (uint64_t)pl[k] >= j.n_pbox) return true;
+            int32_t w[8];
+            load_ints8(reinterpret_cast<const int32_t*>(j.pbox + 2 * (uint64_t)pl[k]), w);
+            if (__int_as_float(w[0]) <= qhi[0] && __int_as_float(w[4]) >= qlo[0] && __int_as_float(w[1]) <= qhi[1] &&
+                __int_as_float(w[5]) >= qlo[1] && __int_as_float(w[2]) <= qhi[2] && __int_as_float(w[6]) >= qlo[2])
+                return true;
         }
     }
     return false;
@@ -436,38 +470,69 @@ __device__ __forceinline__ bool edge_is_live(const EdgeJob& j, uint64_t i, int n
 // rank within its cell (one warp-aggregated atomic per cell and warp).  Each thread takes
 // kLiveEdges edges (a block's edges are contiguous, kLiveEdges rounds of blockDim) and
 // issues the dependent loads of all of them together -- count and offset, first source,
-// its flag -- so that a wave of threads keeps several chains in flight.  Blocks below
-// blocks0 run job j0, the others j1.
-constexpr int kLiveEdges = 4;
+// its flag -- so that a wave of threads keeps several chains in flight.  Bound by those
+// chains' latency: two edges a thread at 32 registers (180 us for 9.6 M edges of a dense join)
+// beat four at 64 and at 40 (245, 215) and one (295).  Blocks below blocks0 run job j0, the
+// others j1.
+constexpr int kLiveEdges = 2;
 
-// Appends edge i to its job's live list when `any` (warp-collective: every lane calls it):
-// one atomic per warp, the entry node beside it, and in binned jobs the edge's rank within
-// its cell.
-__device__ __forceinline__ void live_append(const EdgeJob& j, uint64_t i, bool any, uint32_t en, int lane) {
+// Appends the block's edges first + u * kLiveThreads of each thread to their job's live list
+// where any[u] (every thread of the block calls it): one atomic per block -- one per warp and
+// round, all on one word, took most of the kernel's time -- the entry nodes beside them, and
+// in binned jobs each edge's rank within its cell.
+constexpr int kLiveThreads = 256;
+
+template <int U>
+__device__ __forceinline__ void live_append(const EdgeJob& j, uint64_t first, const bool (&any)[U],
+                                            const uint32_t (&en)[U]) {
+    constexpr int kWarps = kLiveThreads / 32;
+    static_assert(U * kWarps <= 32, "one lane per warp and round");
+    __shared__ uint32_t s_cnt[32];
+    __shared__ uint32_t s_pos;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned int below = (1u << lane) - 1u;
-    const unsigned int m = __ballot_sync(0xffffffffu, any);
-    if (!m) return;
-    const int leader = __ffs(m) - 1;
-    unsigned int pos0 = 0;
-    if (lane == leader) pos0 = atomicAdd(j.n_live, (unsigned int)__popc(m));
-    pos0 = __shfl_sync(0xffffffffu, pos0, leader);
-    const unsigned int pos = pos0 + __popc(m & below);
-    if (any) j.live[pos] = (uint32_t)i;
-    if (any && j.live_entry) j.live_entry[pos] = en;
-    if (j.order) {
-        // Every lane takes part in the match (lanes without a live edge with a cell of
-        // their own, kCells + lane), so that the mask is the full warp.
-        const uint32_t cell = any ? edge_cell(j, i) : (uint32_t)kCells + lane;
-        const unsigned int peers = __match_any_sync(0xffffffffu, cell);
-        const int first = __ffs(peers) - 1;
-        unsigned int r0 = 0;
-        if (any && lane == first) r0 = atomicAdd(&j.cells[cell], (unsigned int)__popc(peers));
-        r0 = __shfl_sync(0xffffffffu, r0, first);
-        if (any) j.rank[pos] = r0 + __popc(peers & below);
+    unsigned int m[U], some = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        m[u] = __ballot_sync(0xffffffffu, any[u]);
+        some |= m[u];
+        if (lane == 0) s_cnt[u * kWarps + warp] = __popc(m[u]);
+    }
+    if (!__syncthreads_or((int)(some != 0))) return;  // most blocks of a sparse join
+    if (warp == 0) {
+        const uint32_t c = lane < U * kWarps ? s_cnt[lane] : 0u;
+        uint32_t x = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        s_cnt[lane] = x - c;
+        if (lane == 31) s_pos = x ? atomicAdd(j.n_live, x) : 0u;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (!m[u]) continue;  // warp-uniform
+        const uint64_t i = first + (uint64_t)u * kLiveThreads;
+        const unsigned int pos = s_pos + s_cnt[u * kWarps + warp] + __popc(m[u] & below);
+        if (any[u]) j.live[pos] = (uint32_t)i;
+        if (any[u] && j.live_entry) j.live_entry[pos] = en[u];
+        if (j.order) {
+            // Every lane takes part in the match (lanes without a live edge with a cell of
+            // their own, kCells + lane), so that the mask is the full warp.
+            const uint32_t cell = any[u] ? edge_cell(j, i) : (uint32_t)kCells + lane;
+            const unsigned int peers = __match_any_sync(0xffffffffu, cell);
+            const int leader = __ffs(peers) - 1;
+            unsigned int r0 = 0;
+            if (any[u] && lane == leader) r0 = atomicAdd(&j.cells[cell], (unsigned int)__popc(peers));
+            r0 = __shfl_sync(0xffffffffu, r0, leader);
+            if (any[u]) j.rank[pos] = r0 + __popc(peers & below);
+        }
     }
 }
 
-__global__ void __launch_bounds__(256) k_edge_live(EdgeJob j0, EdgeJob j1, unsigned int blocks0) {
+__global__ void __launch_bounds__(kLiveThreads, 8) k_edge_live(EdgeJob j0, EdgeJob j1, unsigned int blocks0) {
     const bool second = blockIdx.x >= blocks0;
     const EdgeJob& j = second ? j1 : j0;
     const uint64_t base = (uint64_t)(blockIdx.x - (second ? blocks0 : 0u)) * blockDim.x * kLiveEdges + threadIdx.x;
@@ -492,13 +557,11 @@ __global__ void __launch_bounds__(256) k_edge_live(EdgeJob j0, EdgeJob j1, unsig
         // sources: the root.
         en[u] = (j.entry && in && ns[u] == 1) ? j.entry[so0[u]] : 0u;
     }
-    const int lane = threadIdx.x & 31;
+    bool any[kLiveEdges];
 #pragma unroll
-    for (int u = 0; u < kLiveEdges; ++u) {
-        const uint64_t i = base + (uint64_t)u * blockDim.x;
-        const bool any = ns[u] > 0 && edge_is_live(j, i, ns[u], j.p.sources + off[u], so0[u], c0[u]);
-        live_append(j, i, any, en[u], lane);
-    }
+    for (int u = 0; u < kLiveEdges; ++u)
+        any[u] = ns[u] > 0 && edge_is_live(j, base + (uint64_t)u * blockDim.x, ns[u], j.p.sources + off[u], so0[u], c0[u]);
+    live_append<kLiveEdges>(j, base, any, en);
 }
 
 // Slab index of an edge payload (rs_edge_index).  The reference's payload is in std::map
@@ -602,9 +665,10 @@ __global__ void __launch_bounds__(kSlab) k_edge_live_slab(EdgeJob j0, EdgeJob j1
     const int32_t so0 = ns > 0 ? j.p.sources[off] : -1;
     const bool in = ns > 0 && so0 >= 0 && (uint64_t)so0 < j.n_cull;
     const uint8_t c0 = in ? j.cull[so0] : (uint8_t)0;
-    const uint32_t en = (j.entry && in && ns == 1) ? j.entry[so0] : 0u;
-    const bool any = ns > 0 && edge_is_live(j, i, ns, j.p.sources + off, so0, c0);
-    live_append(j, i, any, en, threadIdx.x & 31);
+    const uint32_t en[1] = {(j.entry && in && ns == 1) ? j.entry[so0] : 0u};
+    const bool any[1] = {ns > 0 && edge_is_live(j, i, ns, j.p.sources + off, so0, c0)};
+    static_assert(kSlab == kLiveThreads, "one slab per block");
+    live_append<1>(j, i, any, en);
 }
 
 // Exclusive prefix sums of the kCells cell counts of each binned job, in place (one block
@@ -1730,6 +1794,13 @@ cudaError_t cull_impl(const rs_bvh* A, const rs_bvh* B, uint8_t* candA, uint8_t*
             if (p) cudaFreeAsync(p, s);
     }
     return e;
+}
+
+// Queues the widening of both sets' object boxes (cull_impl's boxes_out) into out: two
+// float4 per object, A's then B's.
+cudaError_t wide_boxes_async(const int* boxA, uint64_t nA, const int* boxB, uint64_t nB, float4* out, cudaStream_t s) {
+    launch(k_wide_boxes, (unsigned)((nA + nB + 255) / 256), 256, 0, s, boxA, nA, boxB, nB, out);
+    return cudaGetLastError();
 }
 
 // Broad-phase flags of A's objects against B's BVH into candA and of B's objects against

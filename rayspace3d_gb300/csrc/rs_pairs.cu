@@ -18,6 +18,7 @@
 
 namespace rs {
 PairTable table_view(rs_pairset* ps);
+cudaError_t wide_boxes_async(const int* boxA, uint64_t nA, const int* boxB, uint64_t nB, float4* out, cudaStream_t s);
 cudaError_t containment_async(const rs_bvh* target, const rs_bvh* src, int swap, rs_pairset* ps, cudaStream_t s);
 cudaError_t edge_join_async(const rs_bvh* target, const float* d_starts, const float* d_ends,
                             const int32_t* d_offsets, const int32_t* d_counts, const int32_t* d_sources, uint64_t nE,
@@ -397,19 +398,25 @@ static int overlap_join_impl(const rs_bvh* A, const float* d_startsA, const floa
     EdgeCull cullA, cullB;
     if (g_overlap_cull && A->n_obj && B->n_obj && A->n_tris && B->n_tris) {
         const uint64_t n_obj = A->n_obj + B->n_obj;
-        // One allocation: the partner lists, the entry nodes, then the flags.
-        cudaError_t e = dmalloc((void**)&part, n_obj * (kPartners + 1) * sizeof(int32_t) + n_obj, s);
+        // One allocation: the partner lists and the widened boxes (32 bytes an object each), the
+        // entry nodes, then the flags.
+        float4* wide = nullptr;
+        cudaError_t e = dmalloc((void**)&part, n_obj * (kPartners * sizeof(int32_t) + 2 * sizeof(float4) +
+                                                        sizeof(uint32_t) + 1), s);
+        static_assert(kPartners * sizeof(int32_t) == 32, "lists are read by one 32-byte load");
         if (e == cudaSuccess) {
-            entry = reinterpret_cast<uint32_t*>(part + n_obj * kPartners);
+            wide = reinterpret_cast<float4*>(part + n_obj * kPartners);
+            entry = reinterpret_cast<uint32_t*>(wide + 2 * n_obj);
             cand = reinterpret_cast<uint8_t*>(entry + n_obj);
         }
         if (e == cudaSuccess)
             e = cull_impl(A, B, a2b ? cand : nullptr, b2a ? cand + A->n_obj : nullptr, part,
                           part + A->n_obj * kPartners, entry, entry + A->n_obj, boxes, tmps, s);
+        if (e == cudaSuccess) e = wide_boxes_async(boxes[0], A->n_obj, boxes[1], B->n_obj, wide, s);
         if (e == cudaSuccess) {
-            if (a2b) cullA = EdgeCull{cand, A->n_obj, part, boxes[1], B->n_obj, entry, indexA, boxes[0]};
+            if (a2b) cullA = EdgeCull{cand, A->n_obj, part, wide + 2 * A->n_obj, B->n_obj, entry, indexA, boxes[0]};
             if (b2a)
-                cullB = EdgeCull{cand + A->n_obj, B->n_obj, part + A->n_obj * kPartners, boxes[0], A->n_obj,
+                cullB = EdgeCull{cand + A->n_obj, B->n_obj, part + A->n_obj * kPartners, wide, A->n_obj,
                                  entry + A->n_obj, indexB, boxes[1]};
         } else {
             cudaGetLastError();  // culling is an optimisation: run without it

@@ -320,8 +320,10 @@ float dec_ord(int i) {
 // box of w x h touches about (s w + 1)(s h + 1) cells, so n boxes make about
 // s^2 sum(w h) + s (sum w + sum h) + n list entries; cells are made larger until that is at
 // most kEntries a triangle, since many small objects over a wide scene would otherwise list
-// every triangle in a hundred cells and more.  Up to kFree entries the build takes no longer
-// than its launches and stays at four cells a triangle.
+// every triangle in a hundred cells and more.  20,000 level-2 spheres, 6.4 M triangles, asked
+// for 500,009 points: 920 M entries took 27 ms to count and list and .57 ms to ask; at 12
+// entries a triangle 0.93 + 0.99 ms, at 8 0.58 + 1.04, at 5 0.44 + 1.18.  Up to kFree entries
+// the build takes no longer than its launches and stays at four cells a triangle.
 constexpr double kEntries = 8.0;
 constexpr double kFree = 4194304.0;
 
