@@ -107,7 +107,7 @@ __device__ __noinline__ void batch_rays(const BatchQuery& Q, int qi, uint64_t r0
         const bool valid = i < r1;
         Ray r;
         if (valid) r = make_ray(Q.pts[3 * i], Q.pts[3 * i + 1], Q.pts[3 * i + 2], Q.dx, Q.dy, Q.dz, kEps, kTmax);
-        const bool ok = packet_trace<-1>(sm, r, valid, 0, Q.nodes, Q.max_steps, Q.tris);
+        const bool ok = !(packet_trace<-1>(sm, r, valid, 0, Q.nodes, Q.max_steps, Q.tris) >> (threadIdx.x & 31) & 1u);
         if (valid) {
             const int n = sm.n[threadIdx.x & 31];
             if (!ok || n > kPacketHits) batch_spill(Q, qi, i, ovf, ovf_count);

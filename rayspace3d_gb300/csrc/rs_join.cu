@@ -42,6 +42,13 @@ constexpr unsigned int kBinMinLive = 1u << 16;
 // thousand edges wait on their longest packet.  The edges it defers go to
 // deferred[0..*n_def).  entry (nullable): the node each listed edge's traversal starts from.
 constexpr int kPacketWarps = 4;
+// Steps after which a packet leaves its unfinished edges to the long path, a warp for each:
+// the order by cell puts a cluster's longest edges together, and a join otherwise ends
+// waiting for a few packets of them (2.2 and 2.4 ms for the two directions of a clustered
+// join, 14 and 6 of 24 warps an SM in flight on average; now 0.65 + 0.54 and 0.53 +
+// 1.03 ms).  512 and 128 steps: 4 % and 1 % more of it; a join whose sizes are uneven,
+// but not clustered, takes 7 us more than without a limit at 256 steps and 240 at 128.
+constexpr uint32_t kPacketSteps = 256;
 
 __global__ void __launch_bounds__(32 * kPacketWarps, 6) k_edge_rays(
     EdgePayload p, const uint32_t* __restrict__ order, const uint32_t* __restrict__ live,
@@ -73,7 +80,7 @@ __global__ void __launch_bounds__(32 * kPacketWarps, 6) k_edge_rays(
         const uint32_t e = !valid ? 0u : order ? order[j] : (uint32_t)j;
         const int start = valid && entry ? (int)entry[j] : 0;
         valid = valid && e < n_direct;  // always, for a list of this payload's edges
-        if (edge_packet(sm, p, valid, e, start, nodes, max_steps, tris, swap, table))
+        if (edge_packet(sm, p, valid, e, start, nodes, min(max_steps, kPacketSteps), tris, swap, table))
             deferred[atomicAdd(n_def, 1u)] = e;
         __syncwarp();
     }
@@ -144,8 +151,8 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
             int first[2] = {0, 0}, cnt[2] = {0, 0};
             if (node >= 0) {
                 const BNode bn = load_node(nodes, node);
-            const float4 na = bn.a, nb = bn.b, nc = bn.c;
-            const int4 nd = bn.d;
+                const float4 na = bn.a, nb = bn.b, nc = bn.c;
+                const int4 nd = bn.d;
                 const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
                 const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
                 float e, x;
@@ -215,16 +222,19 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
             r.tmax = mid;
             continue;
         }
-        if (lane == 0) {
-            const int32_t* src = p.sources + p.offsets[i];
-            const int nsrc = p.counts[i];
+        int found = 0;  // objects to insert: hobj, whose crossings are copied out
+        if (lane == 0)
             for (int a = 0; a < nh && !w.done; ++a) {
                 if (!w.take(w_sm.t2[a], table.max_hits, table.next_float)) continue;
                 if (w_sm.obj2[a] == last) continue;
                 last = w_sm.obj2[a];
-                insert_sources(table, src, nsrc, last, swap);
+                hobj[found++] = last;
             }
-        }
+        found = __shfl_sync(0xffffffffu, found, 0);
+        __syncwarp();
+        for (int a = lane; a < found; a += 32)
+            insert_sources(table, p.sources + p.offsets[i], p.counts[i], hobj[a], swap);
+        __syncwarp();
         if (!RANGES || r.tmax == tmax || __shfl_sync(0xffffffffu, (int)w.done, 0)) break;
         above = r.tmax;
         r.tmin = fmaxf(r.tmin, above);
@@ -241,10 +251,12 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
 // of the edge in one traversal (or, beyond kLongWarpHits, in a traversal per range of t; the
 // reference's walk takes at most --overlap-max-iterations of them) instead of one thread
 // re-traversing per chunk of 16, which is left for more than kLongWarpHits crossings at one
-// distance (segment_long, in lane 0).
+// distance (segment_long, in lane 0).  512 crossings take 52 KB a block of 4 warps, which
+// leaves 4 blocks an SM: 9 % less for a clustered join's long edges than 256 and 7 blocks,
+// for fewer restarts.
 constexpr int kLongWarps = 4;
 constexpr int kLongWarpStack = 256;
-constexpr int kLongWarpHits = 256;
+constexpr int kLongWarpHits = 512;
 
 __global__ void __launch_bounds__(32 * kLongWarps) k_edge_long_warp(EdgePayload p, const uint32_t* __restrict__ deferred,
                                                                     const unsigned int* __restrict__ n_def,
@@ -1373,8 +1385,8 @@ __global__ void __launch_bounds__(32 * kContWarps) k_containment(const float* __
             int leaf[2] = {0, 0}, cnt[2] = {0, 0};
             if (node >= 0) {
                 const BNode bn = load_node(nodes, node);
-            const float4 na = bn.a, nb = bn.b, nc = bn.c;
-            const int4 nd = bn.d;
+                const float4 na = bn.a, nb = bn.b, nc = bn.c;
+                const int4 nd = bn.d;
                 const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
                 const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
                 float en, ex;

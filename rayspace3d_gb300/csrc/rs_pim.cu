@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kPimT, 6) k_pim(const float* __restrict__ pts,
         r = make_ray(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], dx, dy, dz, kEps, kTmax);
         if (FILTER) keep = box_filter<AXIS>(box, r);
     }
-    const bool ok = packet_trace<AXIS>(sm, r, keep, 0, nodes, max_steps, tris);
+    const bool ok = !(packet_trace<AXIS>(sm, r, keep, 0, nodes, max_steps, tris) >> (threadIdx.x & 31) & 1u);
     const int hits = keep ? sm.n[threadIdx.x & 31] : 0;
     if (!valid) return;
     if (keep && (!ok || hits > kPacketHits)) leave_ray(ovf_list, ovf_count, left, (uint32_t)i);

@@ -785,12 +785,12 @@ struct RayPacket {
 };
 
 // Traces every lane's ray r (valid false: none; r.tmin 1e-6 for all) from node `start`: sm.n
-// has its number of crossings, sm.t and sm.tri the first kPacketHits found.  False when the
-// packet ran out of stack or steps.
+// has its number of crossings, sm.t and sm.tri the first kPacketHits found.  Returns the
+// lanes whose rays are not finished, the packet having run out of stack or of `max_steps`.
 template <int AXIS>
-__device__ __forceinline__ bool packet_trace(RayPacket& sm, const Ray& mine, bool valid, int start,
-                                             const BNode* __restrict__ nodes, uint32_t max_steps,
-                                             const float4* __restrict__ tris) {
+__device__ __forceinline__ unsigned int packet_trace(RayPacket& sm, const Ray& mine, bool valid, int start,
+                                                     const BNode* __restrict__ nodes, uint32_t max_steps,
+                                                     const float4* __restrict__ tris) {
     constexpr unsigned int kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned int below = (1u << lane) - 1u;
@@ -812,7 +812,6 @@ __device__ __forceinline__ bool packet_trace(RayPacket& sm, const Ray& mine, boo
     int sp = __popc(traced);
     uint32_t head = 0, queued = 0, steps = 0;
     unsigned int tests = 0;
-    bool ok = true;
     auto ray_of = [&](int e, bool direction) {
         const float4 o = sm.o[e];
         if (AXIS >= 0)
@@ -857,11 +856,8 @@ __device__ __forceinline__ bool packet_trace(RayPacket& sm, const Ray& mine, boo
         }
         // No more nodes than the stack has room to replace twice over.
         const int take = min(min(sp, 32), max(kPacketStack - sp, 1));
+        if (++steps > max_steps) break;
         sp -= take;
-        if (++steps > max_steps) {  // a step visits a node, and no ray visits one twice
-            ok = false;
-            break;
-        }
         bool h0 = false, h1 = false;
         int e = 0;
         int4 nd = make_int4(0, 0, 0, 0);
@@ -892,8 +888,8 @@ __device__ __forceinline__ bool packet_trace(RayPacket& sm, const Ray& mine, boo
         const bool p0 = h0 && nd.y <= 0, p1 = h1 && nd.w <= 0;
         const unsigned int mp0 = __ballot_sync(kAll, p0), mp1 = __ballot_sync(kAll, p1);
         const int pushed = __popc(mp0) + __popc(mp1);
-        if (sp + pushed > kPacketStack) {
-            ok = false;
+        if (sp + pushed > kPacketStack) {  // the popped nodes lie there still
+            sp += take;
             break;
         }
         if (p0) {
@@ -911,7 +907,10 @@ __device__ __forceinline__ bool packet_trace(RayPacket& sm, const Ray& mine, boo
     }
     __syncwarp();
     add_tests(tests);
-    return ok;
+    unsigned int unfinished = 0;
+    for (int i = lane; i < sp; i += 32) unfinished |= 1u << sm.own[i];
+    for (uint32_t i = lane; i < queued; i += 32) unfinished |= 1u << (sm.leaf[(head + i) & (kPacketRing - 1)].y & 31u);
+    return __reduce_or_sync(kAll, unfinished);
 }
 
 // The advance rule on the crossings that packet_trace left for this lane (at most
@@ -932,8 +931,8 @@ __device__ __forceinline__ Chain packet_chain(const RayPacket& sm, const float4*
 }
 
 // The edge of every lane (valid false: none), traversed from node `start`.  True for a lane
-// whose edge has to be traced by the long path: more than kPacketHits crossings, or the
-// packet ran out of stack or steps; nothing is inserted for it.
+// whose edge has to be traced by the long path: more than kPacketHits crossings, or not
+// finished when the packet ran out of stack or steps; nothing is inserted for it.
 __device__ __forceinline__ bool edge_packet(RayPacket& sm, const EdgePayload& p, bool valid, uint64_t i, int start,
                                             const BNode* __restrict__ nodes, uint32_t max_steps,
                                             const float4* __restrict__ tris, int swap, const PairTable& table) {
@@ -942,10 +941,10 @@ __device__ __forceinline__ bool edge_packet(RayPacket& sm, const EdgePayload& p,
     if (valid)
         valid = segment_ray_of(p.starts[3 * i], p.starts[3 * i + 1], p.starts[3 * i + 2], p.ends[3 * i],
                                p.ends[3 * i + 1], p.ends[3 * i + 2], r);
-    const bool ok = packet_trace<-1>(sm, r, valid, start, nodes, max_steps, tris);
+    const unsigned int unfinished = packet_trace<-1>(sm, r, valid, start, nodes, max_steps, tris);
     if (!valid) return false;
     const int n = sm.n[lane];
-    if (!ok || n > kPacketHits) return true;
+    if ((unfinished >> lane & 1u) || n > kPacketHits) return true;
     // The crossings in (t, id) order, each the least above the one before.
     EdgeWalk w;
     int32_t last = INT_MIN;

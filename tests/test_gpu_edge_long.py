@@ -1,6 +1,7 @@
 """Edges with long crossing lists and wide traversals: lists of a few and of many edges with
-as many crossings as a packet keeps and one more, and, on the warp-per-edge path, 255 to 700 crossings of one edge, hundreds of crossings at one
-distance, and edges of large objects through a dense cluster.  Pair sets equal the CPU
+as many crossings as a packet keeps and one more, and, on the warp-per-edge path, 255 to 1400
+crossings of one edge (512 is what a warp keeps), hundreds of crossings at one distance, and edges
+of large objects through a dense cluster, whose packets run out of steps.  Pair sets equal the CPU
 oracle's."""
 import numpy as np
 import pytest
@@ -53,15 +54,18 @@ def _rods(k):
 
 CASES = {"8 crossings": lambda: (_rods(1), _slabs(4)), "9 crossings": lambda: (_rods(1), _half(5)),
          "594 edges": lambda: (_rods(33), _half(5)), "3600 edges": lambda: (_rods(200), _slabs(4)), "256": lambda: (_rod(4.0), _slabs(128)), "255": lambda: (_rod(4.0), _half(128)),
-         "258": lambda: (_rod(4.0), _slabs(129)), "700": lambda: (_rod(8.0), _slabs(350)),
-         "equal": lambda: (_rod(4.0), _coincident(300)), "cluster": lambda: (_large(60), _cluster(6000))}
+         "258": lambda: (_rod(4.0), _slabs(129)), "511": lambda: (_rod(6.0), _half(256)),
+         "512": lambda: (_rod(6.0), _slabs(256)), "514": lambda: (_rod(6.0), _slabs(257)),
+         "700": lambda: (_rod(8.0), _slabs(350)), "1400": lambda: (_rod(15.0), _slabs(700)),
+         "equal": lambda: (_rod(4.0), _coincident(300)), "equal, more": lambda: (_rod(4.0), _coincident(600)),
+         "large cluster": lambda: (_large(400), _cluster(40000)), "cluster": lambda: (_large(60), _cluster(6000))}
 
 
 @pytest.mark.parametrize("rule", [(100, False), (100000, False), (256, True)])
 @pytest.mark.parametrize("name", sorted(CASES))
 def test_long_edges(cuda, name, rule):
     A, B = CASES[name]()
-    ps = api.PairSet(1 << 16)
+    ps = api.PairSet(1 << 20)
     ps.set_edge_rule(*rule)
     bb = api.Bvh(api.DeviceGeometry(B))
     api.edge_join(bb, api.DeviceGeometry(A), ps)
