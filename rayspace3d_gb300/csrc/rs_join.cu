@@ -101,21 +101,23 @@ struct WarpEdgeSmem {
 // and push the inner children hit; crossings go to a shared-memory list.  Visits the nodes
 // the one-thread traversal visits (the same slab tests over the same [tmin, tmax]), so it
 // finds the same crossings; the lanes rank them by (t, id) (triangle ids are distinct, so
-// ranks are too) and lane 0 walks them with the table's hit rule.
+// ranks are too), lane 0 walks them with the table's hit rule, and the pairs of the hits taken
+// are inserted by all lanes (one lane's inserts, a few hundred dependent atomics an edge,
+// took a tenth of a clustered join's k_edge_long_warp).
 //
 // A step pops no more nodes than the stack has room to replace twice over, so a wide
 // traversal turns into a depth-first one instead of running out of stack: an edge of a
 // large object in a dense cluster overlaps thousands of boxes, and the one-thread loop that
-// used to take such an edge kept a whole join waiting (17 ms of 57).  With RANGES, an edge
-// of more than HITS crossings is walked in ranges of t: the list's middle crossing ends the
-// range and the traversal restarts on it, until a range's crossings fit; the next range
-// begins above it.  Returns false when there are more than HITS crossings (RANGES: at one
-// and the same t) or the step budget or the stack runs out; pairs of ranges walked before
+// used to take such an edge kept a whole join waiting (17 ms of 57).  An edge of more than
+// HITS crossings is walked in ranges of t: the list's middle crossing ends the range and the
+// traversal restarts on it, until a range's crossings fit; the next range begins above it.
+// Returns false when there are more than HITS crossings at one and the same t or the step
+// budget or the stack runs out; pairs of ranges walked before
 // that are in the table, where the one-thread loop's start from the beginning finds them.
-template <int STACK, int HITS, bool RANGES>
+template <int STACK, int HITS>
 __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload& p, uint64_t i,
                               const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris,
-                              int swap, const PairTable& table, int start = 0) {
+                              int swap, const PairTable& table) {
     int* stack = w_sm.stack;
     float* ht = w_sm.t;
     uint32_t* hid = w_sm.id;
@@ -132,7 +134,7 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
     int32_t last = INT_MIN;
     unsigned int tests = 0;
     for (;;) {
-        if (lane == 0) stack[0] = start;
+        if (lane == 0) stack[0] = 0;
         __syncwarp();
         int sp = 1, nh = 0;
         uint32_t visits = 0;
@@ -175,7 +177,7 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
                 if (k < n0 + n1) {
                     float a[3], b[3], c[3];
                     load_tri(tris, k < n0 ? first[0] + k : first[1] + (k - n0), a, b, c, tid, obj);
-                    hit = hit_triangle<-1>(r, a, b, c, t) && (!RANGES || t > above);
+                    hit = hit_triangle<-1>(r, a, b, c, t) && t > above;
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, hit);
                 if (hit) {
@@ -204,7 +206,6 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
         }
         __syncwarp();
         if (!ok) return false;
-        if (!RANGES && nh > HITS) return false;
         const int kept = min(nh, HITS);
         for (int a = lane; a < kept; a += 32) {
             const float t = ht[a];
@@ -216,7 +217,7 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
             w_sm.obj2[rank] = hobj[a];
         }
         __syncwarp();
-        if (RANGES && nh > HITS) {
+        if (nh > HITS) {
             const float mid = w_sm.t2[HITS / 2];
             if (!(mid < r.tmax)) return false;
             r.tmax = mid;
@@ -235,7 +236,7 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
         for (int a = lane; a < found; a += 32)
             insert_sources(table, p.sources + p.offsets[i], p.counts[i], hobj[a], swap);
         __syncwarp();
-        if (!RANGES || r.tmax == tmax || __shfl_sync(0xffffffffu, (int)w.done, 0)) break;
+        if (r.tmax == tmax || __shfl_sync(0xffffffffu, (int)w.done, 0)) break;
         above = r.tmax;
         r.tmin = fmaxf(r.tmin, above);
         r.tmax = tmax;
@@ -269,13 +270,12 @@ __global__ void __launch_bounds__(32 * kLongWarps) k_edge_long_warp(EdgePayload 
     const unsigned int nw = gridDim.x * kLongWarps;
     for (unsigned int j = blockIdx.x * kLongWarps + wi; j < n; j += nw) {  // warp-uniform
         const uint32_t e = deferred[j];
-        if (!edge_ray_warp<kLongWarpStack, kLongWarpHits, true>(sm[wi], p, e, nodes, max_steps, tris, swap, table) &&
+        if (!edge_ray_warp<kLongWarpStack, kLongWarpHits>(sm[wi], p, e, nodes, max_steps, tris, swap, table) &&
             (threadIdx.x & 31) == 0)
             edge_ray_long(p, e, nodes, max_steps, tris, swap, table);
         __syncwarp();
     }
 }
-
 
 // Legacy per-triangle overlap (mesh_overlap.cu:126-179): record r = 3 t + e is edge e of
 // source triangle t.  Triangles with an index >= nV set *bad and are skipped.  Records the
@@ -925,8 +925,8 @@ __global__ void __launch_bounds__(kT) k_cull_flag(CullJob j0, CullJob j1, unsign
             break;
         }
         const BNode bn = load_node(nodes, node);
-            const float4 na = bn.a, nb = bn.b, nc = bn.c;
-            const int4 nd = bn.d;
+        const float4 na = bn.a, nb = bn.b, nc = bn.c;
+        const int4 nd = bn.d;
         bool h0 = cull_overlap(na.x, na.y, na.z, na.w, nb.x, nb.y, qlo, qhi);
         bool h1 = cull_overlap(nb.z, nb.w, nc.x, nc.y, nc.z, nc.w, qlo, qhi);
 #pragma unroll 1
