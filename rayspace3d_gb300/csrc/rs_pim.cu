@@ -502,18 +502,24 @@ struct CallWords {
 std::mutex g_words_mu;
 std::vector<CallWords> g_words[64];
 
-cudaError_t words_acquire(int device, CallWords* out) {
+cudaError_t words_acquire(int device, CallWords* out, cudaStream_t s) {
     if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
     std::lock_guard<std::mutex> g(g_words_mu);
     std::vector<CallWords>& pool = g_words[device];
     if (pool.empty()) {  // as many as are ever in flight together, kept until the process ends
         constexpr int kBlock = 32;
         unsigned long long *d = nullptr, *h = nullptr;
+        // Relaxed, and no work on the legacy stream: another thread may be capturing a stream.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
         cudaError_t e = cudaMalloc((void**)&d, kBlock * 256);
-        if (e == cudaSuccess) e = cudaMemset(d, 0, kBlock * 256);
         if (e == cudaSuccess) e = cudaMallocHost((void**)&h, kBlock * 256);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e == cudaSuccess) e = cudaMemsetAsync(d, 0, kBlock * 256, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             if (d) cudaFree(d);
+            if (h) cudaFreeHost(h);
             return e;
         }
         for (int k = 0; k < kBlock; ++k) pool.push_back(CallWords{d + 32 * k, h + 32 * k});
@@ -556,7 +562,7 @@ int pim_impl(const rs_bvh* cbvh, const float* pts, uint64_t n, float dx, float d
     CallWords words;
     uint32_t* ovf = nullptr;
     cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = words_acquire(device, &words);
+    if (e == cudaSuccess) e = words_acquire(device, &words, s);
     if (e != cudaSuccess) return to_status(e);
     e = dmalloc((void**)&ovf, n * sizeof(uint32_t), s);
     if (e != cudaSuccess) {
