@@ -45,8 +45,8 @@ constexpr int kLookAhead = 8;
 // Tiles whose counts are also summed, for the look-back: all tiles of a wave publish at about
 // the same time, and each then walked up to a wave of single counts (608 tiles, whose 256 words
 // are 1.2 MB; a few prefixes cut it short).  By groups it is 15 counts and 2 words for each group
-// before.  One pass: 1.6 M keys and values 33 -> 28 us, 3.2 M keys 32 -> 25, 6.4 M 80 -> 75;
-// groups of 32 take as long as those of 16.
+// before.  One pass, when it was made so: 1.6 M keys and values 33 -> 28 us, 3.2 M keys 32 -> 25,
+// 6.4 M 80 -> 75; groups of 32 take as long as those of 16.
 constexpr unsigned int kOsGroup = 16;
 
 __device__ __forceinline__ uint32_t os_digit(uint64_t k, int shift, int end_bit) {
@@ -129,13 +129,17 @@ __global__ void __launch_bounds__(kThreads, 4) k_os_pass(const uint64_t* __restr
     __shared__ unsigned int s_tile;
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     if (tid == 0) s_tile = atomicAdd(tile_ctr, 1u);
-    for (int i = tid; i < kWarps * 256; i += kThreads) (&s_cnt[0][0])[i] = 0;
+    for (int i = tid; i < kWarps * 256; i += kThreads) {
+        (&s_cnt[0][0])[i] = 0;
+        reinterpret_cast<uint32_t*>(s_keys)[i] = 0;
+    }
     __syncthreads();
     const unsigned int tile = s_tile;
     const size_t base = (size_t)tile * kOsTile + (size_t)w * kOsWarpSpan;
     uint64_t k[kOsItems];
     uint32_t v[kOsItems];
     unsigned peers[kOsItems];  // lanes of the warp holding the same digit in item r
+    static_assert(kWarps * 256 * sizeof(uint32_t) <= sizeof(s_keys), "a word per warp and digit");
 #pragma unroll
     for (int r = 0; r < kOsItems; ++r) {
         const size_t idx = base + (size_t)r * 32 + lane;
@@ -143,13 +147,24 @@ __global__ void __launch_bounds__(kThreads, 4) k_os_pass(const uint64_t* __restr
         k[r] = valid ? kin[idx] : 0ull;
         if (VALS) v[r] = valid ? vin[idx] : 0u;
     }
-    // Per-warp digit counts (an invalid key gets a digit of its own: 256 + lane).
+    // Per-warp digit counts.  The lanes that share a digit meet in a word of the warp's own, in
+    // the part of shared memory that the keys are staged in later.  __match_any_sync took longer
+    // the more digits a warp had: one pass of 3.2 M keys 25 us where neighbours share digits and
+    // 45 where they do not, 28 and 30 now; 6.4 M 76 -> 51, 1.6 M with values 28 -> 22.5.  Eight
+    // ballots a key: 40 us for either.
+    uint32_t* meet = reinterpret_cast<uint32_t*>(s_keys) + w * 256;
 #pragma unroll
     for (int r = 0; r < kOsItems; ++r) {
         const bool valid = base + (size_t)r * 32 + lane < n;
-        const uint32_t dg = valid ? os_digit(k[r], shift, end_bit) : (256u + lane);
-        peers[r] = __match_any_sync(0xffffffffu, dg);
-        if (valid && lane == __ffs(peers[r]) - 1) s_cnt[w][dg] += __popc(peers[r]);
+        const uint32_t dg = os_digit(k[r], shift, end_bit);
+        if (valid) atomicOr(&meet[dg], 1u << lane);
+        __syncwarp();
+        peers[r] = valid ? meet[dg] : 0u;
+        __syncwarp();
+        if (valid && lane == __ffs(peers[r]) - 1) {
+            s_cnt[w][dg] += __popc(peers[r]);
+            meet[dg] = 0;
+        }
         __syncwarp();
     }
     __syncthreads();
