@@ -394,7 +394,7 @@ def run_engine(args, rank, world, local):
         per_launch = sum(live_check_bytes(g) for g in (da, db)) + 8.0 * n_pairs
         achieved = per_launch / (p["avg_ms"] * 1e-3) / 1e9
         roof_edges = {"bound": "hbm",
-                      "kernel": "k_edge_live + k_edge_rays_warp / k_edge_rays + k_edge_long_warp (both directions)",
+                      "kernel": "k_edge_live + k_edge_rays + k_edge_long_warp (both directions)",
                       "achieved": round(achieved, 2), "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 5),
                       "algorithmic_bytes_per_launch": int(per_launch), "avg_launch_ms": round(p["avg_ms"], 4),
                       "traffic": profiled_traffic("edge_rays_w1000", args.objects)}
