@@ -193,6 +193,7 @@ __global__ void k_obox_init(int* __restrict__ box, uint64_t cap, const int* __re
 // Morton key of each triangle's box centre (and, into obox, the box of each object below
 // obox_cap: triangles of one object are usually stored together, so the lanes of a warp
 // with equal objects reduce first and one of them does the atomics).
+// Triangles with an id below zero are in no object's box: bit 2 of *bad_index says there are some.
 // Grid-stride over the triangles; also counts the four 8-bit digits of each Morton code
 // (the sort's histogram, hist[p * 256 + digit p]) in shared memory, added to `hist` once
 // per block, so the sort does not read the keys back for them.
@@ -212,6 +213,11 @@ __global__ void __launch_bounds__(kT) k_morton(const float* __restrict__ V, uint
         if (obox) {
             const int32_t o = T[t];
             int v[6] = {flt_ord(lo[0]), flt_ord(lo[1]), flt_ord(lo[2]), flt_ord(hi[0]), flt_ord(hi[1]), flt_ord(hi[2])};
+            // A range without a number (lo is then the empty box's already) widens no box: as a
+            // maximum it would make the object's box one that overlaps nothing.
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[3 + k] = isnan(hi[k]) ? (int)0x80000000 : v[3 + k];
+            if (o < 0) atomicOr(bad_index, 4u);
             const unsigned int peers = __match_any_sync(__activemask(), o);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
@@ -651,8 +657,10 @@ int bvh_ready(const rs_bvh* ch) {
         h->vmax[k] = dec(hb[9 + k]);
     }
     h->n_obj = hb[13] >= 0 ? (uint64_t)hb[13] + 1 : 0;
-    // [12]: bit 0 an index out of range, bit 1 a failed sort (bounded wait ran out).
-    h->build_status = (hb[12] & 2) ? RS_ERR_ITER_LIMIT : hb[12] != 0 ? RS_ERR_INVALID : RS_OK;
+    // [12]: bit 0 an index out of range, bit 1 a failed sort (bounded wait ran out), bit 2 an
+    // object id below zero.
+    h->unboxed = (hb[12] & 4) != 0;
+    h->build_status = (hb[12] & 2) ? RS_ERR_ITER_LIMIT : (hb[12] & 1) ? RS_ERR_INVALID : RS_OK;
     return h->build_status;
 }
 
@@ -720,7 +728,7 @@ static int build_impl(const float* d_vertices, uint64_t nV, const uint32_t* d_in
     const size_t b_open = a256(((size_t)nG / 2 + kTB) * sizeof(OpenTree));
     const size_t b_sort = radix_sort_scratch_bytes((size_t)n, 64, 32, false);
     char* scratch = nullptr;
-    int* bounds = nullptr;  // [6..11] vertex bounds (ordered ints), [12] bad-index flag, [13] max object
+    int* bounds = nullptr;  // [6..11] vertex bounds (ordered ints), [12] flags, [13] max object
     unsigned int* n_open = nullptr;
     int* xchg = nullptr;
     uint64_t* keys = nullptr;

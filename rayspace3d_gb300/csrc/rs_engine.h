@@ -42,12 +42,13 @@ struct rs_bvh {
     // pass, for the objects below obox_cap; valid when n_obj <= obox_cap.
     int* obox = nullptr;
     uint64_t obox_cap = 0;
+    bool unboxed = false;  // some triangles have an id below zero: no object's box holds them
     // One device allocation holds nodes, tris and obox.
     void* mem = nullptr;
     int device = 0;
     // Completion of the build, and its device result words until bvh_ready() has read
     // them (asynchronous builds); the fields above that come from them (vmin, vmax,
-    // n_obj) are valid only after bvh_ready().
+    // n_obj, unboxed) are valid only after bvh_ready().
     cudaEvent_t done = nullptr;
     int* pending = nullptr;
     int build_status = RS_OK;

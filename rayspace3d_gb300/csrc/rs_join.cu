@@ -331,6 +331,8 @@ __device__ __forceinline__ int f2ord(float f) {
     const int i = __float_as_int(f);
     return i >= 0 ? i : i ^ 0x7fffffff;
 }
+// Of a range's maximum: one without a number is the empty box's (its minimum, 0x7fffffff, is).
+__device__ __forceinline__ int f2ord_max(float f) { return isnan(f) ? (int)0x80000000 : f2ord(f); }
 __device__ __forceinline__ float ord2f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
 // The box of edge i's segment widened like a broad-phase query box: kCullAbs plus the
@@ -844,8 +846,8 @@ __global__ void k_obj_boxes(const float4* __restrict__ tris, uint64_t n, int* __
     const float4 p = __ldg(&tris[3 * k]), q = __ldg(&tris[3 * k + 1]), r = __ldg(&tris[3 * k + 2]);
     const int32_t obj = __float_as_int(q.w);
     int v[6] = {f2ord(fminf(fminf(p.x, q.x), r.x)), f2ord(fminf(fminf(p.y, q.y), r.y)),
-                f2ord(fminf(fminf(p.z, q.z), r.z)), f2ord(fmaxf(fmaxf(p.x, q.x), r.x)),
-                f2ord(fmaxf(fmaxf(p.y, q.y), r.y)), f2ord(fmaxf(fmaxf(p.z, q.z), r.z))};
+                f2ord(fminf(fminf(p.z, q.z), r.z)), f2ord_max(fmaxf(fmaxf(p.x, q.x), r.x)),
+                f2ord_max(fmaxf(fmaxf(p.y, q.y), r.y)), f2ord_max(fmaxf(fmaxf(p.z, q.z), r.z))};
     const unsigned int peers = __match_any_sync(__activemask(), obj);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -1005,7 +1007,8 @@ struct CullPacket {
 
 // For every object of one set, the number of the other set's objects whose widened boxes
 // overlap its own, and the first kPartners of them as its partner list: every partner is among
-// them, since a triangle's box lies in its object's.  One warp per object.
+// them, since a triangle's box lies in its object's -- in a set without triangles of an id below
+// zero, which are a partner of no box: such a set has no lists.  One warp per object.
 __global__ void __launch_bounds__(256) k_box_pairs(CullJob j0, CullJob j1, unsigned int blocks0) {
     const bool second = blockIdx.x >= blocks0;
     const CullJob j = second ? j1 : j0;
@@ -1770,12 +1773,13 @@ cudaError_t cull_impl(const rs_bvh* A, const rs_bvh* B, uint8_t* candA, uint8_t*
         // take (10k + 10k of 320: 176 us).
         const bool long_walks = boxes[0] && boxes[1] && A->n_obj * B->n_obj <= (1ull << 26) &&
                                 A->n_tris + B->n_tris >= 1024 * (A->n_obj + B->n_obj);
-        if (long_walks) e = dmalloc((void**)&most, n_query * sizeof(uint32_t), s);
-        if (long_walks && e == cudaSuccess) {
+        const bool listed[2] = {long_walks && job[0].part && !B->unboxed, long_walks && job[1].part && !A->unboxed};
+        if (listed[0] || listed[1]) e = dmalloc((void**)&most, n_query * sizeof(uint32_t), s);
+        if (most && e == cudaSuccess) {
             uint32_t* next = most;
             unsigned bb[2] = {0, 0};
             for (int d = 0; d < 2; ++d) {
-                if (!job[d].part) continue;
+                if (!listed[d]) continue;
                 job[d].obox = boxes[1 - d];
                 job[d].n_other = other[d]->n_obj;
                 job[d].most = next;
