@@ -435,8 +435,7 @@ extern "C" int rs_batch_submit(rs_batch* b, void* stream) {
         const int u = bvh_use(effective(b, it.bvh), s);
         if (u != RS_OK) return u;
         if (it.ps) {  // a replayed graph inserts without table_view()
-            it.ps->known_count = -1;
-            it.ps->pristine = false;
+            table_given(it.ps);
             if (ps_use(it.ps, s) != cudaSuccess) return RS_ERR_CUDA;
         }
     }

@@ -100,6 +100,9 @@ int table_status(rs_pairset* ps, cudaStream_t s, cudaError_t e);
 cudaError_t table_regrow(rs_pairset* ps, uint64_t count, uint64_t over, cudaStream_t s);
 // Orders work queued on stream s after the table's creation.
 cudaError_t ps_use(const rs_pairset* ps, cudaStream_t s);
+// To be called before every launch that may insert: what the host knows of the table no longer
+// holds (table_view calls it; a replayed graph has its view already).
+void table_given(rs_pairset* ps);
 // Queues the clearing of a table for a join, unless it is pristine.
 cudaError_t table_clear(rs_pairset* ps, cudaStream_t s);
 // Queues the clearing of the overflow table (and its count) when a launch may have used it.

@@ -1467,9 +1467,14 @@ __global__ void __launch_bounds__(32 * kContWarps) k_containment(const float* __
 
 int recheck_join(int op, unsigned long long* out) { return recheck_op(op, out); }
 
-PairTable table_view(rs_pairset* ps) {
-    ps->known_count = -1;  // a launch is about to insert
+void table_given(rs_pairset* ps) {
+    ps->known_count = -1;
     ps->pristine = false;
+    if (ps->over) ps->over_dirty = true;
+}
+
+PairTable table_view(rs_pairset* ps) {
+    table_given(ps);
     PairTable t;
     t.slots = ps->slots;
     t.capacity = ps->capacity;
@@ -1484,7 +1489,6 @@ PairTable table_view(rs_pairset* ps) {
     t.over_mask = kOverSlots - 1;
     t.over_count = ps->meta + kOverWord;
     t.spill_at = std::max<unsigned long long>(1, ps->capacity / 4 * 3 + (ps->capacity % 4) * 3 / 4);
-    if (ps->over) ps->over_dirty = true;
     return t;
 }
 
