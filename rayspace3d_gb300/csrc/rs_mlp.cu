@@ -17,16 +17,14 @@
 // rs_mlp_set_gemm(1) sends every product to mma.sync (the tests compare the two paths).
 // Weights keep an FP32 master copy (Adam) and a BF16 copy that the GEMMs read.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstring>
-#include <mutex>
-#include <thread>
 #include <vector>
 
 #include <cuda_bf16.h>
 
 #include "rs_engine.h"
+#include "rs_host_stage.h"
 #include "rs_prims.cuh"
 
 namespace rs {
@@ -544,85 +542,6 @@ __global__ void k_pool(const uint4* __restrict__ cells, int R, float* __restrict
 }  // namespace rs
 
 using namespace rs;
-
-namespace rs {
-// Device to pageable host copies of large arrays: threads that each copy every kThreads-th
-// chunk into pinned memory, two chunks in flight, and from there to the caller's array.  The
-// runtime's own pageable copy moves 23 GB/s on one thread, which also takes the page faults
-// of a fresh array; the copy engine moves 211 GB/s.  Belongs to one handle; the first large
-// copy makes it.
-class HostStage {
-  public:
-    ~HostStage() { release(); }
-    cudaError_t copy(void* dst, const void* src, size_t bytes, int device) {
-        std::lock_guard<std::mutex> g(mu_);
-        cudaPointerAttributes at{};
-        const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
-        cudaGetLastError();
-        if (!pageable || bytes < 4 * kChunk || !ready()) return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
-        cudaError_t e = cudaStreamSynchronize(nullptr);  // a copy waits for the legacy stream's work
-        if (e != cudaSuccess) return e;
-        std::atomic<int> failed{(int)cudaSuccess};
-        auto work = [&](int t) {
-            cudaError_t w = cudaSetDevice(device);
-            const size_t chunks = (bytes + kChunk - 1) / kChunk;
-            auto size_of = [&](size_t c) { return std::min(kChunk, bytes - c * kChunk); };
-            auto fetch = [&](size_t c, int k) {
-                if (w == cudaSuccess)
-                    w = cudaMemcpyAsync(buf_ + (2 * t + k) * kChunk, static_cast<const char*>(src) + c * kChunk, size_of(c),
-                                        cudaMemcpyDeviceToHost, stream_[t]);
-                if (w == cudaSuccess) w = cudaEventRecord(event_[2 * t + k], stream_[t]);
-            };
-            size_t c = t;
-            if (c < chunks) fetch(c, 0);
-            for (int k = 0; c < chunks && w == cudaSuccess; c += kThreads, k ^= 1) {
-                if (c + kThreads < chunks) fetch(c + kThreads, k ^ 1);
-                if (w == cudaSuccess) w = cudaEventSynchronize(event_[2 * t + k]);
-                if (w == cudaSuccess)
-                    std::memcpy(static_cast<char*>(dst) + c * kChunk, buf_ + (2 * t + k) * kChunk, size_of(c));
-            }
-            cudaStreamSynchronize(stream_[t]);  // nothing in flight into the buffers after a failure
-            if (w != cudaSuccess) failed = (int)w;
-        };
-        std::thread threads[kThreads];
-        int started = 0;
-        try {
-            for (; started < kThreads - 1; ++started) threads[started] = std::thread(work, started);
-        } catch (...) {  // no more threads: their shares are done here
-        }
-        for (int t = started; t < kThreads; ++t) work(t);
-        for (int t = 0; t < started; ++t) threads[t].join();
-        return (cudaError_t)failed.load();
-    }
-
-  private:
-    static constexpr int kThreads = 8;
-    static constexpr size_t kChunk = size_t(1) << 20;
-    bool ready() {
-        if (buf_) return true;
-        bool ok = cudaMallocHost((void**)&buf_, 2 * kThreads * kChunk) == cudaSuccess;
-        for (int t = 0; t < kThreads && ok; ++t)
-            ok = cudaStreamCreateWithFlags(&stream_[t], cudaStreamNonBlocking) == cudaSuccess;
-        for (int k = 0; k < 2 * kThreads && ok; ++k)
-            ok = cudaEventCreateWithFlags(&event_[k], cudaEventDisableTiming) == cudaSuccess;
-        if (!ok) release();
-        return ok;
-    }
-    void release() {
-        for (cudaEvent_t& e : event_)
-            if (e) cudaEventDestroy(e), e = nullptr;
-        for (cudaStream_t& s : stream_)
-            if (s) cudaStreamDestroy(s), s = nullptr;
-        if (buf_) cudaFreeHost(buf_);
-        buf_ = nullptr;
-        cudaGetLastError();
-    }
-    std::mutex mu_;
-    char* buf_ = nullptr;
-    cudaStream_t stream_[kThreads] = {};
-    cudaEvent_t event_[2 * kThreads] = {};
-};
-}  // namespace rs
 
 struct rs_mlp {
     // Parameters, gradients and Adam moments, each one contiguous FP32 array:
