@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from rayspace3d_gb300 import api, synth
+from rayspace3d_gb300 import api, gen, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -88,3 +88,13 @@ def test_a_long_run_is_not_quadratic(cuda):
     rng = np.random.default_rng(1)
     loose = rng.uniform(0, 100, (6000, 3)), np.arange(6000).reshape(-1, 3), np.arange(2000)
     assert _seconds(_book(2000, 0)) < 20 * _seconds(loose)  # 80 times and more, looking back through the run
+
+
+def test_one_long_list_does_not_start_over(cuda):
+    """A vertex of more triangles than a block's list holds, beside 3.2 M others."""
+    many = gen.instanced_set(10000, 2, 0.5, 2.0, 1000.0, seed=3)
+
+    def beside(n):
+        V, I, T = _device(*_fan(n, 1))
+        return torch.cat([many.V, V]), torch.cat([many.I, I + many.nV]), torch.cat([many.T, T + 10000])
+    assert _seconds(beside(6000)) < 3 * _seconds(beside(2000))  # 5.5 times, starting over by wide words
