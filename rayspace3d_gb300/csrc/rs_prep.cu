@@ -291,22 +291,48 @@ __global__ void __launch_bounds__(kPT) k_vertex_rank(uint64_t nV, const uint32_t
 
 // Counts (FILL false) or lists (FILL true) the records of every lower rank; the fill counts
 // the lists' lengths down to zero.  Triangles with an index >= nV are skipped, as the
-// reference skips them (EdgePreprocessor.cpp:64-66).
+// reference skips them (EdgePreprocessor.cpp:64-66).  Eight lanes and more of one rank share
+// one atomic: where a mesh has collapsed, all of them queue on a few words.
 template <bool FILL>
 __global__ void __launch_bounds__(kPT) k_rank_lists(const uint32_t* __restrict__ I, uint64_t nF, uint64_t nV,
                                                     const uint32_t* __restrict__ rank, uint32_t* __restrict__ count,
                                                     const uint32_t* __restrict__ start,
                                                     uint64_t* __restrict__ items) {
+    constexpr unsigned int kAll = 0xffffffffu;
     const uint64_t t = blockIdx.x * (uint64_t)kPT + threadIdx.x;
-    if (t >= nF) return;
-    const uint32_t v[3] = {I[3 * t], I[3 * t + 1], I[3 * t + 2]};
-    if (v[0] >= nV || v[1] >= nV || v[2] >= nV) return;
-    const uint32_t r[3] = {__ldg(&rank[v[0]]), __ldg(&rank[v[1]]), __ldg(&rank[v[2]])};
+    const int lane = threadIdx.x & 31;
+    uint32_t r[3] = {0, 0, 0};
+    bool valid = t < nF;
+    if (valid) {
+        const uint32_t v[3] = {I[3 * t], I[3 * t + 1], I[3 * t + 2]};
+        valid = v[0] < nV && v[1] < nV && v[2] < nV;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (valid) r[k] = __ldg(&rank[v[k]]);
+    }
+    const unsigned int counted = __ballot_sync(kAll, valid);
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
         const uint32_t a = r[e], b = r[e == 2 ? 0 : e + 1], lo = min(a, b), hi = max(a, b);
-        if (FILL) items[start[lo] + atomicSub(&count[lo], 1u) - 1u] = (uint64_t)hi << 32 | (uint32_t)(3 * t + e);
-        else atomicAdd(&count[lo], 1u);
+        uint32_t slot = 0;
+        unsigned int todo = counted;
+        while (todo) {  // the same in every lane
+            const int leader = __ffs(todo) - 1;
+            const uint32_t one = __shfl_sync(kAll, lo, leader);
+            const unsigned int group = __ballot_sync(kAll, lo == one) & todo;
+            const uint32_t n = __popc(group);
+            if (n < 8) break;
+            uint32_t base = 0;
+            if (lane == leader) base = FILL ? atomicSub(&count[one], n) : atomicAdd(&count[one], n);
+            base = __shfl_sync(kAll, base, leader);
+            if (group >> lane & 1u) slot = base - 1u - __popc(group & ((1u << lane) - 1u));
+            todo &= ~group;
+        }
+        if (todo >> lane & 1u) {
+            if (FILL) slot = atomicSub(&count[lo], 1u) - 1u;
+            else atomicAdd(&count[lo], 1u);
+        }
+        if (FILL && valid) items[start[lo] + slot] = (uint64_t)hi << 32 | (uint32_t)(3 * t + e);
     }
 }
 

@@ -98,3 +98,9 @@ def test_one_long_list_does_not_start_over(cuda):
         V, I, T = _device(*_fan(n, 1))
         return torch.cat([many.V, V]), torch.cat([many.I, I + many.nV]), torch.cat([many.T, T + 10000])
     assert _seconds(beside(6000)) < 3 * _seconds(beside(2000))  # 5.5 times, starting over by wide words
+
+
+def test_records_of_one_rank_do_not_queue(cuda):
+    """A mesh collapsed to a point, against one of as many triangles that is not."""
+    V, I, T = _copies(1500, 1, 3)
+    assert _seconds((V * 1e-9, I, T)) < 3 * _seconds((V, I, T))  # 5 times, with an atomic each
