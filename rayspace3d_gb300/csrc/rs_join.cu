@@ -783,8 +783,9 @@ bool ray_side_stream(cudaStream_t* st_out, cudaEvent_t* fork, cudaEvent_t* joine
     return true;
 }
 
-__global__ void k_first_tri_init(int32_t* __restrict__ first, uint64_t nObj) {
+__global__ void k_first_tri_init(int32_t* __restrict__ first, uint64_t nObj, unsigned int* __restrict__ n_def) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (i == 0) *n_def = 0;
     if (i < nObj) first[i] = INT_MAX;
 }
 
@@ -1221,6 +1222,10 @@ struct Tracking {
     uint32_t* candidates;     // [nObj]
 };
 
+__device__ __forceinline__ Ray containment_ray(float x, float y, float z) {
+    return make_ray(x, y, z, 0.0f, 0.0f, 1.0f, 1e-4f, 1e10f);
+}
+
 // The ray of source object o; false when it has none.
 __device__ __forceinline__ bool containment_ray(const float* __restrict__ V, uint64_t nV,
                                                 const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
@@ -1229,7 +1234,7 @@ __device__ __forceinline__ bool containment_ray(const float* __restrict__ V, uin
     if (ft == INT_MAX) return false;
     const uint32_t vi = I[3 * (uint64_t)ft];
     if (vi >= nV) return false;
-    r = make_ray(V[3 * (uint64_t)vi], V[3 * (uint64_t)vi + 1], V[3 * (uint64_t)vi + 2], 0.0f, 0.0f, 1.0f, 1e-4f, 1e10f);
+    r = containment_ray(V[3 * (uint64_t)vi], V[3 * (uint64_t)vi + 1], V[3 * (uint64_t)vi + 2]);
     return true;
 }
 
@@ -1350,18 +1355,206 @@ __global__ void __launch_bounds__(kT) k_containment_tracked(const float* __restr
 // One warp per object: up to 32 nodes a step from a shared-memory stack, as the edge rays of
 // short lists, and the object ids of all crossings in a list; a target is inserted when it
 // occurs an odd number of times.  One thread per object made the join wait on its longest
-// chain of dependent node loads, with one warp for 32 objects.  A ray of more crossings, or
-// a wider traversal, runs the one-thread passes in lane 0.
+// chain of dependent node loads, with one warp for 32 objects.
+//
+// A list that fills up keeps each object's parity, and when that leaves it half full or more,
+// the lower half of its ids: the traversal goes on for them alone, and the next pass takes the
+// ids above.  Left to the one-thread passes, with 31 lanes idle, 20,000 objects under 300 boxes
+// (600 crossings) took 39.7 ms where a thread for each object had taken 4.2; now 1.15.  A step
+// pops no more nodes than leave kStackRoom entries: a wide traversal turns into a depth-first
+// one, and only a tree deeper than that runs out of stack and goes to the one-thread passes.
 constexpr int kContWarps = 4;    // objects per block
-constexpr int kContStack = 256;  // entries of a warp's stack
+constexpr int kContStack = 320;  // entries of a warp's stack
 constexpr int kContHits = 512;   // crossings a warp keeps
+constexpr int kStackRoom = 64;   // a level of the tree each, descended one node at a time
+constexpr uint64_t kContDefer = 8192;  // objects from which the rays left over get a launch of their own
 
-__global__ void __launch_bounds__(32 * kContWarps) k_containment(const float* __restrict__ V, uint64_t nV,
-                                                                 const uint32_t* __restrict__ I,
-                                                                 const int32_t* __restrict__ first, uint64_t nObj,
-                                                                 const BNode* __restrict__ nodes, uint32_t max_steps,
-                                                                 const float4* __restrict__ tris, int swap,
-                                                                 PairTable table) {
+// Sorts the warp's list of nh ids and leaves one of an object that occurs an odd number of
+// times, and none (even: two) of the others; then, from half of kContHits on, the ids up to the
+// middle one, which becomes *up.  Returns the number left.
+__device__ __noinline__ int fold_ids(uint32_t* ids, int nh, bool even, uint32_t* up) {
+    constexpr unsigned int kAll = 0xffffffffu;
+    constexpr int kPer = kContHits / 32;
+    const int lane = threadIdx.x & 31;
+    for (int i = nh + lane; i < kContHits; i += 32) ids[i] = 0xffffffffu;
+    __syncwarp();
+    for (int k = 2; k <= kContHits; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = lane; i < kContHits; i += 32) {
+                const int q = i ^ j;
+                if (q > i && (ids[i] > ids[q]) == ((i & k) == 0)) {
+                    const uint32_t t = ids[i];
+                    ids[i] = ids[q];
+                    ids[q] = t;
+                }
+            }
+            __syncwarp();
+        }
+    uint32_t v[kPer];
+    unsigned int keep = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int i = 32 * q + lane;
+        v[q] = ids[i];
+        if (i >= nh) continue;
+        int lo = 0, hi = i;  // the first place of this id
+        while (lo < hi) {
+            const int mid = (lo + hi) / 2;
+            if (ids[mid] < v[q]) lo = mid + 1;
+            else hi = mid;
+        }
+        const bool last = i + 1 == nh || ids[i + 1] != v[q];
+        const bool before_last = !last && (i + 2 == nh || ids[i + 2] != v[q]);
+        const int count = i + (last ? 1 : 2) - lo;
+        if ((last && (count & 1 || even)) || (before_last && !(count & 1) && even)) keep |= 1u << q;
+    }
+    __syncwarp();
+    int n = 0;
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const unsigned int m = __ballot_sync(kAll, keep >> q & 1u);
+        if (keep >> q & 1u) ids[n + __popc(m & ((1u << lane) - 1u))] = v[q];
+        n += __popc(m);
+    }
+    __syncwarp();
+    if (n < kContHits / 2) return n;
+    *up = ids[n / 2 - 1];
+    n = n / 2 < n && ids[n / 2] == *up ? n / 2 + 1 : n / 2;
+    __syncwarp();
+    return n;
+}
+
+// The object's crossings in passes of ids by the whole warp, for rays of more of them than one
+// list holds, or of more nodes than its stack does.
+__device__ __forceinline__ void containment_many(const Ray& r, uint64_t o, int* stack, uint32_t* ids,
+                                                 const BNode* __restrict__ nodes, uint32_t max_steps,
+                                                 const float4* __restrict__ tris, int swap, const PairTable& table) {
+    constexpr unsigned int kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned int below = (1u << lane) - 1u;
+    unsigned int tests = 0, crossings = 0, targets = 0;
+    bool ok = true, bounded = false;
+    uint32_t above = 0, up = 0xffffffffu;  // this pass: ids > above (bounded), <= up
+    for (;;) {
+        if (lane == 0) stack[0] = 0;
+        __syncwarp();
+        int sp = 1, nh = 0;
+        uint32_t visits = 0;
+        while (sp > 0) {
+            const int take = min(min(sp, 32), max(kContStack - kStackRoom - sp, 1));
+            const int node = lane < take ? stack[sp - take + lane] : -1;
+            __syncwarp();
+            sp -= take;
+            visits += (uint32_t)take;
+            bool h[2] = {false, false};
+            int leaf[2] = {0, 0}, cnt[2] = {0, 0};
+            if (node >= 0) {
+                const BNode bn = load_node(nodes, node);
+                const float4 na = bn.a, nb = bn.b, nc = bn.c;
+                const int4 nd = bn.d;
+                const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
+                const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
+                float en, ex;
+                h[0] = slab<2>(r, lo0, hi0, r.tmin, r.tmax, en, ex);
+                h[1] = slab<2>(r, lo1, hi1, r.tmin, r.tmax, en, ex);
+                leaf[0] = nd.x;
+                cnt[0] = nd.y;
+                leaf[1] = nd.z;
+                cnt[1] = nd.w;
+            }
+            const bool p0 = h[0] && cnt[0] == 0, p1 = h[1] && cnt[1] == 0;
+            const unsigned b0 = __ballot_sync(kAll, p0), b1 = __ballot_sync(kAll, p1);
+            const int pushed = __popc(b0) + __popc(b1);
+            if (visits > max_steps || sp + pushed > kContStack) {
+                ok = false;
+                break;
+            }
+            int pos = sp + __popc(b0 & below) + __popc(b1 & below);
+            if (p0) stack[pos++] = leaf[0];
+            if (p1) stack[pos] = leaf[1];
+            sp += pushed;
+            // Triangles of the leaves hit: the first child's, then the second's.
+            const int n0 = h[0] ? cnt[0] : 0, n1 = h[1] ? cnt[1] : 0;
+            tests += (unsigned int)(n0 + n1);
+            const int rounds = __reduce_max_sync(kAll, n0 + n1);
+            for (int k = 0; k < rounds; ++k) {
+                bool hit = false;
+                uint32_t tid;
+                int32_t obj = 0;
+                if (k < n0 + n1) {
+                    float a[3], b[3], c[3], t;
+                    load_tri(tris, k < n0 ? leaf[0] + k : leaf[1] + (k - n0), a, b, c, tid, obj);
+                    hit = hit_triangle<2>(r, a, b, c, t);
+                }
+                unsigned m = __ballot_sync(kAll, hit);
+                if (!bounded) crossings += __popc(m);
+                if (bounded || up != 0xffffffffu) {  // this pass leaves ids out
+                    hit = hit && (uint32_t)obj <= up && !(bounded && (uint32_t)obj <= above);
+                    m = __ballot_sync(kAll, hit);
+                }
+                if (nh + __popc(m) > kContHits) {  // the same in every lane
+                    nh = fold_ids(ids, nh, table.stats != nullptr, &up);
+                    hit = hit && (uint32_t)obj <= up;
+                    m = __ballot_sync(kAll, hit);
+                }
+                if (hit) ids[nh + __popc(m & below)] = (uint32_t)obj;
+                nh += __popc(m);
+            }
+            __syncwarp();
+        }
+        __syncwarp();
+        if (!ok) break;
+        unsigned int distinct = 0;
+        for (int a = lane; a < nh; a += 32) {
+            const uint32_t id = ids[a];
+            int before = 0, all = 0;
+            for (int b = 0; b < nh; ++b) {
+                const bool same = ids[b] == id;
+                all += same;
+                before += same && b < a;
+            }
+            if (before) continue;  // its first occurrence decides
+            ++distinct;
+            if (all & 1) table_insert(table, containment_key(o, id, swap));
+        }
+        targets += distinct;
+        __syncwarp();
+        if (up == 0xffffffffu) break;
+        above = up;
+        up = 0xffffffffu;
+        bounded = true;
+    }
+    if (!ok) {  // finds the pairs of the passes before again
+        if (lane == 0) containment_thread<false>(r, o, nodes, max_steps, tris, swap, table, Tracking{});
+        return;
+    }
+    add_tests(tests);
+    if (table.stats) {
+        targets = __reduce_add_sync(kAll, targets);
+        if (lane == 0) {
+            atomicAdd(&table.stats[4], 1ull);
+            if (crossings) atomicAdd(&table.stats[5], (unsigned long long)crossings);
+            if (targets) atomicAdd(&table.stats[6], (unsigned long long)targets);
+        }
+    }
+}
+
+// The same from within k_containment, which keeps its registers: not inlined, all by value.
+__device__ __noinline__ void containment_many_call(float ox, float oy, float oz, uint64_t o, int* stack, uint32_t* ids,
+                                                   const BNode* __restrict__ nodes, uint32_t max_steps,
+                                                   const float4* __restrict__ tris, int swap, const PairTable table) {
+    containment_many(containment_ray(ox, oy, oz), o, stack, ids, nodes, max_steps, tris, swap, table);
+}
+
+// DEFER: such objects go to deferred[0..*n_def), for k_containment_many.  Without the call the
+// kernel has 64 registers instead of 72 and spills none, which is 5 to 15 % from some thousand
+// objects on (a target of 100,000 spheres: 10,000 objects 944 -> 875 us, 200,000 10.0 -> 8.6 ms);
+// the second launch costs 4 us, 1 % of a join of 150 objects.
+template <bool DEFER>
+__device__ __forceinline__ void containment_objects(
+    const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
+    uint64_t nObj, const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris, int swap,
+    const PairTable& table, uint32_t* __restrict__ deferred, unsigned int* __restrict__ n_def) {
     constexpr unsigned int kAll = 0xffffffffu;
     __shared__ int s_stack[kContWarps][kContStack];
     __shared__ uint32_t s_id[kContWarps][kContHits];
@@ -1379,7 +1572,7 @@ __global__ void __launch_bounds__(32 * kContWarps) k_containment(const float* __
         bool ok = true;
         unsigned int tests = 0;
         while (sp > 0) {
-            const int take = min(sp, 32);
+            const int take = min(min(sp, 32), max(kContStack - kStackRoom - sp, 1));
             const int node = lane < take ? stack[sp - take + lane] : -1;
             __syncwarp();
             sp -= take;
@@ -1430,10 +1623,12 @@ __global__ void __launch_bounds__(32 * kContWarps) k_containment(const float* __
                 nh += __popc(m);
             }
             __syncwarp();
+            if (nh > kContHits) break;
         }
         __syncwarp();
         if (!ok || nh > kContHits) {
-            if (lane == 0) containment_thread<false>(r, o, nodes, max_steps, tris, swap, table, Tracking{});
+            if (!DEFER) containment_many_call(r.o[0], r.o[1], r.o[2], o, stack, ids, nodes, max_steps, tris, swap, table);
+            else if (lane == 0) deferred[atomicAdd(n_def, 1u)] = (uint32_t)o;
             __syncwarp();
             continue;
         }
@@ -1459,6 +1654,38 @@ __global__ void __launch_bounds__(32 * kContWarps) k_containment(const float* __
                 if (distinct) atomicAdd(&table.stats[6], (unsigned long long)distinct);
             }
         }
+        __syncwarp();
+    }
+}
+
+__global__ void __launch_bounds__(32 * kContWarps, 7) k_containment(
+    const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
+    uint64_t nObj, const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris, int swap,
+    PairTable table) {
+    containment_objects<false>(V, nV, I, first, nObj, nodes, max_steps, tris, swap, table, nullptr, nullptr);
+}
+
+__global__ void __launch_bounds__(32 * kContWarps, 8) k_containment_first(
+    const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
+    uint64_t nObj, const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris, int swap,
+    PairTable table,
+    uint32_t* __restrict__ deferred, unsigned int* __restrict__ n_def) {
+    containment_objects<true>(V, nV, I, first, nObj, nodes, max_steps, tris, swap, table, deferred, n_def);
+}
+
+__global__ void __launch_bounds__(32 * kContWarps) k_containment_many(
+    const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
+    const uint32_t* __restrict__ deferred, const unsigned int* __restrict__ n_def, const BNode* __restrict__ nodes,
+    uint32_t max_steps, const float4* __restrict__ tris, int swap, PairTable table) {
+    __shared__ int s_stack[kContWarps][kContStack];
+    __shared__ uint32_t s_id[kContWarps][kContHits];
+    const int wi = threadIdx.x >> 5;
+    const unsigned int n = *n_def;
+    for (unsigned int d = blockIdx.x * kContWarps + wi; d < n; d += gridDim.x * kContWarps) {
+        Ray r;
+        if (containment_ray(V, nV, I, first, deferred[d], r))
+            containment_many(r, deferred[d], s_stack[wi], s_id[wi], nodes, max_steps, tris, swap,
+                             table);
         __syncwarp();
     }
 }
@@ -1950,19 +2177,32 @@ static cudaError_t containment_async(const rs_bvh* target, const float* V, uint6
                               const int32_t* t2o, uint64_t nObj, int swap, rs_pairset* ps, const Tracking* trk,
                               cudaStream_t s) {
     if (nObj == 0 || nF == 0 || target->n_tris == 0) return cudaSuccess;
-    int32_t* first = nullptr;
-    cudaError_t e = dmalloc((void**)&first, nObj * sizeof(int32_t), s);
+    int32_t* first = nullptr;  // first triangles, deferred objects, their number
+    cudaError_t e = dmalloc((void**)&first, (2 * nObj + 1) * sizeof(int32_t), s);
     if (e != cudaSuccess) return e;
-    launch(k_first_tri_init, (unsigned)((nObj + 255) / 256), 256, 0, s, first, nObj);
+    uint32_t* deferred = reinterpret_cast<uint32_t*>(first + nObj);
+    unsigned int* n_def = deferred + nObj;
+    launch(k_first_tri_init, (unsigned)((nObj + 255) / 256), 256, 0, s, first, nObj, n_def);
     launch(k_first_tri, (unsigned)((nF + 256 * kFirstPer - 1) / (256 * kFirstPer)), 256, 0, s, t2o, nF, first, nObj);
     const int ptok = prof_begin(P_CONTAINMENT, s);
-    if (trk)
+    if (trk) {
         launch(k_containment_tracked, (unsigned)((nObj + kT - 1) / kT), kT, 0, s, V, nV, I, (const int32_t*)first, nObj,
                (const BNode*)target->nodes, max_steps(target), (const float4*)target->tris, swap, table_view(ps), *trk);
-    else
-        launch(k_containment, (unsigned)std::min<uint64_t>((nObj + kContWarps - 1) / kContWarps, 16ull * sm_count()),
-               32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first, nObj, (const BNode*)target->nodes,
-               max_steps(target), (const float4*)target->tris, swap, table_view(ps));
+    } else {
+        const PairTable table = table_view(ps);
+        const unsigned grid = (unsigned)std::min<uint64_t>((nObj + kContWarps - 1) / kContWarps, 16ull * sm_count());
+        const BNode* nodes = target->nodes;
+        const float4* tris = target->tris;
+        if (nObj <= kContDefer) {
+            launch(k_containment, grid, 32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first, nObj, nodes,
+                   max_steps(target), tris, swap, table);
+        } else {
+            launch(k_containment_first, grid, 32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first, nObj, nodes,
+                   max_steps(target), tris, swap, table, deferred, n_def);
+            launch(k_containment_many, grid, 32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first,
+                   (const uint32_t*)deferred, (const unsigned int*)n_def, nodes, max_steps(target), tris, swap, table);
+        }
+    }
     prof_end(P_CONTAINMENT, s, ptok);
     e = cudaGetLastError();
     cudaFreeAsync(first, s);

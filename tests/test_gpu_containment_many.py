@@ -1,0 +1,90 @@
+"""Containment rays that cross more triangles than a warp's list holds (512): objects crossed once,
+twice and hundreds of times each, more objects than the list has room for, ids below zero, and
+boxes that all lie on the ray, which no stack holds at once.  Pairs equal the CPU oracle's, the
+counters what the geometry says, and the time stays near that of rays the list holds."""
+import ctypes
+import time
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import bind
+from rayspace3d_gb300 import _lib, api, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _nested(k):
+    """k concentric cubes: a ray from the centre crosses each once, and each contains it."""
+    return [(np.full(3, -1.0 - 0.01 * j), np.full(3, 1.0 + 0.01 * j)) for j in range(k)]
+
+
+def _stacked(k):
+    """k boxes above the origin, crossed twice each."""
+    return [(np.array([-1.0, -1.0, 50.0 + j]), np.array([1.0, 1.0, 50.5 + j])) for j in range(k)]
+
+
+def _sources(n):
+    c = np.random.default_rng(3).uniform(-0.4, 0.4, (n, 3))
+    return synth.box_set([(p - 0.05, p + 0.05) for p in c], edges=False)
+
+
+def _target(boxes, objects=None):
+    """The boxes' objects in a mixed order, or the given ids."""
+    g = synth.box_set(boxes, edges=False)
+    ids = np.random.default_rng(len(boxes)).permutation(len(boxes)) if objects is None else np.asarray(objects)
+    return synth.make_geometry(g.vertices, g.indices, ids[g.tri2obj], edges=False)
+
+
+CASES = {"540 nested": (lambda: _target(_nested(540)), 540, 540),
+         "3000 nested": (lambda: _target(_nested(3000)), 3000, 3000),
+         "257 stacked": (lambda: _target(_stacked(257)), 514, 257),
+         "1500 stacked in 20": (lambda: _target(_nested(20) + _stacked(1500)), 3020, 1520),
+         "one of 700 boxes among 600": (lambda: _target(_nested(600) + _stacked(700), [*range(600)] + [77] * 700), 2000, 600),
+         "two of 401 each": (lambda: _target(_nested(802), [5, 9] * 401), 802, 2)}
+
+
+@pytest.mark.parametrize("name", sorted(CASES))
+@pytest.mark.parametrize("n", [1, 50])
+def test_pairs_and_counters(cuda, name, n):
+    make, crossings, candidates = CASES[name]
+    A, B = _sources(n), make()
+    b, src = api.Bvh(api.DeviceGeometry(B)), api.DeviceGeometry(A)
+    want = np.sort(bind.containment(A, B.vertices, B.indices, B.tri2obj))
+    L = _lib.load()
+    for track in (0, 1):
+        ps = api.PairSet(1 << 18)
+        L.rs_pairset_set_tracking(ps.handle, track)
+        api.containment(b, src, ps)
+        np.testing.assert_array_equal(ps.finalize().cpu().numpy().astype(np.uint64), want)
+        if track:
+            c = (ctypes.c_uint64 * 8)()
+            assert L.rs_pairset_counters(ps.handle, c, None) == 0
+            assert list(c)[4:7] == [n, n * crossings, n * candidates]
+
+
+def test_an_id_below_zero(cuda):
+    A, B = _sources(3), _target(_nested(600), [-1, 4] * 300)
+    B = synth.make_geometry(B.vertices, B.indices, np.where(np.arange(len(B.indices)) < 12, 4, B.tri2obj), edges=False)
+    ps = api.PairSet(1 << 10)  # 4 is crossed 301 times, -1 299 times
+    api.containment(api.Bvh(api.DeviceGeometry(B)), api.DeviceGeometry(A), ps)
+    got = {tuple(p) for p in api.keys_to_pairs(ps.finalize()).tolist()}
+    assert got == {(o, t) for o in range(3) for t in (4, -1)}
+
+
+def test_a_list_that_overflows_costs_no_fallback(cuda):
+    src = api.DeviceGeometry(_sources(20000))
+
+    def seconds(k):
+        b = api.Bvh(api.DeviceGeometry(_target(_stacked(k))))
+        best = np.inf
+        ps = api.PairSet(1 << 10)
+        for _ in range(3):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            api.containment(b, src, ps)
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t)
+        return best
+    assert seconds(300) < 10 * seconds(200)  # 36 times, by the one-thread passes
