@@ -783,9 +783,9 @@ bool ray_side_stream(cudaStream_t* st_out, cudaEvent_t* fork, cudaEvent_t* joine
     return true;
 }
 
-__global__ void k_first_tri_init(int32_t* __restrict__ first, uint64_t nObj, unsigned int* __restrict__ n_def) {
+__global__ void k_first_tri_init(int32_t* __restrict__ first, uint64_t nObj, unsigned int* __restrict__ n_left) {
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i == 0) *n_def = 0;
+    if (i == 0) *n_left = 0;
     if (i < nObj) first[i] = INT_MAX;
 }
 
@@ -1222,10 +1222,6 @@ struct Tracking {
     uint32_t* candidates;     // [nObj]
 };
 
-__device__ __forceinline__ Ray containment_ray(float x, float y, float z) {
-    return make_ray(x, y, z, 0.0f, 0.0f, 1.0f, 1e-4f, 1e10f);
-}
-
 // The ray of source object o; false when it has none.
 __device__ __forceinline__ bool containment_ray(const float* __restrict__ V, uint64_t nV,
                                                 const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
@@ -1234,7 +1230,7 @@ __device__ __forceinline__ bool containment_ray(const float* __restrict__ V, uin
     if (ft == INT_MAX) return false;
     const uint32_t vi = I[3 * (uint64_t)ft];
     if (vi >= nV) return false;
-    r = containment_ray(V[3 * (uint64_t)vi], V[3 * (uint64_t)vi + 1], V[3 * (uint64_t)vi + 2]);
+    r = make_ray(V[3 * (uint64_t)vi], V[3 * (uint64_t)vi + 1], V[3 * (uint64_t)vi + 2], 0.0f, 0.0f, 1.0f, 1e-4f, 1e10f);
     return true;
 }
 
@@ -1367,7 +1363,11 @@ constexpr int kContWarps = 4;    // objects per block
 constexpr int kContStack = 320;  // entries of a warp's stack
 constexpr int kContHits = 512;   // crossings a warp keeps
 constexpr int kStackRoom = 64;   // a level of the tree each, descended one node at a time
-constexpr uint64_t kContDefer = 8192;  // objects from which the rays left over get a launch of their own
+// Objects from which rays are traced in packets first.  80,000 objects with a target of 3 large
+// spheres, 20,000 and 100,000 dense ones: 298, 632 and 4,500 us with packets, 500, 735 and 3,970
+// without (a thread an object: 410, 980, 54,000); 200,000 objects: 395, 1,190 and 9,590 against 895,
+// 1,445 and 8,590.  At 40,000 packets save 100 us at most and cost 950 where every ray is long.
+constexpr uint64_t kContPackets = 65536;
 
 // Sorts the warp's list of nh ids and leaves one of an object that occurs an odd number of
 // times, and none (even: two) of the others; then, from half of kContHits on, the ids up to the
@@ -1539,22 +1539,15 @@ __device__ __forceinline__ void containment_many(const Ray& r, uint64_t o, int* 
     }
 }
 
-// The same from within k_containment, which keeps its registers: not inlined, all by value.
-__device__ __noinline__ void containment_many_call(float ox, float oy, float oz, uint64_t o, int* stack, uint32_t* ids,
-                                                   const BNode* __restrict__ nodes, uint32_t max_steps,
-                                                   const float4* __restrict__ tris, int swap, const PairTable table) {
-    containment_many(containment_ray(ox, oy, oz), o, stack, ids, nodes, max_steps, tris, swap, table);
-}
-
-// DEFER: such objects go to deferred[0..*n_def), for k_containment_many.  Without the call the
-// kernel has 64 registers instead of 72 and spills none, which is 5 to 15 % from some thousand
-// objects on (a target of 100,000 spheres: 10,000 objects 944 -> 875 us, 200,000 10.0 -> 8.6 ms);
-// the second launch costs 4 us, 1 % of a join of 150 objects.
-template <bool DEFER>
-__device__ __forceinline__ void containment_objects(
+// Objects 0..nObj-1, or list[0..*n_list).  Those left over follow when the warp is through with
+// the others: called from the loop they cost the others up to 12 % (1,000 objects under 200 boxes
+// 190 -> 218 us), in a launch of their own 2 % of a join of 150 objects.  deferred (nObj words):
+// every warp has the places of the objects that it takes.  64 registers, some spilled, and 8
+// blocks an SM beat 72 and 7: 200,000 objects in 100,000 spheres 9.6 ms against 11.0.
+__global__ void __launch_bounds__(32 * kContWarps, 8) k_containment(
     const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
     uint64_t nObj, const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris, int swap,
-    const PairTable& table, uint32_t* __restrict__ deferred, unsigned int* __restrict__ n_def) {
+    PairTable table, const uint32_t* __restrict__ list, const unsigned int* __restrict__ n_list, uint32_t* deferred) {
     constexpr unsigned int kAll = 0xffffffffu;
     __shared__ int s_stack[kContWarps][kContStack];
     __shared__ uint32_t s_id[kContWarps][kContHits];
@@ -1562,7 +1555,11 @@ __device__ __forceinline__ void containment_objects(
     const unsigned int below = (1u << lane) - 1u;
     int* stack = s_stack[wi];
     uint32_t* ids = s_id[wi];
-    for (uint64_t o = blockIdx.x * (uint64_t)kContWarps + wi; o < nObj; o += (uint64_t)gridDim.x * kContWarps) {
+    const uint64_t k0 = blockIdx.x * (uint64_t)kContWarps + wi, warps = (uint64_t)gridDim.x * kContWarps;
+    const uint64_t n = list ? (uint64_t)*n_list : nObj;
+    uint64_t left = k0;
+    for (uint64_t k = k0; k < n; k += warps) {
+        const uint64_t o = list ? list[k] : k;
         Ray r;
         if (!containment_ray(V, nV, I, first, o, r)) continue;  // the same in every lane
         if (lane == 0) stack[0] = 0;
@@ -1627,8 +1624,8 @@ __device__ __forceinline__ void containment_objects(
         }
         __syncwarp();
         if (!ok || nh > kContHits) {
-            if (!DEFER) containment_many_call(r.o[0], r.o[1], r.o[2], o, stack, ids, nodes, max_steps, tris, swap, table);
-            else if (lane == 0) deferred[atomicAdd(n_def, 1u)] = (uint32_t)o;
+            if (lane == 0) deferred[left] = (uint32_t)o;
+            left += warps;
             __syncwarp();
             continue;
         }
@@ -1656,36 +1653,55 @@ __device__ __forceinline__ void containment_objects(
         }
         __syncwarp();
     }
-}
-
-__global__ void __launch_bounds__(32 * kContWarps, 7) k_containment(
-    const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
-    uint64_t nObj, const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris, int swap,
-    PairTable table) {
-    containment_objects<false>(V, nV, I, first, nObj, nodes, max_steps, tris, swap, table, nullptr, nullptr);
-}
-
-__global__ void __launch_bounds__(32 * kContWarps, 8) k_containment_first(
-    const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
-    uint64_t nObj, const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris, int swap,
-    PairTable table,
-    uint32_t* __restrict__ deferred, unsigned int* __restrict__ n_def) {
-    containment_objects<true>(V, nV, I, first, nObj, nodes, max_steps, tris, swap, table, deferred, n_def);
-}
-
-__global__ void __launch_bounds__(32 * kContWarps) k_containment_many(
-    const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
-    const uint32_t* __restrict__ deferred, const unsigned int* __restrict__ n_def, const BNode* __restrict__ nodes,
-    uint32_t max_steps, const float4* __restrict__ tris, int swap, PairTable table) {
-    __shared__ int s_stack[kContWarps][kContStack];
-    __shared__ uint32_t s_id[kContWarps][kContHits];
-    const int wi = threadIdx.x >> 5;
-    const unsigned int n = *n_def;
-    for (unsigned int d = blockIdx.x * kContWarps + wi; d < n; d += gridDim.x * kContWarps) {
+    for (uint64_t k = k0; k < left; k += warps) {
+        const uint64_t o = deferred[k];
         Ray r;
-        if (containment_ray(V, nV, I, first, deferred[d], r))
-            containment_many(r, deferred[d], s_stack[wi], s_id[wi], nodes, max_steps, tris, swap,
-                             table);
+        if (containment_ray(V, nV, I, first, o, r)) containment_many(r, o, stack, ids, nodes, max_steps, tris, swap, table);
+        __syncwarp();
+    }
+}
+
+// Many objects, `size` a packet (RayPacket); those of more than kPacketHits crossings, or of an
+// unfinished packet, go to deferred[0..*n_def), for k_containment.  With objects enough to fill
+// the GPU it is the lanes that count: most rays of a sparse set visit a few dozen nodes and cross
+// little, and a warp for each has one lane in ten busy.
+__global__ void __launch_bounds__(32 * kContWarps, 6) k_containment_packets(
+    const float* __restrict__ V, uint64_t nV, const uint32_t* __restrict__ I, const int32_t* __restrict__ first,
+    uint64_t nObj, uint32_t size, const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris,
+    int swap, PairTable table, uint32_t* __restrict__ deferred, unsigned int* __restrict__ n_def) {
+    __shared__ RayPacket packets[kContWarps];
+    RayPacket& sm = packets[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    for (uint64_t k = blockIdx.x * (uint64_t)kContWarps + (threadIdx.x >> 5); k * size < nObj;
+         k += (uint64_t)gridDim.x * kContWarps) {
+        const uint64_t o = k * size + lane;
+        Ray r;
+        const bool valid = (uint32_t)lane < size && o < nObj && containment_ray(V, nV, I, first, o, r);
+        const unsigned int unfinished =
+            packet_trace<2>(sm, r, valid, 0, nodes, min(max_steps, kPacketSteps), tris, 1e-4f);
+        const int n = valid ? sm.n[lane] : 0;
+        if (valid && (unfinished >> lane & 1u || n > kPacketHits)) {
+            deferred[atomicAdd(n_def, 1u)] = (uint32_t)o;
+        } else if (valid) {
+            unsigned int targets = 0;
+            for (int a = 0; a < n; ++a) {
+                const uint32_t id = __float_as_uint(__ldg(&tris[3 * (size_t)sm.tri[a][lane] + 1].w));
+                int before = 0, all = 0;
+                for (int b = 0; b < n; ++b) {
+                    const bool same = __float_as_uint(__ldg(&tris[3 * (size_t)sm.tri[b][lane] + 1].w)) == id;
+                    all += same;
+                    before += same && b < a;
+                }
+                if (before) continue;  // its first occurrence decides
+                ++targets;
+                if (all & 1) table_insert(table, containment_key(o, id, swap));
+            }
+            if (table.stats) {
+                atomicAdd(&table.stats[4], 1ull);
+                if (n) atomicAdd(&table.stats[5], (unsigned long long)n);
+                if (targets) atomicAdd(&table.stats[6], (unsigned long long)targets);
+            }
+        }
         __syncwarp();
     }
 }
@@ -2177,12 +2193,12 @@ static cudaError_t containment_async(const rs_bvh* target, const float* V, uint6
                               const int32_t* t2o, uint64_t nObj, int swap, rs_pairset* ps, const Tracking* trk,
                               cudaStream_t s) {
     if (nObj == 0 || nF == 0 || target->n_tris == 0) return cudaSuccess;
-    int32_t* first = nullptr;  // first triangles, deferred objects, their number
-    cudaError_t e = dmalloc((void**)&first, (2 * nObj + 1) * sizeof(int32_t), s);
+    int32_t* first = nullptr;  // first triangles, deferred objects, those the packets left, their number
+    cudaError_t e = dmalloc((void**)&first, (3 * nObj + 1) * sizeof(int32_t), s);
     if (e != cudaSuccess) return e;
-    uint32_t* deferred = reinterpret_cast<uint32_t*>(first + nObj);
-    unsigned int* n_def = deferred + nObj;
-    launch(k_first_tri_init, (unsigned)((nObj + 255) / 256), 256, 0, s, first, nObj, n_def);
+    uint32_t *deferred = reinterpret_cast<uint32_t*>(first + nObj), *left = deferred + nObj;
+    unsigned int* n_left = left + nObj;
+    launch(k_first_tri_init, (unsigned)((nObj + 255) / 256), 256, 0, s, first, nObj, n_left);
     launch(k_first_tri, (unsigned)((nF + 256 * kFirstPer - 1) / (256 * kFirstPer)), 256, 0, s, t2o, nF, first, nObj);
     const int ptok = prof_begin(P_CONTAINMENT, s);
     if (trk) {
@@ -2193,15 +2209,16 @@ static cudaError_t containment_async(const rs_bvh* target, const float* V, uint6
         const unsigned grid = (unsigned)std::min<uint64_t>((nObj + kContWarps - 1) / kContWarps, 16ull * sm_count());
         const BNode* nodes = target->nodes;
         const float4* tris = target->tris;
-        if (nObj <= kContDefer) {
-            launch(k_containment, grid, 32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first, nObj, nodes,
-                   max_steps(target), tris, swap, table);
-        } else {
-            launch(k_containment_first, grid, 32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first, nObj, nodes,
-                   max_steps(target), tris, swap, table, deferred, n_def);
-            launch(k_containment_many, grid, 32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first,
-                   (const uint32_t*)deferred, (const unsigned int*)n_def, nodes, max_steps(target), tris, swap, table);
+        const uint32_t* list = nullptr;  // all objects
+        if (nObj > kContPackets) {
+            const uint64_t warps = 6ull * kContWarps * sm_count();  // a resident wave
+            const uint32_t size = (uint32_t)std::min<uint64_t>((nObj + warps - 1) / warps, 32);
+            launch(k_containment_packets, 6u * sm_count(), 32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first, nObj,
+                   size, nodes, max_steps(target), tris, swap, table, left, n_left);
+            list = left;
         }
+        launch(k_containment, grid, 32 * kContWarps, 0, s, V, nV, I, (const int32_t*)first, nObj, nodes,
+               max_steps(target), tris, swap, table, list, (const unsigned int*)n_left, deferred);
     }
     prof_end(P_CONTAINMENT, s, ptok);
     e = cudaGetLastError();

@@ -784,13 +784,13 @@ struct RayPacket {
     unsigned char own[kPacketStack];
 };
 
-// Traces every lane's ray r (valid false: none; r.tmin 1e-6 for all) from node `start`: sm.n
+// Traces every lane's ray r (valid false: none; r.tmin is `tmin` for all) from node `start`: sm.n
 // has its number of crossings, sm.t and sm.tri the first kPacketHits found.  Returns the
 // lanes whose rays are not finished, the packet having run out of stack or of `max_steps`.
 template <int AXIS>
 __device__ __forceinline__ unsigned int packet_trace(RayPacket& sm, const Ray& mine, bool valid, int start,
                                                      const BNode* __restrict__ nodes, uint32_t max_steps,
-                                                     const float4* __restrict__ tris) {
+                                                     const float4* __restrict__ tris, float tmin = kEps) {
     constexpr unsigned int kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned int below = (1u << lane) - 1u;
@@ -816,12 +816,12 @@ __device__ __forceinline__ unsigned int packet_trace(RayPacket& sm, const Ray& m
         const float4 o = sm.o[e];
         if (AXIS >= 0)
             return make_ray(o.x, o.y, o.z, AXIS == 0 ? 1.0f : 0.0f, AXIS == 1 ? 1.0f : 0.0f, AXIS == 2 ? 1.0f : 0.0f,
-                            kEps, o.w);
+                            tmin, o.w);
         const float4 inv = sm.inv[e];
         Ray r;
         r.o[0] = o.x; r.o[1] = o.y; r.o[2] = o.z;
         r.inv[0] = inv.x; r.inv[1] = inv.y; r.inv[2] = inv.z;
-        r.tmin = kEps;
+        r.tmin = tmin;
         r.tmax = o.w;
         if (direction) {
             const float4 d = sm.d[e];

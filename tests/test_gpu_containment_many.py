@@ -88,3 +88,47 @@ def test_a_list_that_overflows_costs_no_fallback(cuda):
             best = min(best, time.perf_counter() - t)
         return best
     assert seconds(300) < 10 * seconds(200)  # 36 times, by the one-thread passes
+
+
+@pytest.mark.parametrize("n", [65536, 65537, 70003])
+def test_more_objects_than_warps(cuda, n):
+    """Around the number from which rays go in packets: columns of 3, 9 and 12 boxes, one of 520 nested,
+    one beside everything, an object in seven without a triangle."""
+    column = np.arange(n) % 5
+    c = np.random.default_rng(n).uniform(-0.4, 0.4, (n, 3)) + np.stack([100.0 * column, 0 * column, 0 * column], 1)
+    # one triangle an object: its first vertex is the ray's origin
+    V = (c[:, None] + np.array([[0, 0, 0], [0.01, 0, 0], [0, 0.01, 0.01]])).astype(np.float32).reshape(-1, 3)
+    keep = np.arange(n) % 7 != 3
+    keep[-1] = True
+    I = np.arange(3 * n).reshape(-1, 3)[keep]
+    A = synth.make_geometry(V, I, np.arange(n)[keep], edges=False)
+    at = lambda boxes, k: [(lo + [100.0 * k, 0, 0], hi + [100.0 * k, 0, 0]) for lo, hi in boxes]
+    B = _target(at(_nested(3), 0) + at(_nested(1) + _stacked(4), 1) + at(_nested(12), 2) + at(_nested(520), 3))
+    ps = api.PairSet(1 << 24)
+    L = _lib.load()
+    L.rs_pairset_set_tracking(ps.handle, 1)
+    api.containment(api.Bvh(api.DeviceGeometry(B)), api.DeviceGeometry(A), ps)
+    want = np.sort(bind.containment(A, B.vertices, B.indices, B.tri2obj))
+    np.testing.assert_array_equal(ps.finalize().cpu().numpy().astype(np.uint64), want)
+    per = np.bincount(column[keep], minlength=5)
+    c = (ctypes.c_uint64 * 8)()
+    assert L.rs_pairset_counters(ps.handle, c, None) == 0
+    assert list(c)[4:7] == [keep.sum(), int(per @ [3, 9, 12, 520, 0]), int(per @ [3, 5, 12, 520, 0])]
+
+
+def test_many_short_rays_fill_their_warps(cuda):
+    """200,000 objects below three: four times as many take far less than four times as long."""
+    from rayspace3d_gb300 import gen
+    target = api.Bvh(gen.instanced_set(3, 6, 40.0, 50.0, 100.0, seed=6))
+
+    def seconds(n):
+        src = gen.instanced_set(n, 0, 0.05, 0.2, 100.0, seed=5)
+        ps, best = api.PairSet(1 << 20), np.inf
+        for _ in range(5):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            api.containment(target, src, ps)
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t)
+        return best
+    assert seconds(800000) < 2.5 * seconds(200000)
