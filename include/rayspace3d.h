@@ -316,16 +316,17 @@ int rs_batch_add_edges(rs_batch* batch, const rs_bvh* target, const float* d_sta
                        const int32_t* d_offsets, const int32_t* d_counts, const int32_t* d_sources, uint64_t nE,
                        int swap, rs_pairset* ps, int* index);
 /* chunk: rays a warp takes per pull (multiple of 32, default 64); stack_depth: 32 or 64
- * traversal stack entries (default 64); use_graph: capture and replay (default 1). */
+ * (default 64), without effect: no traversal has a stack of the caller's depth any more;
+ * use_graph: capture and replay (default 1). */
 int rs_batch_set_options(rs_batch* batch, int chunk, int stack_depth, int use_graph);
 int rs_batch_submit(rs_batch* batch, void* stream);
 /* Waits for the last submit; per-query statuses into h_status (nullable); returns the
  * first failing one. */
 int rs_batch_wait(rs_batch* batch, int* h_status);
-/* Times the batch over BVH leaf sizes {2,4,8,16}, chunks {32,64,128} and stack depths
- * {32,64} (three runs each, configurations whose queries fail are skipped), keeps the
- * fastest (rebuilding the batch's BVHs with its leaf size when it differs from the
- * caller's) and reports it. */
+/* Times the batch over BVH leaf sizes {2,4,8,16} and chunks {32,64,128} (three runs each,
+ * configurations whose queries fail are skipped), keeps the fastest (rebuilding the
+ * batch's BVHs with its leaf size when it differs from the caller's) and reports it;
+ * *h_stack_depth is always 64. */
 int rs_batch_autotune(rs_batch* batch, int* h_leaf_size, int* h_chunk, int* h_stack_depth, double* h_ms,
                       void* stream);
 

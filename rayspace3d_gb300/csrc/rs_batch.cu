@@ -12,7 +12,7 @@
 // that cross more than 8 triangles (axis-aligned points: 256) go to one overflow list that a
 // second launch resolves exactly.  The launches of an unchanged
 // batch are captured once as a CUDA graph and replayed.  rs_batch_autotune times the
-// batch over BVH leaf sizes, chunk sizes and traversal stack depths and keeps the best.
+// batch over BVH leaf sizes and chunk sizes and keeps the best.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -151,7 +151,6 @@ __global__ void __launch_bounds__(kBT, 6) k_batch(const BatchQuery* __restrict__
     }
 }
 
-template <int STACK>
 __global__ void __launch_bounds__(kBT) k_batch_fallback(const BatchQuery* __restrict__ q,
                                                         const uint2* __restrict__ ovf,
                                                         const unsigned long long* __restrict__ ovf_count) {
@@ -167,10 +166,10 @@ __global__ void __launch_bounds__(kBT) k_batch_fallback(const BatchQuery* __rest
             continue;
         }
         const Ray r = make_ray(Q.pts[3 * i], Q.pts[3 * i + 1], Q.pts[3 * i + 2], Q.dx, Q.dy, Q.dz, kEps, kTmax);
-        if (Q.axis == 0) pim_fallback_ray<0, STACK>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
-        else if (Q.axis == 1) pim_fallback_ray<1, STACK>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
-        else if (Q.axis == 2) pim_fallback_ray<2, STACK>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
-        else pim_fallback_ray<-1, STACK>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
+        if (Q.axis == 0) pim_fallback_ray<0, kStack>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
+        else if (Q.axis == 1) pim_fallback_ray<1, kStack>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
+        else if (Q.axis == 2) pim_fallback_ray<2, kStack>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
+        else pim_fallback_ray<-1, kStack>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
     }
 }
 
@@ -205,7 +204,6 @@ struct rs_batch_item {
 struct rs_batch {
     std::vector<rs_batch_item> items;
     int chunk = 64;
-    int stack = 64;
     int use_graph = 1;
     // Device state of the committed batch.
     bool dirty = true;
@@ -339,12 +337,9 @@ cudaError_t enqueue(rs_batch* b, cudaStream_t s) {
     if (b->total_chunks) {
         launch(k_batch, b->grid, kBT, kBatchSmem, s, (const BatchQuery*)b->d_q, nq, b->total_chunks, b->chunk,
                b->d_counters, b->d_ovf, b->d_counters + 1);
-        if (b->d_ovf && b->stack == 32)
-            launch(k_batch_fallback<32>, fallback_grid(b), kBT, 0, s, (const BatchQuery*)b->d_q,
-                   (const uint2*)b->d_ovf, (const unsigned long long*)b->d_counters + 1);
-        else if (b->d_ovf)
-            launch(k_batch_fallback<64>, fallback_grid(b), kBT, 0, s, (const BatchQuery*)b->d_q,
-                   (const uint2*)b->d_ovf, (const unsigned long long*)b->d_counters + 1);
+        if (b->d_ovf)
+            launch(k_batch_fallback, fallback_grid(b), kBT, 0, s, (const BatchQuery*)b->d_q, (const uint2*)b->d_ovf,
+                   (const unsigned long long*)b->d_counters + 1);
     }
     return cudaGetLastError();
 }
@@ -413,9 +408,8 @@ extern "C" int rs_batch_set_options(rs_batch* b, int chunk, int stack_depth, int
     if (chunk == 0) chunk = 64;
     if (stack_depth == 0) stack_depth = 64;
     if (chunk < 32 || chunk > 4096 || (chunk & 31) || (stack_depth != 32 && stack_depth != 64)) return RS_ERR_INVALID;
-    if (chunk != b->chunk || stack_depth != b->stack) b->dirty = true;
+    if (chunk != b->chunk) b->dirty = true;
     b->chunk = chunk;
-    b->stack = stack_depth;
     b->use_graph = use_graph != 0;
     if (!b->use_graph && b->exec) {
         cudaGraphExecDestroy(b->exec);
@@ -495,10 +489,9 @@ extern "C" int rs_batch_autotune(rs_batch* b, int* h_leaf, int* h_chunk, int* h_
         if (std::find(orig.begin(), orig.end(), it.bvh) == orig.end()) orig.push_back(it.bvh);
     const int leaves[4] = {2, 4, 8, 16};
     const int chunks[3] = {32, 64, 128};
-    const int stacks[2] = {32, 64};
     const int graph = b->use_graph;
     double best = -1.0;
-    int best_leaf = 4, best_chunk = b->chunk, best_stack = b->stack;
+    int best_leaf = 4, best_chunk = b->chunk;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -519,25 +512,22 @@ extern "C" int rs_batch_autotune(rs_batch* b, int* h_leaf, int* h_chunk, int* h_
         if (result != RS_OK) break;
         b->dirty = true;
         for (int ch : chunks) {
-            for (int sd : stacks) {
-                rs_batch_set_options(b, ch, sd, 0);
-                double ms_sum = 0.0;
-                bool ok = true;
-                for (int rep = 0; rep < 3 && ok; ++rep) {
-                    cudaEventRecord(e0, s);
-                    ok = rs_batch_submit(b, s) == RS_OK;
-                    cudaEventRecord(e1, s);
-                    ok = ok && rs_batch_wait(b, nullptr) == RS_OK;
-                    float ms = 0.0f;
-                    cudaEventElapsedTime(&ms, e0, e1);
-                    if (rep > 0) ms_sum += ms;  // the first run warms up
-                }
-                if (ok && (best < 0.0 || ms_sum / 2.0 < best)) {
-                    best = ms_sum / 2.0;
-                    best_leaf = leaf;
-                    best_chunk = ch;
-                    best_stack = sd;
-                }
+            rs_batch_set_options(b, ch, 0, 0);
+            double ms_sum = 0.0;
+            bool ok = true;
+            for (int rep = 0; rep < 3 && ok; ++rep) {
+                cudaEventRecord(e0, s);
+                ok = rs_batch_submit(b, s) == RS_OK;
+                cudaEventRecord(e1, s);
+                ok = ok && rs_batch_wait(b, nullptr) == RS_OK;
+                float ms = 0.0f;
+                cudaEventElapsedTime(&ms, e0, e1);
+                if (rep > 0) ms_sum += ms;  // the first run warms up
+            }
+            if (ok && (best < 0.0 || ms_sum / 2.0 < best)) {
+                best = ms_sum / 2.0;
+                best_leaf = leaf;
+                best_chunk = ch;
             }
         }
     }
@@ -558,11 +548,11 @@ extern "C" int rs_batch_autotune(rs_batch* b, int* h_leaf, int* h_chunk, int* h_
             b->own[h] = nb;
         }
     }
-    rs_batch_set_options(b, best_chunk, best_stack, graph);
+    rs_batch_set_options(b, best_chunk, 0, graph);
     b->dirty = true;
     if (h_leaf) *h_leaf = best_leaf;
     if (h_chunk) *h_chunk = best_chunk;
-    if (h_stack) *h_stack = best_stack;
+    if (h_stack) *h_stack = kStack;
     if (h_ms) *h_ms = best;
     if (result == RS_OK && best < 0.0) result = RS_ERR_ITER_LIMIT;  // no configuration completed
     return result;

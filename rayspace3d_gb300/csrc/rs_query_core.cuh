@@ -624,8 +624,7 @@ __device__ __forceinline__ void count_edge(const PairTable& table, int taken) {
 template <int STACK>
 __device__ __forceinline__ bool segment_fast(const EdgeColumn& col, const Ray& r, const int32_t* __restrict__ src,
                                              int nsrc, const BNode* __restrict__ nodes, uint32_t max_steps,
-                                             const float4* __restrict__ tris, int swap, const PairTable& table,
-                                             int start = 0) {
+                                             const float4* __restrict__ tris, int swap, const PairTable& table) {
     const int S = col.stride;
     int n = 0;
     unsigned int tests = 0;
@@ -653,7 +652,7 @@ __device__ __forceinline__ bool segment_fast(const EdgeColumn& col, const Ray& r
             }
             ++n;
         }
-    }, start);
+    });
     add_tests(tests);
     if (!ok || n > kEdgeHits) return false;
     EdgeWalk w;
