@@ -151,25 +151,33 @@ __global__ void __launch_bounds__(kBT, 6) k_batch(const BatchQuery* __restrict__
     }
 }
 
+// Edges a thread each, then points a warp each.
 __global__ void __launch_bounds__(kBT) k_batch_fallback(const BatchQuery* __restrict__ q,
                                                         const uint2* __restrict__ ovf,
                                                         const unsigned long long* __restrict__ ovf_count) {
+    static_assert(kBT == 32 * kRangeWarps, "a warp's shared memory");
+    __shared__ RangeWarp warps[kRangeWarps];
     const unsigned long long cnt = min(*ovf_count, (unsigned long long)kOverflowCap);
-    for (unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; e < cnt;
-         e += (unsigned long long)gridDim.x * blockDim.x) {
-        const uint2 item = ovf[e];
-        const BatchQuery& Q = q[item.x];
-        const uint64_t i = item.y;
-        if (Q.kind == 1) {
-            edge_ray_long(EdgePayload{Q.starts, Q.ends, Q.offsets, Q.counts, Q.sources}, i, Q.nodes, Q.max_steps,
+    const unsigned long long threads = (unsigned long long)gridDim.x * blockDim.x;
+    for (unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; e < cnt; e += threads) {
+        const BatchQuery& Q = q[ovf[e].x];
+        if (Q.kind == 1)
+            edge_ray_long(EdgePayload{Q.starts, Q.ends, Q.offsets, Q.counts, Q.sources}, ovf[e].y, Q.nodes, Q.max_steps,
                           Q.tris, Q.swap, Q.table);
-            continue;
-        }
+    }
+    __syncwarp();
+    RangeWarp& w = warps[threadIdx.x >> 5];
+    for (unsigned long long e = blockIdx.x * (unsigned long long)kRangeWarps + (threadIdx.x >> 5); e < cnt;
+         e += threads / 32) {
+        const BatchQuery& Q = q[ovf[e].x];
+        if (Q.kind == 1) continue;  // the same in every lane
+        const uint64_t i = ovf[e].y;
         const Ray r = make_ray(Q.pts[3 * i], Q.pts[3 * i + 1], Q.pts[3 * i + 2], Q.dx, Q.dy, Q.dz, kEps, kTmax);
-        if (Q.axis == 0) pim_fallback_ray<0, kStack>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
-        else if (Q.axis == 1) pim_fallback_ray<1, kStack>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
-        else if (Q.axis == 2) pim_fallback_ray<2, kStack>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
-        else pim_fallback_ray<-1, kStack>(Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
+        if (Q.axis == 0) pim_range_ray<0>(w, Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
+        else if (Q.axis == 1) pim_range_ray<1>(w, Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
+        else if (Q.axis == 2) pim_range_ray<2>(w, Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
+        else pim_range_ray<-1>(w, Q.nodes, Q.max_steps, Q.tris, r, Q.status, Q.obj, Q.in, i);
+        __syncwarp();
     }
 }
 

@@ -1362,7 +1362,6 @@ __global__ void __launch_bounds__(kT) k_containment_tracked(const float* __restr
 constexpr int kContWarps = 4;    // objects per block
 constexpr int kContStack = 320;  // entries of a warp's stack
 constexpr int kContHits = 512;   // crossings a warp keeps
-constexpr int kStackRoom = 64;   // a level of the tree each, descended one node at a time
 // Objects from which rays are traced in packets first.  80,000 objects with a target of 3 large
 // spheres, 20,000 and 100,000 dense ones: 298, 632 and 4,500 us with packets, 500, 735 and 3,970
 // without (a thread an object: 410, 980, 54,000); 200,000 objects: 395, 1,190 and 9,590 against 895,

@@ -143,22 +143,23 @@ __global__ void __launch_bounds__(kT, kGridBlocks) k_pim_grid(const float* __res
         [&](uint32_t i) { leave_ray(ovf_list, ovf_count, left, i); });
 }
 
-// Exact fallback for rays with more than kHits crossings (pim_fallback_ray).
+// The rays left over: of more than kDenseHits crossings on a column grid, of more than kPacketHits
+// or of an unfinished packet otherwise.  80 registers and 6 blocks an SM: 10 % less than 126 and
+// 4, or 72 and 7.
 template <int AXIS>
-__global__ void __launch_bounds__(kT) k_pim_fallback(const float* __restrict__ pts, float dx, float dy, float dz,
-                                                     const BNode* __restrict__ nodes, uint32_t max_steps,
-                                                     const float4* __restrict__ tris,
-                                                     int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
-                                                     unsigned int* __restrict__ status,
-                                                     const uint32_t* __restrict__ ovf_list,
-                                                     const unsigned long long* __restrict__ ovf_count) {
+__global__ void __launch_bounds__(32 * kRangeWarps, 6) k_pim_fallback(
+    const float* __restrict__ pts, float dx, float dy, float dz, const BNode* __restrict__ nodes, uint32_t max_steps,
+    const float4* __restrict__ tris, int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in,
+    unsigned int* __restrict__ status, const uint32_t* __restrict__ ovf_list,
+    const unsigned long long* __restrict__ ovf_count) {
+    __shared__ RangeWarp warps[kRangeWarps];
     const unsigned long long cnt = *ovf_count;
-    for (unsigned long long q = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; q < cnt;
-         q += (unsigned long long)gridDim.x * blockDim.x) {
-        const uint32_t i = ovf_list[q];
-        const Ray r = make_ray(pts[3 * (uint64_t)i], pts[3 * (uint64_t)i + 1], pts[3 * (uint64_t)i + 2], dx, dy, dz,
-                               kEps, kTmax);
-        pim_fallback_ray<AXIS, kStack>(nodes, max_steps, tris, r, status, out_obj, out_in, i);
+    for (unsigned long long q = blockIdx.x * (unsigned long long)kRangeWarps + (threadIdx.x >> 5); q < cnt;
+         q += (unsigned long long)gridDim.x * kRangeWarps) {
+        const uint64_t i = ovf_list[q];
+        const Ray r = make_ray(pts[3 * i], pts[3 * i + 1], pts[3 * i + 2], dx, dy, dz, kEps, kTmax);
+        pim_range_ray<AXIS>(warps[threadIdx.x >> 5], nodes, max_steps, tris, r, status, out_obj, out_in, i);
+        __syncwarp();
     }
 }
 
@@ -450,7 +451,8 @@ int run_pim_axis(const rs_bvh* bvh, const float* pts, uint64_t n, float dx, floa
         if (e == cudaSuccess) e = e2;
     }
     if (e == cudaSuccess && h[1]) {
-        launch(k_pim_fallback<AXIS>, (unsigned)((h[1] + kT - 1) / kT), kT, 0, s, pts, dx, dy, dz, bvh->nodes,
+        const uint64_t blocks = std::min<uint64_t>((h[1] + kRangeWarps - 1) / kRangeWarps, 16ull * sm_count());
+        launch(k_pim_fallback<AXIS>, (unsigned)blocks, 32 * kRangeWarps, 0, s, pts, dx, dy, dz, bvh->nodes,
                max_steps(bvh), (const float4*)bvh->tris, obj, in, status, (const uint32_t*)ovf,
                (const unsigned long long*)(meta + 1));
         e = cudaMemcpyAsync(h, meta, kWords, cudaMemcpyDeviceToHost, s);
