@@ -213,22 +213,25 @@ __global__ void __launch_bounds__(kT) k_morton(const float* __restrict__ V, uint
         if (obox) {
             const int32_t o = T[t];
             int v[6] = {flt_ord(lo[0]), flt_ord(lo[1]), flt_ord(lo[2]), flt_ord(hi[0]), flt_ord(hi[1]), flt_ord(hi[2])};
-            // A range without a number (lo is then the empty box's already) widens no box: as a
-            // maximum it would make the object's box one that overlaps nothing.
+            // A range without a number, 0x7fffffff from either bound, widens no box: as a maximum it
+            // would make the object's box one that overlaps nothing.  One more, it is the least.
 #pragma unroll
-            for (int k = 0; k < 3; ++k) v[3 + k] = isnan(hi[k]) ? (int)0x80000000 : v[3 + k];
-            if (o < 0) atomicOr(bad_index, 4u);
+            for (int k = 3; k < 6; ++k) v[k] = (int)((unsigned int)v[k] + 1u);
             const unsigned int peers = __match_any_sync(__activemask(), o);
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 v[k] = __reduce_min_sync(peers, v[k]);
                 v[3 + k] = __reduce_max_sync(peers, v[3 + k]);
             }
-            if ((int)(threadIdx.x & 31) == __ffs(peers) - 1 && o >= 0 && (uint64_t)o < obox_cap) {
+            if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) {
+                if (o < 0) {
+                    atomicOr(bad_index, 4u);
+                } else if ((uint64_t)o < obox_cap) {
 #pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    atomicMin(&obox[6 * (uint64_t)o + k], v[k]);
-                    atomicMax(&obox[6 * (uint64_t)o + 3 + k], v[3 + k]);
+                    for (int k = 0; k < 3; ++k) {
+                        atomicMin(&obox[6 * (uint64_t)o + k], v[k]);
+                        atomicMax(&obox[6 * (uint64_t)o + 3 + k], v[3 + k] == (int)0x80000000 ? v[3 + k] : v[3 + k] - 1);
+                    }
                 }
             }
         }
