@@ -105,7 +105,7 @@ struct WarpEdgeSmem {
 // are inserted by all lanes (one lane's inserts, a few hundred dependent atomics an edge,
 // took a tenth of a clustered join's k_edge_long_warp).
 //
-// A step pops no more nodes than the stack has room to replace twice over, so a wide
+// A step pops no more nodes than leave kStackRoom entries of the stack, so a wide
 // traversal turns into a depth-first one instead of running out of stack: an edge of a
 // large object in a dense cluster overlaps thousands of boxes, and the one-thread loop that
 // used to take such an edge kept a whole join waiting (17 ms of 57).  An edge of more than
@@ -140,7 +140,7 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
         uint32_t visits = 0;
         bool ok = true;
         while (sp > 0) {
-            const int take = min(min(sp, 32), max(STACK - sp, 1));
+            const int take = min(min(sp, 32), max(STACK - kStackRoom - sp, 1));
             const int node = lane < take ? stack[sp - take + lane] : -1;
             __syncwarp();
             sp -= take;
@@ -252,11 +252,11 @@ __device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload
 // of the edge in one traversal (or, beyond kLongWarpHits, in a traversal per range of t; the
 // reference's walk takes at most --overlap-max-iterations of them) instead of one thread
 // re-traversing per chunk of 16, which is left for more than kLongWarpHits crossings at one
-// distance (segment_long, in lane 0).  512 crossings take 52 KB a block of 4 warps, which
+// distance (segment_long, in lane 0).  512 crossings take 53 KB a block of 4 warps, which
 // leaves 4 blocks an SM: 9 % less for a clustered join's long edges than 256 and 7 blocks,
 // for fewer restarts.
 constexpr int kLongWarps = 4;
-constexpr int kLongWarpStack = 256;
+constexpr int kLongWarpStack = 320;
 constexpr int kLongWarpHits = 512;
 
 __global__ void __launch_bounds__(32 * kLongWarps) k_edge_long_warp(EdgePayload p, const uint32_t* __restrict__ deferred,
@@ -1128,7 +1128,7 @@ __global__ void __launch_bounds__(32 * kCullWarps, kCullResident) k_cull_query(C
                 __syncwarp();
                 continue;
             }
-            const int take = min(min(sp, 32), max(kCullStack - sp, 1));
+            const int take = min(min(sp, 32), max(kCullStack - kStackRoom - sp, 1));
             sp -= take;
             visits += (uint32_t)take;
             if (visits > budget) {

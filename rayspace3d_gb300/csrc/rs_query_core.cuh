@@ -468,6 +468,11 @@ __device__ __forceinline__ void grid_points(const GridView& g, const float4* __r
 // the previous one, so the crossings are walked in the same order as the sorted list.
 constexpr int kLongHits = 64;
 
+// Entries that a warp's traversal keeps free of its stack when it pops many nodes at a time: one
+// for each level of the tree that it then descends by one node at a time.  Popping what just fits
+// fills the stack to its last entry, and the next node with two inner children breaks off.
+constexpr int kStackRoom = 64;
+
 template <int AXIS>
 __device__ __forceinline__ void pim_fallback_ray(const BNode* __restrict__ nodes, uint32_t max_steps,
                                                  const float4* __restrict__ tris, const Ray& r,
@@ -568,7 +573,6 @@ __device__ __forceinline__ void pim_fallback_ray(const BNode* __restrict__ nodes
 // suited better: 5 M of them 7.9 ms, now 8.9.
 constexpr int kRangeHits = 512;
 constexpr int kRangeStack = 320;
-constexpr int kStackRoom = 64;  // a level of the tree each, descended one node at a time
 constexpr int kRangeWarps = 4;  // a block
 
 struct RangeWarp {
@@ -1006,8 +1010,8 @@ __device__ __forceinline__ unsigned int packet_trace(RayPacket& sm, const Ray& m
             __syncwarp();
             continue;
         }
-        // No more nodes than the stack has room to replace twice over.
-        const int take = min(min(sp, 32), max(kPacketStack - sp, 1));
+        // No more nodes than leave kStackRoom entries: a wide traversal turns into a depth-first one.
+        const int take = min(min(sp, 32), max(kPacketStack - kStackRoom - sp, 1));
         if (++steps > max_steps) break;
         sp -= take;
         bool h0 = false, h1 = false;
