@@ -86,191 +86,68 @@ __global__ void __launch_bounds__(32 * kPacketWarps, 6) k_edge_rays(
     }
 }
 
-// Shared-memory columns of one warp's edge: a stack of STACK node entries, and HITS
-// crossings twice (as found, then sorted).
-template <int STACK, int HITS>
-struct WarpEdgeSmem {
-    int stack[STACK];
-    float t[HITS], t2[HITS];
-    uint32_t id[HITS], id2[HITS];
-    int32_t obj[HITS], obj2[HITS];
-};
-
-// One edge by one warp: the lanes pop up to 32 nodes per step from the warp's
-// shared-memory stack, test both children of each, test the triangles of the leaves hit
-// and push the inner children hit; crossings go to a shared-memory list.  Visits the nodes
-// the one-thread traversal visits (the same slab tests over the same [tmin, tmax]), so it
-// finds the same crossings; the lanes rank them by (t, id) (triangle ids are distinct, so
-// ranks are too), lane 0 walks them with the table's hit rule, and the pairs of the hits taken
-// are inserted by all lanes (one lane's inserts, a few hundred dependent atomics an edge,
-// took a tenth of a clustered join's k_edge_long_warp).
-//
-// A step pops no more nodes than leave kStackRoom entries of the stack, so a wide
-// traversal turns into a depth-first one instead of running out of stack: an edge of a
-// large object in a dense cluster overlaps thousands of boxes, and the one-thread loop that
-// used to take such an edge kept a whole join waiting (17 ms of 57).  An edge of more than
-// HITS crossings is walked in ranges of t: the list's middle crossing ends the range and the
-// traversal restarts on it, until a range's crossings fit; the next range begins above it.
-// Returns false when there are more than HITS crossings at one and the same t or the step
-// budget or the stack runs out; pairs of ranges walked before
-// that are in the table, where the one-thread loop's start from the beginning finds them.
-template <int STACK, int HITS>
-__device__ bool edge_ray_warp(WarpEdgeSmem<STACK, HITS>& w_sm, const EdgePayload& p, uint64_t i,
-                              const BNode* __restrict__ nodes, uint32_t max_steps, const float4* __restrict__ tris,
-                              int swap, const PairTable& table) {
-    int* stack = w_sm.stack;
-    float* ht = w_sm.t;
-    uint32_t* hid = w_sm.id;
-    int32_t* hobj = w_sm.obj;
+// One edge by one warp, its crossings in ranges of t (range_collect).  Lane 0 walks a range with
+// the table's hit rule, and the pairs of the hits taken are inserted by all lanes (one lane's
+// inserts, a few hundred dependent atomics an edge, took a tenth of a clustered join's
+// k_edge_long_warp).  An edge of a large object in a dense cluster overlaps thousands of boxes,
+// and the one-thread loop kept a whole join waiting (17 ms of 57).  A full list that threw its
+// traversal away and began again with half the range took 84 ms for 240,000 edges through 2,000
+// boxes, where a thread an edge had taken 75; now 39.
+// Returns false when range_collect does; pairs of ranges walked before that are in the table,
+// where the one-thread loop's start from the beginning finds them.
+__device__ __forceinline__ bool edge_ray_warp(RangeWarp& w_sm, const EdgePayload& p, uint64_t i,
+                                              const BNode* __restrict__ nodes, uint32_t max_steps,
+                                              const float4* __restrict__ tris, int swap, const PairTable& table) {
     const int lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
     Ray r;
     if (!segment_ray_of(p.starts[3 * i], p.starts[3 * i + 1], p.starts[3 * i + 2], p.ends[3 * i], p.ends[3 * i + 1],
                         p.ends[3 * i + 2], r))
         return true;
     const float tmax = r.tmax;
-    float above = -INFINITY;  // crossings up to here are walked
+    float above = -INFINITY;
     EdgeWalk w;
     int32_t last = INT_MIN;
+    int nh = 0;
     unsigned int tests = 0;
-    for (;;) {
-        if (lane == 0) stack[0] = 0;
-        __syncwarp();
-        int sp = 1, nh = 0;
-        uint32_t visits = 0;
-        bool ok = true;
-        while (sp > 0) {
-            const int take = min(min(sp, 32), max(STACK - kStackRoom - sp, 1));
-            const int node = lane < take ? stack[sp - take + lane] : -1;
-            __syncwarp();
-            sp -= take;
-            visits += (uint32_t)take;
-            if (visits > max_steps) {
-                ok = false;
-                break;
-            }
-            bool h[2] = {false, false};
-            int first[2] = {0, 0}, cnt[2] = {0, 0};
-            if (node >= 0) {
-                const BNode bn = load_node(nodes, node);
-                const float4 na = bn.a, nb = bn.b, nc = bn.c;
-                const int4 nd = bn.d;
-                const float lo0[3] = {na.x, na.y, na.z}, hi0[3] = {na.w, nb.x, nb.y};
-                const float lo1[3] = {nb.z, nb.w, nc.x}, hi1[3] = {nc.y, nc.z, nc.w};
-                float e, x;
-                h[0] = slab<-1>(r, lo0, hi0, r.tmin, r.tmax, e, x);
-                h[1] = slab<-1>(r, lo1, hi1, r.tmin, r.tmax, e, x);
-                first[0] = nd.x;
-                cnt[0] = nd.y;
-                first[1] = nd.z;
-                cnt[1] = nd.w;
-            }
-            // Triangles of the leaves hit: the first child's, then the second's.
-            const int n0 = h[0] ? cnt[0] : 0, n1 = h[1] ? cnt[1] : 0;
-            tests += (unsigned int)(n0 + n1);
-            const int rounds = __reduce_max_sync(0xffffffffu, n0 + n1);
-            for (int k = 0; k < rounds; ++k) {
-                bool hit = false;
-                float t = 0.0f;
-                uint32_t tid = 0;
-                int32_t obj = 0;
-                if (k < n0 + n1) {
-                    float a[3], b[3], c[3];
-                    load_tri(tris, k < n0 ? first[0] + k : first[1] + (k - n0), a, b, c, tid, obj);
-                    hit = hit_triangle<-1>(r, a, b, c, t) && t > above;
-                }
-                const unsigned m = __ballot_sync(0xffffffffu, hit);
-                if (hit) {
-                    const int pos = nh + __popc(m & lt);
-                    if (pos < HITS) {
-                        ht[pos] = t;
-                        hid[pos] = tid;
-                        hobj[pos] = obj;
-                    }
-                }
-                nh += __popc(m);
-            }
-            if (nh > HITS) break;
-            const bool p0 = h[0] && cnt[0] == 0, p1 = h[1] && cnt[1] == 0;
-            const unsigned b0 = __ballot_sync(0xffffffffu, p0), b1 = __ballot_sync(0xffffffffu, p1);
-            const int total = __popc(b0) + __popc(b1);
-            if (sp + total > STACK) {
-                ok = false;
-                break;
-            }
-            int pos = sp + __popc(b0 & lt) + __popc(b1 & lt);
-            if (p0) stack[pos++] = first[0];
-            if (p1) stack[pos] = first[1];
-            __syncwarp();
-            sp += total;
-        }
-        __syncwarp();
-        if (!ok) return false;
-        const int kept = min(nh, HITS);
-        for (int a = lane; a < kept; a += 32) {
-            const float t = ht[a];
-            const uint32_t id = hid[a];
-            int rank = 0;
-            for (int b = 0; b < kept; ++b) rank += hit_less(ht[b], hid[b], t, id) ? 1 : 0;
-            w_sm.t2[rank] = t;
-            w_sm.id2[rank] = id;
-            w_sm.obj2[rank] = hobj[a];
-        }
-        __syncwarp();
-        if (nh > HITS) {
-            const float mid = w_sm.t2[HITS / 2];
-            if (!(mid < r.tmax)) return false;
-            r.tmax = mid;
-            continue;
-        }
-        int found = 0;  // objects to insert: hobj, whose crossings are copied out
+    do {
+        if (!range_collect<-1>(w_sm, nodes, max_steps, tris, r, above, nh, tests)) return false;
+        range_sort(w_sm, nh);
+        int found = 0;  // objects to insert, over those walked
         if (lane == 0)
             for (int a = 0; a < nh && !w.done; ++a) {
-                if (!w.take(w_sm.t2[a], table.max_hits, table.next_float)) continue;
-                if (w_sm.obj2[a] == last) continue;
-                last = w_sm.obj2[a];
-                hobj[found++] = last;
+                if (!w.take(range_t(w_sm, a), table.max_hits, table.next_float)) continue;
+                if (w_sm.obj[a] == last) continue;
+                last = w_sm.obj[a];
+                w_sm.obj[found++] = last;
             }
         found = __shfl_sync(0xffffffffu, found, 0);
         __syncwarp();
         for (int a = lane; a < found; a += 32)
-            insert_sources(table, p.sources + p.offsets[i], p.counts[i], hobj[a], swap);
+            insert_sources(table, p.sources + p.offsets[i], p.counts[i], w_sm.obj[a], swap);
         __syncwarp();
-        if (r.tmax == tmax || __shfl_sync(0xffffffffu, (int)w.done, 0)) break;
-        above = r.tmax;
-        r.tmin = fmaxf(r.tmin, above);
-        r.tmax = tmax;
-        __syncwarp();
-    }
+    } while (!__shfl_sync(0xffffffffu, (int)w.done, 0) && next_range(r, tmax, above));
     add_tests(tests);
     if (lane == 0) count_edge(table, w.n);
     __syncwarp();
     return true;
 }
 
-// Long path over the deferred edges, one warp per edge: the warp collects every crossing
-// of the edge in one traversal (or, beyond kLongWarpHits, in a traversal per range of t; the
-// reference's walk takes at most --overlap-max-iterations of them) instead of one thread
-// re-traversing per chunk of 16, which is left for more than kLongWarpHits crossings at one
-// distance (segment_long, in lane 0).  512 crossings take 53 KB a block of 4 warps, which
-// leaves 4 blocks an SM: 9 % less for a clustered join's long edges than 256 and 7 blocks,
-// for fewer restarts.
-constexpr int kLongWarps = 4;
-constexpr int kLongWarpStack = 320;
-constexpr int kLongWarpHits = 512;
+// Long path over the deferred edges, one warp per edge; the one-thread loop (segment_long, in
+// lane 0, 16 crossings a traversal) is left for hundreds of crossings at one distance.
+constexpr int kLongWarps = kRangeWarps;
 
-__global__ void __launch_bounds__(32 * kLongWarps) k_edge_long_warp(EdgePayload p, const uint32_t* __restrict__ deferred,
+__global__ void __launch_bounds__(32 * kLongWarps, 4) k_edge_long_warp(EdgePayload p, const uint32_t* __restrict__ deferred,
                                                                     const unsigned int* __restrict__ n_def,
                                                                     const BNode* __restrict__ nodes, uint32_t max_steps,
                                                                     const float4* __restrict__ tris, int swap,
                                                                     PairTable table) {
-    __shared__ WarpEdgeSmem<kLongWarpStack, kLongWarpHits> sm[kLongWarps];
+    __shared__ RangeWarp sm[kLongWarps];
     const unsigned int n = *n_def;
     const int wi = threadIdx.x >> 5;
     const unsigned int nw = gridDim.x * kLongWarps;
     for (unsigned int j = blockIdx.x * kLongWarps + wi; j < n; j += nw) {  // warp-uniform
         const uint32_t e = deferred[j];
-        if (!edge_ray_warp<kLongWarpStack, kLongWarpHits>(sm[wi], p, e, nodes, max_steps, tris, swap, table) &&
+        if (!edge_ray_warp(sm[wi], p, e, nodes, max_steps, tris, swap, table) &&
             (threadIdx.x & 31) == 0)
             edge_ray_long(p, e, nodes, max_steps, tris, swap, table);
         __syncwarp();

@@ -563,14 +563,17 @@ __device__ __forceinline__ void pim_fallback_ray(const BNode* __restrict__ nodes
     write_result(ch, i, out_obj, out_in);
 }
 
-// The rays that a query leaves over, one warp each.  All crossings go to a list, in ranges of t:
-// a full list keeps those up to its middle one, which becomes the range's end, and the traversal
-// goes on with what is left of its stack; the next range begins above it.  Sorted by (t, id), a
-// range's crossings are walked by the advance rule.  A thread a ray found the crossings beyond
-// its 64th by a traversal each: 20,000 points in 300 shells, up to 600 crossings, took 10.3 s (4.8
-// while such rays shared their warps with others), now 1.8 ms; 2 M oblique rays of up to 40
-// crossings 23.5 ms, now 12.5.  Oblique rays of 9 to 12 crossings are the ones that threads had
-// suited better: 5 M of them 7.9 ms, now 8.9.
+// Rays of many crossings, one warp each: up to 32 nodes a step from a shared-memory stack, and all
+// crossings in a list, in ranges of t: a full list keeps those up to its middle one, which becomes
+// the range's end, and the traversal goes on with what is left of its stack; the next range
+// begins above it.  Sorted by (t, id), a range's crossings are walked by the caller's rule.  Visits
+// the nodes that one thread's traversal of the range would, so it finds the same crossings.
+//
+// Points: what a query leaves over.  A thread a ray found the crossings beyond its 64th by a
+// traversal each: 20,000 points in 300 shells, up to 600 crossings, took 10.3 s (4.8 while such
+// rays shared their warps with others), now 1.8 ms; 2 M oblique rays of up to 40 crossings 23.5 ms,
+// now 12.5.  Oblique rays of 9 to 12 crossings are the ones that threads had suited better: 5 M of
+// them 7.9 ms, now 8.9.
 constexpr int kRangeHits = 512;
 constexpr int kRangeStack = 320;
 constexpr int kRangeWarps = 4;  // a block
@@ -609,107 +612,120 @@ __device__ __forceinline__ float range_t(const RangeWarp& w, int i) {
     return __uint_as_float((uint32_t)(w.key[i] >> 32));
 }
 
+// Every crossing of ray r with t in (above, r.tmax] into the warp's list, unsorted, nh of them; when
+// they are more than it holds, those of a range that begins there, whose end becomes r.tmax.
+// False when the stack, the steps or, at one distance, the list run out.
+template <int AXIS>
+__device__ __forceinline__ bool range_collect(RangeWarp& w, const BNode* __restrict__ nodes, uint32_t max_steps,
+                                              const float4* __restrict__ tris, Ray& r, float above, int& nh,
+                                              unsigned int& tests) {
+    constexpr unsigned int kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned int below = (1u << lane) - 1u;
+    if (lane == 0) w.stack[0] = 0;
+    __syncwarp();
+    int sp = 1;
+    uint32_t visits = 0;
+    nh = 0;
+    while (sp > 0) {
+        const int take = min(min(sp, 32), max(kRangeStack - kStackRoom - sp, 1));
+        const int node = lane < take ? w.stack[sp - take + lane] : -1;
+        __syncwarp();
+        sp -= take;
+        visits += (uint32_t)take;
+        bool h[2] = {false, false};
+        int leaf[2] = {0, 0}, cnt[2] = {0, 0};
+        if (node >= 0) {
+            const BNode bn = load_node(nodes, node);
+            const float lo0[3] = {bn.a.x, bn.a.y, bn.a.z}, hi0[3] = {bn.a.w, bn.b.x, bn.b.y};
+            const float lo1[3] = {bn.b.z, bn.b.w, bn.c.x}, hi1[3] = {bn.c.y, bn.c.z, bn.c.w};
+            float en, ex;
+            h[0] = slab<AXIS>(r, lo0, hi0, r.tmin, r.tmax, en, ex);
+            h[1] = slab<AXIS>(r, lo1, hi1, r.tmin, r.tmax, en, ex);
+            leaf[0] = bn.d.x;
+            cnt[0] = bn.d.y;
+            leaf[1] = bn.d.z;
+            cnt[1] = bn.d.w;
+        }
+        const bool p0 = h[0] && cnt[0] == 0, p1 = h[1] && cnt[1] == 0;
+        const unsigned int b0 = __ballot_sync(kAll, p0), b1 = __ballot_sync(kAll, p1);
+        const int pushed = __popc(b0) + __popc(b1);
+        if (visits > max_steps || sp + pushed > kRangeStack) return false;
+        int pos = sp + __popc(b0 & below) + __popc(b1 & below);
+        if (p0) w.stack[pos++] = leaf[0];
+        if (p1) w.stack[pos] = leaf[1];
+        sp += pushed;
+        // Triangles of the leaves hit: the first child's, then the second's.
+        const int n0 = h[0] ? cnt[0] : 0, n1 = h[1] ? cnt[1] : 0;
+        tests += (unsigned int)(n0 + n1);
+        const int rounds = __reduce_max_sync(kAll, n0 + n1);
+        for (int k = 0; k < rounds; ++k) {
+            bool hit = false;
+            float t = 0.0f;
+            uint32_t tid = 0;
+            int32_t obj = 0;
+            if (k < n0 + n1) {
+                float a[3], b[3], c[3];
+                load_tri(tris, k < n0 ? leaf[0] + k : leaf[1] + (k - n0), a, b, c, tid, obj);
+                hit = hit_triangle<AXIS>(r, a, b, c, t) && t > above;
+            }
+            unsigned int m = __ballot_sync(kAll, hit);
+            if (nh + __popc(m) > kRangeHits) {
+                range_sort(w, nh);
+                const float mid = range_t(w, nh / 2);
+                int n = nh / 2 + 1;
+                while (n < nh && range_t(w, n) == mid) ++n;
+                __syncwarp();
+                r.tmax = mid;
+                nh = n;
+                hit = hit && t <= mid;
+                m = __ballot_sync(kAll, hit);
+                if (nh + __popc(m) > kRangeHits) return false;  // hundreds at one distance
+            }
+            if (hit) {
+                const int at = nh + __popc(m & below);
+                w.key[at] = (uint64_t)__float_as_uint(t) << 32 | tid;
+                w.obj[at] = obj;
+            }
+            nh += __popc(m);
+        }
+        __syncwarp();
+    }
+    return true;
+}
+
+// The range after the one that ends at r.tmax; false when that was the last.
+__device__ __forceinline__ bool next_range(Ray& r, float tmax, float& above) {
+    if (r.tmax == tmax) return false;
+    above = r.tmax;
+    r.tmin = fmaxf(r.tmin, above);
+    r.tmax = tmax;
+    return true;
+}
+
 template <int AXIS>
 __device__ __forceinline__ void pim_range_ray(RangeWarp& w, const BNode* __restrict__ nodes, uint32_t max_steps,
                                               const float4* __restrict__ tris, Ray r, unsigned int* __restrict__ status,
                                               int32_t* __restrict__ out_obj, uint8_t* __restrict__ out_in, uint64_t i) {
-    constexpr unsigned int kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const unsigned int below = (1u << lane) - 1u;
     const Ray whole = r;
     float above = -INFINITY;
     Chain ch;
-    int walked = 0;
-    bool ok = true;
-    for (;;) {
-        if (lane == 0) w.stack[0] = 0;
-        __syncwarp();
-        int sp = 1, nh = 0;
-        uint32_t visits = 0;
-        while (sp > 0 && ok) {
-            const int take = min(min(sp, 32), max(kRangeStack - kStackRoom - sp, 1));
-            const int node = lane < take ? w.stack[sp - take + lane] : -1;
-            __syncwarp();
-            sp -= take;
-            visits += (uint32_t)take;
-            bool h[2] = {false, false};
-            int leaf[2] = {0, 0}, cnt[2] = {0, 0};
-            if (node >= 0) {
-                const BNode bn = load_node(nodes, node);
-                const float lo0[3] = {bn.a.x, bn.a.y, bn.a.z}, hi0[3] = {bn.a.w, bn.b.x, bn.b.y};
-                const float lo1[3] = {bn.b.z, bn.b.w, bn.c.x}, hi1[3] = {bn.c.y, bn.c.z, bn.c.w};
-                float en, ex;
-                h[0] = slab<AXIS>(r, lo0, hi0, r.tmin, r.tmax, en, ex);
-                h[1] = slab<AXIS>(r, lo1, hi1, r.tmin, r.tmax, en, ex);
-                leaf[0] = bn.d.x;
-                cnt[0] = bn.d.y;
-                leaf[1] = bn.d.z;
-                cnt[1] = bn.d.w;
-            }
-            const bool p0 = h[0] && cnt[0] == 0, p1 = h[1] && cnt[1] == 0;
-            const unsigned int b0 = __ballot_sync(kAll, p0), b1 = __ballot_sync(kAll, p1);
-            const int pushed = __popc(b0) + __popc(b1);
-            if (visits > max_steps || sp + pushed > kRangeStack) {
-                ok = false;
-                break;
-            }
-            int pos = sp + __popc(b0 & below) + __popc(b1 & below);
-            if (p0) w.stack[pos++] = leaf[0];
-            if (p1) w.stack[pos] = leaf[1];
-            sp += pushed;
-            // Triangles of the leaves hit: the first child's, then the second's.
-            const int n0 = h[0] ? cnt[0] : 0, n1 = h[1] ? cnt[1] : 0;
-            const int rounds = __reduce_max_sync(kAll, n0 + n1);
-            for (int k = 0; k < rounds; ++k) {
-                bool hit = false;
-                float t = 0.0f;
-                uint32_t tid = 0;
-                int32_t obj = 0;
-                if (k < n0 + n1) {
-                    float a[3], b[3], c[3];
-                    load_tri(tris, k < n0 ? leaf[0] + k : leaf[1] + (k - n0), a, b, c, tid, obj);
-                    hit = hit_triangle<AXIS>(r, a, b, c, t) && t > above;
-                }
-                unsigned int m = __ballot_sync(kAll, hit);
-                if (nh + __popc(m) > kRangeHits) {
-                    range_sort(w, nh);
-                    const float mid = range_t(w, nh / 2);
-                    int n = nh / 2 + 1;
-                    while (n < nh && range_t(w, n) == mid) ++n;
-                    __syncwarp();
-                    r.tmax = mid;
-                    nh = n;
-                    hit = hit && t <= mid;
-                    m = __ballot_sync(kAll, hit);
-                    if (nh + __popc(m) > kRangeHits) {  // hundreds at one distance
-                        ok = false;
-                        break;
-                    }
-                }
-                if (hit) {
-                    const int at = nh + __popc(m & below);
-                    w.key[at] = (uint64_t)__float_as_uint(t) << 32 | tid;
-                    w.obj[at] = obj;
-                }
-                nh += __popc(m);
-            }
-            __syncwarp();
-        }
-        __syncwarp();
-        if (!ok) break;
+    int walked = 0, nh = 0;
+    unsigned int tests = 0;
+    bool ok;
+    while ((ok = range_collect<AXIS>(w, nodes, max_steps, tris, r, above, nh, tests))) {
         range_sort(w, nh);
         for (int k = 0; k < nh && ch.count < kPimMaxIters; ++k) ch.step(range_t(w, k), w.obj[k]);
         walked += nh;
         __syncwarp();
-        if (r.tmax == whole.tmax || ch.count >= kPimMaxIters) break;
+        if (ch.count >= kPimMaxIters || !next_range(r, whole.tmax, above)) break;
         if (walked >= kFallbackIters) {
             if (lane == 0) atomicOr(status, ST_ITER_LIMIT);
             break;
         }
-        above = r.tmax;
-        r.tmin = fmaxf(r.tmin, above);
-        r.tmax = whole.tmax;
     }
+    __syncwarp();
     if (lane != 0) return;
     if (ok) write_result(ch, i, out_obj, out_in);
     else pim_fallback_ray<AXIS>(nodes, max_steps, tris, whole, status, out_obj, out_in, i);

@@ -1,5 +1,5 @@
-"""How many nodes a warp's traversal pops at a time (packet_trace, k_cull_query, edge_ray_warp,
-k_containment, containment_many, pim_range_ray), restated: on trees whose nodes are all hit, down
+"""How many nodes a warp's traversal pops at a time (packet_trace, range_collect, k_cull_query,
+k_containment, containment_many), restated: on trees whose nodes are all hit, down
 to 20 complete levels, on lopsided ones of 64, and from one root or 32, the stack holds every
 child; with nothing kept free it breaks off."""
 import os
@@ -9,7 +9,7 @@ import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "rayspace3d_gb300", "csrc")
 RULE = re.compile(r"const int take = min\(min\(sp, 32\), max\((\w+) - kStackRoom - sp, 1\)\);")
-LOOPS = {"rs_query_core.cuh": 2, "rs_join.cu": 4}
+LOOPS = {"rs_query_core.cuh": 2, "rs_join.cu": 3}
 
 
 def _sources():
@@ -30,7 +30,7 @@ def _stacks():
     for f, text in _sources().items():
         names = RULE.findall(text)
         assert len(names) == LOOPS[f] == len(re.findall(r"const int take = ", text)), f
-        sizes += [_constant("kLongWarpStack" if n == "STACK" else n) for n in names]
+        sizes += [_constant(n) for n in names]
     return sorted(set(sizes))
 
 
