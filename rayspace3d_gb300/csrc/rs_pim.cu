@@ -495,14 +495,15 @@ BoxBounds make_box(const rs_bvh* bvh) {
 
 // The status word and overflow count of a call, device memory that is zero while it waits in
 // its device's pool, and pinned words for their copy and run_pim's `left`: a call then needs
-// neither an allocation nor a memset for them, and a copy back only when rays were left.  A call has one to itself until it has
-// synchronised, so calls on other streams and threads have others.
+// neither an allocation nor a memset for them, and a copy back only when rays were left.  A call
+// has one to itself until it has synchronised, so calls on other streams and threads have others.
 struct CallWords {
     unsigned long long* dev = nullptr;
     unsigned long long* host = nullptr;
 };
 std::mutex g_words_mu;
 std::vector<CallWords> g_words[64];
+size_t g_words_made[64];  // room in the vector for all of them, so that giving one back cannot throw
 
 cudaError_t words_acquire(int device, CallWords* out, cudaStream_t s) {
     if (device < 0 || device >= 64) return cudaErrorInvalidDevice;
@@ -511,6 +512,11 @@ cudaError_t words_acquire(int device, CallWords* out, cudaStream_t s) {
     if (pool.empty()) {  // as many as are ever in flight together, kept until the process ends
         constexpr int kBlock = 32;
         unsigned long long *d = nullptr, *h = nullptr;
+        try {
+            pool.reserve(g_words_made[device] + kBlock);
+        } catch (...) {
+            return cudaErrorMemoryAllocation;
+        }
         // Relaxed, and no work on the legacy stream: another thread may be capturing a stream.
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         cudaThreadExchangeStreamCaptureMode(&mode);
@@ -525,6 +531,7 @@ cudaError_t words_acquire(int device, CallWords* out, cudaStream_t s) {
             return e;
         }
         for (int k = 0; k < kBlock; ++k) pool.push_back(CallWords{d + 32 * k, h + 32 * k});
+        g_words_made[device] += kBlock;
     }
     *out = pool.back();
     pool.pop_back();
