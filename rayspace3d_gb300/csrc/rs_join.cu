@@ -2,16 +2,17 @@
 //
 // Edge rays replace __raygen__mesh_overlap_edges / trace_edge_multi_hits_edges
 // (query/src/cuda/mesh_overlap_edges.cu:106-216) and __raygen__mesh_overlap
-// (mesh_intersection.cu:16-91,288-334): one thread per unique edge traces the
-// segment once (the reference re-traces per hit and, in the intersection variant,
-// per source object), takes its crossings with the reference's hit rule and inserts
-// (source, target) pairs straight into the pair table.  The edges a broad phase keeps
-// are binned by the Morton cell of their midpoint first, so the 32 rays of a warp
-// start close together and descend the same subtrees.  Containment replaces
-// __raygen__mesh_containment_anyhit + __anyhit__ah_containment
-// (mesh_intersection_anyhit.cu:46-240): one +Z ray per
-// source object, parity per target object kept in registers instead of a
-// 256-slot global scratch per object.
+// (mesh_intersection.cu:16-91,288-334): a warp traces up to 32 unique edges as a packet, each
+// once (the reference re-traces per hit and, in the intersection variant, per source
+// object), takes their crossings with the reference's hit rule and inserts (source, target)
+// pairs straight into the pair table; edges of many crossings follow, a warp each.  The
+// edges a broad phase keeps are binned by the Morton cell of their midpoint first, so that
+// the rays of a warp start close together and descend the same subtrees.  Containment
+// replaces __raygen__mesh_containment_anyhit + __anyhit__ah_containment
+// (mesh_intersection_anyhit.cu:46-240): one +Z ray per source object by a warp (in packets
+// first when there are very many), the object ids of its crossings in shared memory instead
+// of a 256-slot global scratch per object; only the per-source diagnostics take a thread an
+// object with the parities in registers.
 #include <algorithm>
 #include <climits>
 

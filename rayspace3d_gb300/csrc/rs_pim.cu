@@ -7,17 +7,16 @@
 //
 // The reference re-traces a closest-hit query from t_min = t + 1e-6 until it misses
 // (crossings + 1 traversals per ray).  Here every crossing with t in [1e-6, 1e16] is
-// collected once into a per-thread register list, sorted by (t, triangle id), and the
-// reference's advance rule is applied to the sorted list.  A ray with more crossings
-// than the list holds is queued for an exact fallback that walks the hits in the same
-// order by re-traversal.
+// collected once, by the warp, and the reference's advance rule is applied to the crossings
+// in (t, triangle id) order.  Rays of more crossings than the query keeps follow in a second
+// launch, a warp each, in ranges of t (pim_range_ray).
 //
 // Candidates come from one of two structures with the same hit set:
 //  * rays along +x, +y or +z use a column grid: a uniform 2D grid over the projection
 //    of the leaf-ordered triangles.  Triangle boxes and query points go through the
 //    same monotone cell formula, so every triangle whose projection can contain the
-//    (perturbed) point is in the point's cell;
-//  * any other direction traverses the BVH.
+//    (perturbed) point is in the point's cell; up to 8 crossings a lane, 256 a warp;
+//  * any other direction traverses the BVH in packets of 32 rays, up to 8 crossings each.
 #include <algorithm>
 #include <climits>
 #include <cmath>

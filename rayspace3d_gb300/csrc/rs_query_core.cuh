@@ -732,10 +732,11 @@ __device__ __forceinline__ void pim_range_ray(RangeWarp& w, const BNode* __restr
 }
 
 // ---------------------------------------------------------------------------
-// Edge rays.  The fast path traces an edge once with its stack and its crossings
-// (up to kEdgeHits) in a column of shared memory; an edge with more crossings, or a
-// traversal deeper than the fast stack, is deferred untouched to the long path, which
-// runs the reference's trace loop literally.
+// Edge rays by one thread.  The per-triangle join's fast path traces an edge once with its
+// stack and its crossings (up to kEdgeHits) in a column of shared memory; an edge with more
+// crossings, or a traversal deeper than the fast stack, is deferred untouched to the long
+// path.  Payload edges go in packets and ranges (edge_packet below, edge_ray_warp) and come
+// to the long path for hundreds of crossings at one distance only.
 // ---------------------------------------------------------------------------
 constexpr int kEdgeHits = 4;
 
@@ -845,8 +846,8 @@ __device__ __forceinline__ bool segment_fast(const EdgeColumn& col, const Ray& r
 // walked in (t, triangle id) order with the table's hit rule, kLongChunk at a time.  Each
 // pass traverses once, nearer child first, and keeps the kLongChunk smallest crossings
 // beyond the last one walked (the ray's tmax shrinks to the largest kept one once the
-// chunk is full, so the pass visits little beyond it); the walk then takes them, and a full chunk starts the
-// next pass after its last crossing.  A crossing's t does not depend on tmin or tmax (the
+// chunk is full, so the pass visits little beyond it); the walk then takes them, and a full
+// chunk starts the next pass after its last crossing.  A crossing's t does not depend on tmin or tmax (the
 // node and triangle slab tests only accept or reject), so the passes see exactly the
 // crossings the reference's one-hit-per-trace loop sees, in the same order, while an
 // edge with h crossings costs about h / kLongChunk traversals instead of h.
