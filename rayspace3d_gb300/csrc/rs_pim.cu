@@ -197,7 +197,7 @@ __device__ __forceinline__ int ford(float f) {
 }
 
 // Bounds of all triangles (b: ordered ints: u, v, w ranges) and the sums of their projected
-// boxes' widths, heights and areas (finite ones), which choose the cell size.
+// boxes' widths, heights and areas (finite ones each), which choose the cell size.
 template <int AXIS>
 __global__ void k_cg_bounds(const float4* __restrict__ tris, int n, int* __restrict__ b, double* __restrict__ sums) {
     // [0..5] minima of u, -u, v, -v, w, -w, then the three sums (a thread sums a few dozen
@@ -210,11 +210,9 @@ __global__ void k_cg_bounds(const float4* __restrict__ tris, int n, int* __restr
 #pragma unroll
         for (int q = 0; q < 6; ++q) v[q] = fminf(v[q], m[q]);
         const float w = t.uh - t.ul, h = t.vh - t.vl;
-        if (w * h < INFINITY) {
-            v[6] += w;
-            v[7] += h;
-            v[8] += w * h;
-        }
+        v[6] += w < INFINITY ? w : 0.0f;
+        v[7] += h < INFINITY ? h : 0.0f;
+        v[8] += w * h < INFINITY ? w * h : 0.0f;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -338,6 +336,45 @@ double grid_cells(double n, double w, double h, const double* sum) {
     return std::min(std::max(finest * (s / s0) * (s / s0), 1.0), finest);
 }
 
+struct GridSize {
+    int gu, gv;
+};
+
+// Columns and rows of about `target` cells, shaped like the projected bounds (endless ones have a
+// scale of zero, so one cell).
+GridSize grid_shape(double target, double w, double h) {
+    GridSize g{1, 1};
+    if (!std::isfinite(w)) w = 0.0;
+    if (!std::isfinite(h)) h = 0.0;
+    if (w > 0 && h > 0) {
+        g.gu = (int)std::lround(std::min(std::max(std::sqrt(target * w / h), 1.0), 8192.0));
+        g.gv = (int)std::lround(std::min(std::max(target / g.gu, 1.0), 8192.0));
+    } else if (w > 0) {
+        g.gu = (int)std::min(std::max(target, 1.0), 8192.0);
+    } else if (h > 0) {
+        g.gv = (int)std::min(std::max(target, 1.0), 8192.0);
+    }
+    return g;
+}
+
+// The grid's size, halved until its own cells -- not square where the bounds are longer than
+// 8,192 cells, or flat -- keep about the entries that grid_cells allows, and until no place of
+// the boxes in them can make 2^32 (a box of w x h cells touches at most (w + 2)(h + 2); from
+// 2^30 triangles on, that many around the same cells' corners, one in two is allowed for).
+GridSize grid_size(double n, double w, double h, const double* sum) {
+    const double budget = std::max(kEntries * n, kFree), slack = n < 1073741824.0 ? 4.0 : 2.0;
+    // Areas that overflowed a float are not in the sum.
+    const double area = w * h < 1e38 ? sum[2] : std::min(sum[0] * h, sum[1] * w);
+    for (double target = grid_cells(n, w, h, sum);; target *= 0.5) {
+        const GridSize g = grid_shape(target, w, h);
+        const double su = w > 0 && std::isfinite(w) ? g.gu / w : 0.0, sv = h > 0 && std::isfinite(h) ? g.gv / h : 0.0;
+        const double boxes = su > 0 && sv > 0 ? su * sv * area : 0.0, edges = su * sum[0] + sv * sum[1];
+        if (g.gu * g.gv == 1 ||
+            (boxes + edges + n <= 2.0 * budget && boxes + 2.0 * edges + slack * n < 4294967296.0))
+            return g;
+    }
+}
+
 template <int AXIS>
 cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
     rs_column_grid& cg = bvh->cgrid[AXIS];
@@ -367,17 +404,8 @@ cudaError_t build_grid(rs_bvh* bvh, cudaStream_t s) {
     const double depth = (double)cg.w1 - cg.w0;
     cg.sw = depth > 0 ? (float)(256.0 / depth) : 0.0f;
     const double w = (double)cg.u1 - cg.u0, hh = (double)cg.v1 - cg.v0;
-    const double target = grid_cells(n, w, hh, h.sum);
-    int gu = 1, gv = 1;
-    if (w > 0 && hh > 0) {
-        gu = (int)std::lround(std::sqrt(target * w / hh));
-        gu = std::min(std::max(gu, 1), 8192);
-        gv = (int)std::min(std::max(std::lround(target / gu), 1L), 8192L);
-    } else if (w > 0) {
-        gu = (int)std::min(target, 8192.0);
-    } else if (hh > 0) {
-        gv = (int)std::min(target, 8192.0);
-    }
+    const GridSize size = grid_size(n, w, hh, h.sum);
+    const int gu = size.gu, gv = size.gv;
     cg.gu = gu;
     cg.gv = gv;
     cg.su = w > 0 ? (float)gu / (float)w : 0.0f;
