@@ -92,8 +92,8 @@ __global__ void __launch_bounds__(32 * kPacketWarps, 6) k_edge_rays(
 // inserts, a few hundred dependent atomics an edge, took a tenth of a clustered join's
 // k_edge_long_warp).  An edge of a large object in a dense cluster overlaps thousands of boxes,
 // and the one-thread loop kept a whole join waiting (17 ms of 57).  A full list that threw its
-// traversal away and began again with half the range took 84 ms for 240,000 edges through 2,000
-// boxes, where a thread an edge had taken 75; now 39.
+// traversal away and began again with half the range took 84 ms for the edges of 20,000 boxes that
+// reach through 2,000 others, where a thread an edge had taken 75; now 39.
 // Returns false when range_collect does; pairs of ranges walked before that are in the table,
 // where the one-thread loop's start from the beginning finds them.
 __device__ __forceinline__ bool edge_ray_warp(RangeWarp& w_sm, const EdgePayload& p, uint64_t i,
